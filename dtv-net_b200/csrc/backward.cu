@@ -8,9 +8,9 @@
 // one launch per view (or per 21 views), read-modify-writing the whole volume
 // each time (backwardKernel.cu:50,101-103). Here the view loop is inside the
 // kernel; the projective map of each view (FP64-derived, see geometry.cu)
-// gives the detector coordinates with one reciprocal per voxel-view.
+// gives the detector coordinates with one reciprocal per voxel-view (one per
+// column and view on z-affine orbits).
 #include <algorithm>
-#include <type_traits>
 #include <vector>
 #include <string.h>
 
@@ -23,66 +23,42 @@ struct BPParams {
   int power;
   int extent;
   float scale;
-  int64_t sino_pad_elems;  // one padded view
-  int warp;                // columns of a warp and a quad (DTV_TUNE_BP_WARP)
-  int vsplit;              // 2: two halves of a block sum the two halves of the views
+  int64_t view_recs;  // records of one view
+  int warp;           // columns of a warp and a quad (DTV_TUNE_BP_WARP)
+  int cull;           // blocks skip the views whose detector they miss
 };
 
 constexpr int kBPTile = 16;  // columns per block edge
 // Views whose 3x4 maps travel in one launch's parameters: read through the
-// constant cache, they leave the L1/texture pipe to the sinogram fetches.
+// constant cache, they leave the L1 pipe to the sinogram records.
 constexpr int kBPParamViews = 640;
 struct BPMaps {
   float m[kBPParamViews][12];
 };
 static_assert(sizeof(BPMaps) <= 31 * 1024, "kernel parameter space");
-// voxels per thread along z: 8, or 4 / 2 where a volume has too few columns
-// to fill the GPU (bp_zc); the results do not depend on it
-constexpr int kZCMax = 8;
-constexpr int64_t kBPWantBlocks = 4 * 148;  // four resident blocks per SM
 constexpr int kBPThreads = kBPTile * kBPTile;
+// voxels per thread along z (16 measured 3 % slower through the texture unit and
+// 10 - 20 % through records: fewer resident warps)
+constexpr int kZC = 8;
 
-struct SoftBil {
-  const float* s;  // padded view
-  int pu;
-  float mu, mv;
-  __device__ __forceinline__ float operator()(float u, float v) const {
-    const float fu = floorf(u), fv = floorf(v);
-    const float au = u - fu, av = v - fv;
-    const int iu = (int)fminf(fmaxf(fu, -2.f), mu) + kPad;
-    const int iv = (int)fminf(fmaxf(fv, -2.f), mv) + kPad;
-    const float* b = s + iv * pu + iu;
-    const float v00 = __ldg(b), v01 = __ldg(b + 1), v10 = __ldg(b + pu), v11 = __ldg(b + pu + 1);
-    const float c0 = fmaf(au, v01 - v00, v00), c1 = fmaf(au, v11 - v10, v10);
-    return fmaf(av, c1 - c0, c0);
-  }
-};
+// Where a bilinear detector sample comes from.
+// kTex: the texture unit (a layered FP32 texture, 8-bit weights), one fetch.
+// kRec: one 16-byte record through L1, FP32 weights. Record (U, V) of a view
+// (padded by kPad zeros on each side) holds its cell's bilinear polynomial
+// s(au, av) = A + au B + av C + au av D in the order (A, C, B, D): A = s(U, V),
+// B = s(U+1, V) - A, C = s(U, V+1) - A, D the mixed difference.
+// kBoth: both, two sums per voxel (the correction pass of a texture plan
+// against an exact one).
+enum BPMode { kRec = 0, kTex = 1, kBoth = 2 };
 
-// The same bilinear sample from 16-byte records of the padded view (exact
-// plans): record (U, V) = (s(U, V), s(U+1, V), s(U, V+1), s(U+1, V+1)) at
-// padded indices, one 128-bit load per voxel-view.
-struct QuadBil {
-  const float4* q;  // records of the view
-  int pu;
-  float mu, mv;
-  __device__ __forceinline__ float operator()(float u, float v) const {
-    const float fu = floorf(u), fv = floorf(v);
-    const float au = u - fu, av = v - fv;
-    const int iu = (int)fminf(fmaxf(fu, -2.f), mu) + kPad;
-    const int iv = (int)fminf(fmaxf(fv, -2.f), mv) + kPad;
-    const float4 r = __ldg(q + iv * pu + iu);
-    const float c0 = fmaf(au, r.y - r.x, r.x), c1 = fmaf(au, r.w - r.z, r.z);
-    return fmaf(av, c1 - c0, c0);
-  }
-};
-
-// Where the backprojector's detector values come from. kSrcBoth: the texture
-// and the quad records of the same sinogram, two sums per voxel (the
-// correction pass of a texture-filtered plan against an exact one).
-enum BPSource { kSrcSoft = 0, kSrcTex = 1, kSrcQuad = 2, kSrcBoth = 3 };
+// Adding 1.5 * 2^23 leaves an integer in the sum's low bits; with rounding down
+// the sum is the floor. The float to integer conversions this replaces run at
+// a quarter rate (40 % of that pipe, and 2.4 x the instructions per sample).
+constexpr float kIntMagic = 12582912.f;
+constexpr unsigned int kIntMagicBits = 0x4B400000u;
 
 // Where a block's sums go: out = base + sum (out = sum when base is NULL; base
-// may be out). kSrcBoth: out takes the quad-record sum E, and
+// may be out). kBoth: out takes the record sum E, and
 // diff = diff_base + (E - T) with T the texture sum.
 struct BPOut {
   float* out;
@@ -91,10 +67,6 @@ struct BPOut {
   const float* diff_base;
 };
 
-// kZAff: every view's u and h are independent of z (a detector parallel to the
-// rotation axis, as in the circular orbits), so per column and view the kernel
-// computes u, 1/h and the weight once and each voxel costs one FMA for v, one
-// fetch and one FMA.
 // Where a view's 3x4 map comes from: the launch parameters (one chunk of
 // views) or the plan's device table.
 struct ParamMaps {
@@ -106,68 +78,161 @@ struct TableMaps {
   __device__ __forceinline__ const float* row(int jn) const { return v[jn].m; }
 };
 
-// One block's columns: tile `tile` of 16x16 (x, y) columns, z-chunk `zc` of ZC
-// voxels, views n0 .. n0 + n_chunk - 1. With bp.vsplit == 2 (volumes too small
-// to fill the GPU otherwise) the tile is 16x8 columns and the block's two
-// halves take the first and the second half of the views; the second half's
-// sums are added to the first's through shared memory, in that order, so the
-// result is deterministic.
-template <int kSrc, bool kZAff, int ZC, bool kSplit, class Maps>
-__device__ __forceinline__ void bp_columns(const BPParams& bp, const Maps& maps, int n0, int n_chunk,
-                                           const float* __restrict__ spad, cudaTextureObject_t tex,
-                                           const BPOut& dst, int tile, int zc) {
-  const int tiles_x = (bp.nx + kBPTile - 1) / kBPTile;
-  // this thread's column in the 16 x 16 tile; a warp covers 16 x 2, 8 x 4 or
-  // 4 x 8 columns (the narrower, the fewer detector rows' cache sectors one
-  // fetch instruction touches when a voxel spans several pixels)
-  const int t = (int)threadIdx.x;
-  constexpr bool split = kSplit;  // bp.vsplit == 2, chosen by the launch
-  const int half = split ? t >> 7 : 0;
-  int li, lj;
-  if constexpr (split) {
-    li = t & 15;
-    lj = (t & 127) >> 4;
-  } else if (bp.warp >= 3) {
-    // quads (4 consecutive lanes) of 2 x 2 columns; a warp of 8 quads covers
-    // 8 x 4 (warp 3) or 4 x 8 (warp 4) columns
-    const int q = (t >> 2) & 7, qi = t & 1, qj = (t >> 1) & 1, w = t >> 5;
-    if (bp.warp == 3) {
-      li = ((q & 3) << 1 | qi) | ((w & 1) << 3);
-      lj = ((q >> 2) << 1 | qj) | ((w >> 1) << 2);
-    } else {
-      li = ((q & 1) << 1 | qi) | ((w & 3) << 2);
-      lj = ((q >> 1) << 1 | qj) | ((w >> 2) << 3);
-    }
-  } else if (bp.warp == 1) {
-    li = (t & 7) | (((t >> 5) & 1) << 3);
-    lj = ((t >> 3) & 3) | ((t >> 6) << 2);
-  } else if (bp.warp == 2) {
-    li = (t & 3) | (((t >> 5) & 3) << 2);
-    lj = ((t >> 2) & 7) | ((t >> 7) << 3);
-  } else {
-    li = t & 15;
-    lj = t >> 4;
+// The cells of two coordinates (t = floor + kIntMagic) and the fractions in them.
+struct Frac2 {
+  f32x2_t t, a;
+};
+__device__ __forceinline__ Frac2 frac2(f32x2_t v) {
+  Frac2 r;
+  r.t = add2_rm(v, splat2(kIntMagic));
+  r.a = sub2(v, sub2(r.t, splat2(kIntMagic)));
+  return r;
+}
+// The record's bilinear sample; au2 = (au, au).
+__device__ __forceinline__ float bilinear(const float4 r, f32x2_t au2, float av) {
+  float p, q;  // (A + au B, C + au D)
+  unpack2(fma2(au2, f32x2(r.z, r.w), f32x2(r.x, r.y)), p, q);
+  return fmaf(av, q, p);
+}
+
+// The first record of column u's cell in a view, as an address biased so that
+// adding (float bits of floor(v) + kIntMagic) * row bytes gives row floor(v).
+__device__ __forceinline__ unsigned long long cell_base(const char* view, unsigned int tu_bits,
+                                                        unsigned int row_bytes) {
+  const long long iu = (int)(tu_bits - kIntMagicBits) + kPad;
+  return (unsigned long long)view + (unsigned long long)(iu * 16) +
+         (unsigned long long)row_bytes * kPad - (unsigned long long)kIntMagicBits * row_bytes;
+}
+__device__ __forceinline__ float4 cell_at(unsigned long long base, unsigned int tv_bits,
+                                          unsigned int row_bytes) {
+  return __ldg(reinterpret_cast<const float4*>(base + (unsigned long long)tv_bits * row_bytes));
+}
+
+// Whether view map w can see any voxel of the box [i0, i1] x [j0, j1] x
+// [k0, k1]: false only if all eight corners lie in front of the source and
+// project beyond one edge of the detector by more than a pixel past the last
+// sample that reaches it (the box then projects into their convex hull, and
+// every one of its samples is exactly zero).
+__host__ __device__ __forceinline__ bool box_seen(const float* w, float i0, float i1, float j0, float j1,
+                                         float k0, float k1, float nu, float nv) {
+  float umin = 3.4e38f, umax = -3.4e38f, vmin = 3.4e38f, vmax = -3.4e38f, hmin = 3.4e38f;
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    const float x = (c & 1) ? i1 : i0, y = (c & 2) ? j1 : j0, z = (c & 4) ? k1 : k0;
+    const float h = fmaf(w[8], x, fmaf(w[9], y, fmaf(w[10], z, w[11])));
+    const float u = fmaf(w[0], x, fmaf(w[1], y, fmaf(w[2], z, w[3]))) / h;
+    const float v = fmaf(w[4], x, fmaf(w[5], y, fmaf(w[6], z, w[7]))) / h;
+    hmin = fminf(hmin, h);
+    umin = fminf(umin, u); umax = fmaxf(umax, u);
+    vmin = fminf(vmin, v); vmax = fmaxf(vmax, v);
   }
-  const int i = (tile % tiles_x) * kBPTile + li;
-  const int j = (tile / tiles_x) * (split ? kBPTile / 2 : kBPTile) + lj;
+  return !(hmin > 1e-3f && (umax < -2.f || umin > nu + 1.f || vmax < -2.f || vmin > nv + 1.f));
+}
+
+// One block's columns: column tile `tile`, z-chunk `zc` of kZC voxels, views
+// n0 .. n0 + n_chunk - 1. S == 1: a tile is 16 x 16 columns. S > 1 (volumes
+// too small to fill the GPU otherwise): the block's S groups of 256 / S threads
+// own the same tile of (64 / (2 S)) x 8 columns and each takes one of S equal
+// runs of the views; their sums are added through shared memory in the order
+// of the runs, so the result is deterministic.
+//
+// kZAff: every view's u and h are independent of z (a detector parallel to the
+// rotation axis, as in the circular orbits), so per column and view the kernel
+// computes u, 1/h and the weight once and marches v. Voxels go in pairs along
+// z through packed FP32. A thread's z-run projects to a monotone run of v (and
+// u), so two end tests replace per-voxel bounds: wholly on the detector runs
+// unchecked, wholly beside it is skipped (its samples are zeros), and only
+// runs across an edge clamp each voxel.
+//
+// Bound: through the texture unit its fetch rate (256^3 x 64 views of 384^2:
+// 0.84 ms; 1.03 ms before a column's views beside the detector were skipped,
+// 16 % of that scan's column-views). Through records the L1 lines of a warp's
+// load (6.5 per load, 2 clocks each where they miss) and their latency: 1.62 ms
+// from four scalar loads, 1.22 ms from records with conversions, 0.90 ms now.
+// The records could also reproduce the texture filter (its weights are
+// alpha beta to 1/256 exactly), but at 1.06 - 1.11 ms they lose to it.
+template <int S>
+struct BPShape {
+  static constexpr int kGroup = kBPThreads / S;           // threads, one column each
+  static constexpr int kH = S == 1 ? kBPTile : 8;         // tile rows (y)
+  static constexpr int kW = kGroup / kH;                  // tile columns (x)
+};
+
+template <int kMode, bool kZAff, int S, bool kCull, class Maps>
+__device__ __forceinline__ void bp_columns(const BPParams& bp, const Maps& maps, int n0, int n_chunk,
+                                           const float4* __restrict__ recs, cudaTextureObject_t tex,
+                                           const BPOut& dst, int tile, int zc) {
+  static_assert(kZC % 2 == 0, "voxels go in pairs");
+  constexpr int ZC = kZC;
+  using Shape = BPShape<S>;
+  const int tiles_x = (bp.nx + Shape::kW - 1) / Shape::kW;
+  const int t = (int)threadIdx.x;
+  const int group = S > 1 ? t / Shape::kGroup : 0;
+  // this thread's column in the tile: quads (4 consecutive lanes) of 2 x 2
+  // columns, a warp of 8 quads covers 4 x 8 columns, or with S == 1 as
+  // DTV_TUNE_BP_WARP says: 16 x 2, 8 x 4 or 4 x 8 of row quads, 8 x 4 of squares
+  const int q = (t >> 2) & 7, qi = t & 1, qj = (t >> 1) & 1, wp = (t % Shape::kGroup) >> 5;
+  int li = ((q & 1) << 1 | qi) | ((wp & (Shape::kW / 4 - 1)) << 2);
+  int lj = ((q >> 1) << 1 | qj) | (S == 1 ? (wp >> 2) << 3 : 0);
+  if constexpr (S == 1) {
+    if (bp.warp == 3) {
+      li = ((q & 3) << 1 | qi) | ((wp & 1) << 3);
+      lj = ((q >> 2) << 1 | qj) | ((wp >> 1) << 2);
+    } else if (bp.warp == 2) {
+      li = (t & 3) | (((t >> 5) & 3) << 2);
+      lj = ((t >> 2) & 7) | ((t >> 7) << 3);
+    } else if (bp.warp == 1) {
+      li = (t & 7) | (((t >> 5) & 1) << 3);
+      lj = ((t >> 3) & 3) | ((t >> 6) << 2);
+    } else if (bp.warp == 0) {
+      li = t & 15;
+      lj = t >> 4;
+    }
+  }
+  const int ti = (tile % tiles_x) * Shape::kW, tj = (tile / tiles_x) * Shape::kH;
+  const int i = ti + li, j = tj + lj;
   const int k0 = zc * ZC;
   const bool valid = i < bp.nx && j < bp.ny;
-  if (!valid && !split) return;  // the split halves meet at a barrier below
-  // this thread's views: all of the chunk, or one half of it
-  const int hv = (n_chunk + 1) / 2;
-  const int jn0 = split ? half * hv : 0;
-  const int jn1 = !valid ? jn0 : (split && half == 0 ? hv : n_chunk);
-  constexpr bool kBoth = kSrc == kSrcBoth;
-  float acc[ZC], act[kBoth ? ZC : 1];
+  // kCull: the views some voxel of the block can be seen in, one bit each
+  __shared__ unsigned int seen[kCull ? kBPParamViews / 32 : 1];
+  if constexpr (kCull) {
+    for (int jb = 0; jb < n_chunk; jb += kBPThreads) {
+      const int jn = jb + t;
+      const bool s = jn < n_chunk &&
+                     box_seen(maps.row(jn), (float)ti, (float)(ti + Shape::kW - 1), (float)tj,
+                              (float)(tj + Shape::kH - 1), (float)k0, (float)(k0 + ZC - 1),
+                              (float)bp.nu, (float)bp.nv);
+      const unsigned int m = __ballot_sync(0xffffffffu, s);
+      if ((t & 31) == 0 && jn < n_chunk) seen[jn >> 5] = m;
+    }
+    __syncthreads();
+  }
+  if (!valid && S == 1) return;  // the groups of a split block meet at a barrier below
+  // this thread's views: all of the chunk, or its group's run of them
+  const int hv = (n_chunk + S - 1) / S;
+  const int jn0 = min(group * hv, n_chunk);
+  const int jn1 = valid ? min(jn0 + hv, n_chunk) : jn0;
+  float acc[ZC], act[kMode == kBoth ? ZC : 1];
 #pragma unroll
   for (int z = 0; z < ZC; ++z) acc[z] = 0.f;
 #pragma unroll
-  for (int z = 0; z < (kBoth ? ZC : 1); ++z) act[z] = 0.f;
+  for (int z = 0; z < (kMode == kBoth ? ZC : 1); ++z) act[z] = 0.f;
   const float fi = (float)i, fj = (float)j;
-  const int pu = bp.nu + 2 * kPad;
   const float mu = (float)bp.nu, mv = (float)bp.nv;
-  for (int jn = jn0; jn < jn1; ++jn) {
-    const int n = n0 + jn;
+  const unsigned int row_bytes = (unsigned int)(bp.nu + 2 * kPad) * 16u;
+  const float kf0 = (float)k0;
+  // the next view at or after jn that the block can be seen in
+  auto next_seen = [&](int jn) {
+    if constexpr (kCull) {
+      while (jn < jn1) {
+        const unsigned int m = seen[jn >> 5] >> (jn & 31);
+        if (m) return jn + __ffs((int)m) - 1;
+        jn = (jn | 31) + 1;
+      }
+    }
+    return jn;
+  };
+  for (int jn = next_seen(jn0); jn < jn1; jn = next_seen(jn + 1)) {
     const float* w = maps.row(jn);
     const float m0 = w[0], m1 = w[1], m2 = w[2], m3 = w[3];
     const float m4 = w[4], m5 = w[5], m6 = w[6], m7 = w[7];
@@ -175,77 +240,187 @@ __device__ __forceinline__ void bp_columns(const BPParams& bp, const Maps& maps,
     const float bu = fmaf(m0, fi, fmaf(m1, fj, m3));
     const float bv = fmaf(m4, fi, fmaf(m5, fj, m7));
     const float bh = fmaf(m8, fi, fmaf(m9, fj, m11));
-    using Smp = typename std::conditional<kSrc == kSrcQuad || kBoth, QuadBil, SoftBil>::type;
-    Smp smp;
-    if constexpr (kSrc == kSrcQuad || kBoth)
-      smp = QuadBil{reinterpret_cast<const float4*>(spad) + (int64_t)n * bp.sino_pad_elems, pu,
-                    mu, mv};
-    else
-      smp = SoftBil{spad + (int64_t)n * bp.sino_pad_elems, pu, mu, mv};
+    const char* view = reinterpret_cast<const char*>(recs + (int64_t)(n0 + jn) * bp.view_recs);
     if constexpr (kZAff) {
       const float rh = __frcp_rn(bh);
       // v from the absolute slice index: the same bits for every z-chunking.
       // Coordinates are rounded explicitly (no contraction into FMAs), so
       // every kernel instance samples a voxel-view at the same position.
       const float u = __fmul_rn(bu, rh), vb = __fmul_rn(bv, rh), dv = __fmul_rn(m6, rh);
-      const float tu = __fadd_rn(u, 0.5f);  // texture coordinate (texel centres at i + 1/2)
       float wgt = bp.scale;
       if (bp.power == 2) wgt *= rh * rh;
       else if (bp.power == 1) wgt *= rh;
-      const bool col_out = bp.extent && (tu < -1.f || tu > bp.nx + 1.f);
-      if (col_out) continue;
+      if (bp.extent) {
+        const float tu = __fadd_rn(u, 0.5f);
+        if (tu < -1.f || tu > bp.nx + 1.f) continue;
+      }
+      const float va = fmaf(kf0, dv, vb), ve = fmaf(kf0 + (float)(ZC - 1), dv, vb);
+      const float vlo = fminf(va, ve), vhi = fmaxf(va, ve);
+      // zero samples only (a non-finite weight still goes through below)
+      if ((u < -1.f || u >= mu || vhi < -1.f || vlo >= mv) && fabsf(wgt) < 3.4e38f) continue;
+      const float tu = __fadd_rn(u, 0.5f);  // texture coordinate (texel centres at i + 1/2)
+      const Frac2 fu = frac2(splat2(fminf(fmaxf(u, -2.f), mu)));
+      float tu_f, dummy;
+      unpack2(fu.t, tu_f, dummy);
+      const unsigned long long base = cell_base(view, __float_as_uint(tu_f), row_bytes);
+      const bool inside = vlo >= -1.f && vhi < mv && u >= -1.f && u < mu && !bp.extent;
+      if (kMode == kTex || inside) {
 #pragma unroll
-      for (int z = 0; z < ZC; ++z) {
-        const float v = fmaf((float)(k0 + z), dv, vb);
-        const float tv = __fadd_rn(v, 0.5f);
-        float wz = wgt;
-        if (bp.extent && (tv < -1.f || tv > bp.ny + 1.f)) wz = 0.f;
-        float val;
-        if constexpr (kSrc == kSrcTex) val = tex2DLayered<float>(tex, tu, tv, n);
-        else val = smp(u, v);
-        acc[z] = fmaf(val, wz, acc[z]);
-        if constexpr (kBoth) act[z] = fmaf(tex2DLayered<float>(tex, tu, tv, n), wz, act[z]);
+        for (int z = 0; z < ZC; z += 2) {
+          const f32x2_t v2 =
+              fma2(f32x2(kf0 + (float)z, kf0 + (float)(z + 1)), splat2(dv), splat2(vb));
+          float v[2], w2[2] = {wgt, wgt};
+          unpack2(v2, v[0], v[1]);
+          if constexpr (kMode != kRec) {
+#pragma unroll
+            for (int y = 0; y < 2; ++y) {
+              const float tv = __fadd_rn(v[y], 0.5f);
+              if (bp.extent && (tv < -1.f || tv > bp.ny + 1.f)) w2[y] = 0.f;
+              float& a = kMode == kBoth ? act[kMode == kBoth ? z + y : 0] : acc[z + y];
+              a = fmaf(tex2DLayered<float>(tex, tu, tv, n0 + jn), w2[y], a);
+            }
+          }
+          if constexpr (kMode != kTex) {
+            const Frac2 fv = frac2(v2);
+            float t[2], av[2];
+            unpack2(fv.t, t[0], t[1]);
+            unpack2(fv.a, av[0], av[1]);
+#pragma unroll
+            for (int y = 0; y < 2; ++y)
+              acc[z + y] = fmaf(bilinear(cell_at(base, __float_as_uint(t[y]), row_bytes), fu.a, av[y]),
+                                wgt, acc[z + y]);
+          }
+        }
+      } else {
+#pragma unroll
+        for (int z = 0; z < ZC; ++z) {
+          const float v = fmaf(kf0 + (float)z, dv, vb);
+          const float tv = __fadd_rn(v, 0.5f);
+          float wz = wgt;
+          if (bp.extent && (tv < -1.f || tv > bp.ny + 1.f)) wz = 0.f;
+          const Frac2 fv = frac2(splat2(fminf(fmaxf(v, -2.f), mv)));
+          float t0, av;
+          unpack2(fv.t, t0, dummy);
+          unpack2(fv.a, av, dummy);
+          acc[z] = fmaf(bilinear(cell_at(base, __float_as_uint(t0), row_bytes), fu.a, av), wz, acc[z]);
+          if constexpr (kMode == kBoth)
+            act[z] = fmaf(tex2DLayered<float>(tex, tu, tv, n0 + jn), wz, act[z]);
+        }
       }
     } else {
+      // u, v, h of two voxels at slices (ka, kb)
+      struct UVH {
+        f32x2_t u, v, rh;
+        float ha, hb;
+      };
+      auto project = [&](float ka, float kb) {
+        const f32x2_t kk = f32x2(ka, kb);
+        UVH p;
+        unpack2(fma2(splat2(m10), kk, splat2(bh)), p.ha, p.hb);
+        p.rh = f32x2(rcp_newton(p.ha), rcp_newton(p.hb));
+        p.u = mul2(fma2(splat2(m2), kk, splat2(bu)), p.rh);
+        p.v = mul2(fma2(splat2(m6), kk, splat2(bv)), p.rh);
+        return p;
+      };
+      bool inside, beside;
+      {
+        const UVH p = project(kf0, kf0 + (float)(ZC - 1));
+        float ua, ub, va, ve;
+        unpack2(p.u, ua, ub);
+        unpack2(p.v, va, ve);
+        const bool front = p.ha > 0.f && p.hb > 0.f;
+        const float ulo = fminf(ua, ub), uhi = fmaxf(ua, ub), vlo = fminf(va, ve),
+                    vhi = fmaxf(va, ve);
+        // u and v are monotone along the run up to rounding, hence the margin
+        beside = front && (uhi < -1.02f || ulo > mu + 0.02f || vhi < -1.02f || vlo > mv + 0.02f);
+        inside = front && ulo >= -1.f && uhi < mu && vlo >= -1.f && vhi < mv;
+        if (bp.extent)
+          inside = inside && __fadd_rn(uhi, 0.5f) <= bp.nx + 1.f && __fadd_rn(vhi, 0.5f) <= bp.ny + 1.f;
+      }
+      if (beside) continue;
+      const unsigned long long vbase =
+          cell_base(view, kIntMagicBits, row_bytes) - (unsigned long long)kIntMagicBits * 16u;
+      auto step = [&](int z, bool checked) {
+        const UVH p = project(kf0 + (float)z, kf0 + (float)(z + 1));
+        f32x2_t wg = splat2(bp.scale);
+        if (bp.power == 2) wg = mul2(wg, mul2(p.rh, p.rh));
+        else if (bp.power == 1) wg = mul2(wg, p.rh);
+        float w0, w1, u0 = 0.f, u1 = 0.f, v0 = 0.f, v1 = 0.f;
+        unpack2(wg, w0, w1);
+        f32x2_t uu = p.u, vv = p.v;
+        if (checked) {
+          unpack2(uu, u0, u1);
+          unpack2(vv, v0, v1);
+          if (bp.extent) {
+            auto out = [&](float u, float v) {
+              const float tu = __fadd_rn(u, 0.5f), tv = __fadd_rn(v, 0.5f);
+              return tu < -1.f || tu > bp.nx + 1.f || tv < -1.f || tv > bp.ny + 1.f;
+            };
+            if (out(u0, v0)) w0 = 0.f;
+            if (out(u1, v1)) w1 = 0.f;
+          }
+          uu = f32x2(fminf(fmaxf(u0, -2.f), mu), fminf(fmaxf(u1, -2.f), mu));
+          vv = f32x2(fminf(fmaxf(v0, -2.f), mv), fminf(fmaxf(v1, -2.f), mv));
+        }
+        if constexpr (kMode != kRec) {
+          unpack2(p.u, u0, u1);
+          unpack2(p.v, v0, v1);
+          const float uy[2] = {u0, u1}, vy[2] = {v0, v1};
 #pragma unroll
-      for (int z = 0; z < ZC; ++z) {
-        const float fk = (float)(k0 + z);
-        const float h = fmaf(m10, fk, bh);
-        const float rh = __frcp_rn(h);
-        const float u = __fmul_rn(fmaf(m2, fk, bu), rh);
-        const float v = __fmul_rn(fmaf(m6, fk, bv), rh);
-        const float tu = __fadd_rn(u, 0.5f), tv = __fadd_rn(v, 0.5f);
-        float wgt = bp.scale;
-        if (bp.power == 2) wgt *= rh * rh;
-        else if (bp.power == 1) wgt *= rh;
-        if (bp.extent && (tu < -1.f || tu > bp.nx + 1.f || tv < -1.f || tv > bp.ny + 1.f))
-          wgt = 0.f;
-        float val;
-        if constexpr (kSrc == kSrcTex) val = tex2DLayered<float>(tex, tu, tv, n);
-        else val = smp(u, v);
-        acc[z] = fmaf(val, wgt, acc[z]);
-        if constexpr (kBoth) act[z] = fmaf(tex2DLayered<float>(tex, tu, tv, n), wgt, act[z]);
+          for (int y = 0; y < 2; ++y) {
+            float& a = kMode == kBoth ? act[kMode == kBoth ? z + y : 0] : acc[z + y];
+            a = fmaf(tex2DLayered<float>(tex, __fadd_rn(uy[y], 0.5f), __fadd_rn(vy[y], 0.5f), n0 + jn),
+                     y ? w1 : w0, a);
+          }
+        }
+        if constexpr (kMode != kTex) {
+          const Frac2 fu = frac2(uu), fv = frac2(vv);
+          float tu[2], tv[2], au[2], av[2];
+          unpack2(fu.t, tu[0], tu[1]);
+          unpack2(fv.t, tv[0], tv[1]);
+          unpack2(fu.a, au[0], au[1]);
+          unpack2(fv.a, av[0], av[1]);
+#pragma unroll
+          for (int y = 0; y < 2; ++y) {
+            const float4 r = cell_at(vbase + (unsigned long long)__float_as_uint(tu[y]) * 16u,
+                                     __float_as_uint(tv[y]), row_bytes);
+            acc[z + y] = fmaf(bilinear(r, splat2(au[y]), av[y]), y ? w1 : w0, acc[z + y]);
+          }
+        }
+      };
+      if (inside) {
+#pragma unroll
+        for (int z = 0; z < ZC; z += 2) step(z, false);
+      } else {
+#pragma unroll
+        for (int z = 0; z < ZC; z += 2) step(z, true);
       }
     }
   }
-  if constexpr (split) {
-    // the second half hands its sums to the first: acc = first + second
+  if constexpr (S > 1) {
+    // groups 1 .. S-1 hand their sums to group 0, which adds them in order
     // (dynamic shared memory, given only to split launches)
     extern __shared__ float red[];
-    const int lt = t & 127;
-    if (half == 1) {
+    constexpr int kPer = (kMode == kBoth ? 2 : 1) * ZC;
+    const int lt = t % Shape::kGroup;
+    if (group > 0) {
+      float* r = red + (group - 1) * kPer * Shape::kGroup + lt;
 #pragma unroll
       for (int z = 0; z < ZC; ++z) {
-        red[z * 128 + lt] = acc[z];
-        if constexpr (kBoth) red[(ZC + z) * 128 + lt] = act[z];
+        r[z * Shape::kGroup] = acc[z];
+        if constexpr (kMode == kBoth) r[(ZC + z) * Shape::kGroup] = act[z];
       }
     }
     __syncthreads();
-    if (half == 1 || !valid) return;
+    if (group > 0 || !valid) return;
 #pragma unroll
-    for (int z = 0; z < ZC; ++z) {
-      acc[z] = acc[z] + red[z * 128 + lt];
-      if constexpr (kBoth) act[z] = act[z] + red[(ZC + z) * 128 + lt];
+    for (int g = 0; g < S - 1; ++g) {
+      const float* r = red + g * kPer * Shape::kGroup + lt;
+#pragma unroll
+      for (int z = 0; z < ZC; ++z) {
+        acc[z] = acc[z] + r[z * Shape::kGroup];
+        if constexpr (kMode == kBoth) act[z] = act[z] + r[(ZC + z) * Shape::kGroup];
+      }
     }
   }
   const int64_t plane = (int64_t)bp.nx * bp.ny;
@@ -256,7 +431,7 @@ __device__ __forceinline__ void bp_columns(const BPParams& bp, const Maps& maps,
     if (k < bp.nz) {
       const int64_t e = col + k * plane;
       dst.out[e] = dst.base ? dst.base[e] + acc[z] : acc[z];
-      if constexpr (kBoth) {
+      if constexpr (kMode == kBoth) {
         const float d = acc[z] - act[z];
         dst.diff[e] = dst.diff_base ? dst.diff_base[e] + d : d;
       }
@@ -264,112 +439,120 @@ __device__ __forceinline__ void bp_columns(const BPParams& bp, const Maps& maps,
   }
 }
 
-template <int kSrc, bool kZAff, int ZC, bool kSplit>
-__global__ void __launch_bounds__(kBPThreads) bp_kernel(BPParams bp, const __grid_constant__ BPMaps maps,
+// Unsplit record kernels are held to 48 registers for five blocks per SM: their
+// loads' latency is the bound (256^3 x 64 views: 0.97 -> 0.90 ms).
+template <int kMode, bool kZAff, int S, bool kCull>
+__global__ void __launch_bounds__(kBPThreads, kMode == kRec && kZAff && S == 1 ? 5 : 1) bp_kernel(BPParams bp, const __grid_constant__ BPMaps maps,
                                                         int n0, int n_chunk,
-                                                        const float* __restrict__ spad,
+                                                        const float4* __restrict__ recs,
                                                         cudaTextureObject_t tex, BPOut dst) {
-  bp_columns<kSrc, kZAff, ZC, kSplit>(bp, ParamMaps{&maps}, n0, n_chunk, spad, tex, dst,
-                                      (int)blockIdx.x, (int)blockIdx.y);
+  bp_columns<kMode, kZAff, S, kCull>(bp, ParamMaps{&maps}, n0, n_chunk, recs, tex, dst,
+                                         (int)blockIdx.x, (int)blockIdx.y);
 }
 
-// Records of the exact backprojector: record (U, V) of view n from the four
-// detector values (u, v) = (U - 2 .. U - 1, V - 2 .. V - 1), zero outside the
-// view. Only records that reach the view (U in [1, nu+1], V in [1, nv+1]) are
-// written; the rest keep the plan's initial zeros.
-__global__ void stage_sino_quad_kernel(const float* __restrict__ in, float4* __restrict__ out,
-                                       int nu, int nv, int n_views) {
-  const int U = blockIdx.x * 32 + (threadIdx.x & 31) + 1;
-  const int V = blockIdx.y * 8 + (threadIdx.x >> 5) + 1;
-  const int n = blockIdx.z;
-  if (U > nu + 1 || V > nv + 1 || n >= n_views) return;
-  const float* s = in + (int64_t)n * nu * nv;
-  const int u = U - kPad, v = V - kPad;
-  auto at = [&](int uu, int vv) {
-    return (uu >= 0 && uu < nu && vv >= 0 && vv < nv) ? __ldg(s + (int64_t)vv * nu + uu) : 0.f;
+// Writes the records of a sinogram (all views): record (U, V) of a view from
+// the four detector values (u, v) = (U - 2 .. U - 1, V - 2 .. V - 1), zero
+// outside the view. Only records that reach the view (U in [1, nu+1], V in
+// [1, nv+1]) are written; the rest keep the plan's initial zeros. A warp owns
+// 32 columns of kSinoRows records: each row of the view is loaded once and its
+// right neighbours come from the next lane, so the pass is bound by its
+// 16-byte writes.
+constexpr int kSinoRows = 8;
+__global__ void __launch_bounds__(256) stage_sino_kernel(const float* __restrict__ in,
+                                                         float4* __restrict__ out, int nu, int nv,
+                                                         int64_t warps) {
+  const int lane = threadIdx.x & 31;
+  const int64_t job = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (job >= warps) return;
+  const int tu = (nu + 1 + 31) / 32, tv = (nv + 1 + kSinoRows - 1) / kSinoRows;
+  const int bu = (int)(job % tu);
+  const int64_t r = job / tu;
+  const int V0 = (int)(r % tv) * kSinoRows + 1;
+  const int64_t n = r / tv;
+  const int u = bu * 32 + lane - 1;  // detector column of record U = u + kPad
+  const float* s = in + n * nu * nv;
+  auto row = [&](int v, float& a, float& d) {  // s(u, v) and its difference to the right
+    const bool vin = v >= 0 && v < nv;
+    a = vin && u >= 0 && u < nu ? __ldg(s + (int64_t)v * nu + u) : 0.f;
+    float right = __shfl_down_sync(0xffffffffu, a, 1);
+    if (lane == 31) right = vin && u + 1 < nu ? __ldg(s + (int64_t)v * nu + u + 1) : 0.f;
+    d = right - a;
   };
-  out[(int64_t)n * (nu + 2 * kPad) * (nv + 2 * kPad) + (int64_t)V * (nu + 2 * kPad) + U] =
-      make_float4(at(u, v), at(u + 1, v), at(u, v + 1), at(u + 1, v + 1));
-}
-
-__global__ void stage_sino_pad_kernel(const float* __restrict__ in, float* __restrict__ out, int nu,
-                                      int nv, int64_t n_views_total) {
+  float a[kSinoRows + 1], d[kSinoRows + 1];
+#pragma unroll
+  for (int k = 0; k <= kSinoRows; ++k) row(V0 - kPad + k, a[k], d[k]);
   const int pu = nu + 2 * kPad;
-  const int64_t per = (int64_t)nu * nv, pper = (int64_t)pu * (nv + 2 * kPad);
-  const int64_t total = per * n_views_total;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t n = i / per;
-    const int r = (int)(i - n * per);
-    const int u = r % nu, v = r / nu;
-    out[n * pper + (int64_t)(v + kPad) * pu + u + kPad] = __ldg(in + i);
+  float4* o = out + n * (int64_t)pu * (nv + 2 * kPad) + (int64_t)V0 * pu + u + kPad;
+  if (u > nu - 1) return;
+#pragma unroll
+  for (int k = 0; k < kSinoRows; ++k)
+    if (V0 + k <= nv + 1)
+      o[(int64_t)k * pu] = make_float4(a[k], a[k + 1] - a[k], d[k], d[k + 1] - d[k]);
+}
+
+// View groups per block: the least S of 1, 2, 4, 8 that gives the grid three
+// blocks per SM (8 voxels per thread throughout). A property of the plan's
+// geometry alone, so every launch of the plan sums its views in the same order.
+// 64^3 x 60 views, records: S = 1 47 us, 2 and 4 35 us, 8 37 us; 128^3 x 48
+// views: 126, 122, 128, 143 us.
+constexpr int64_t kBPWantBlocks = 3 * 148;
+constexpr int kBPSplits = 8;
+
+static int bp_tiles(const GeomParams& gp, int S) {
+  const int h = S == 1 ? kBPTile : 8, w = kBPThreads / S / h;
+  return ((gp.nx + w - 1) / w) * ((gp.ny + h - 1) / h);
+}
+static int bp_split(const GeomParams& gp) {
+  int S = 1;
+  while (S < kBPSplits && 2 * S <= gp.n_views &&
+         (int64_t)bp_tiles(gp, S) * ((gp.nz + kZC - 1) / kZC) < kBPWantBlocks)
+    S *= 2;
+  return S;
+}
+static size_t bp_smem(int mode, int S) {
+  return (size_t)(S - 1) * (mode == kBoth ? 2 : 1) * kZC * (kBPThreads / S) * sizeof(float);
+}
+
+struct BPLaunch {
+  dim3 grid;
+  int S;
+  cudaStream_t st;
+};
+
+template <int kMode, bool kZAff, bool kCull>
+static void launch_bp_shape(const BPLaunch& l, const BPParams& bp, const BPMaps& maps, int n0,
+                            int cnt, const float4* recs, cudaTextureObject_t tex,
+                            const BPOut& dst) {
+  const size_t sm = bp_smem(kMode, l.S);
+  if (l.S == 8)
+    bp_kernel<kMode, kZAff, 8, kCull><<<l.grid, kBPThreads, sm, l.st>>>(bp, maps, n0, cnt, recs, tex, dst);
+  else if (l.S == 4)
+    bp_kernel<kMode, kZAff, 4, kCull><<<l.grid, kBPThreads, sm, l.st>>>(bp, maps, n0, cnt, recs, tex, dst);
+  else if (l.S == 2)
+    bp_kernel<kMode, kZAff, 2, kCull><<<l.grid, kBPThreads, sm, l.st>>>(bp, maps, n0, cnt, recs, tex, dst);
+  else
+    bp_kernel<kMode, kZAff, 1, kCull><<<l.grid, kBPThreads, sm, l.st>>>(bp, maps, n0, cnt, recs, tex, dst);
+}
+
+template <int kMode>
+static void launch_bp_mode(const BPLaunch& l, bool zaff, const BPParams& bp, const BPMaps& maps,
+                           int n0, int cnt, const float4* recs, cudaTextureObject_t tex,
+                           const BPOut& dst) {
+  if (bp.cull) {
+    if (zaff) launch_bp_shape<kMode, true, true>(l, bp, maps, n0, cnt, recs, tex, dst);
+    else launch_bp_shape<kMode, false, true>(l, bp, maps, n0, cnt, recs, tex, dst);
+  } else {
+    if (zaff) launch_bp_shape<kMode, true, false>(l, bp, maps, n0, cnt, recs, tex, dst);
+    else launch_bp_shape<kMode, false, false>(l, bp, maps, n0, cnt, recs, tex, dst);
   }
 }
 
-// Voxels per thread along z: the largest of 8, 4, 2 whose grid has
-// kBPWantBlocks blocks (2 if none has).
-template <class BlocksFor>
-static int bp_zc(BlocksFor blocks_for) {
-  for (int c = kZCMax; c > 2; c /= 2)
-    if (blocks_for(c) >= kBPWantBlocks) return c;
-  return 2;
-}
-
-template <int kSrc, bool kZAff, bool kSplit>
-static void launch_bp_split(int zc, dim3 grid, cudaStream_t st, const BPParams& bp,
-                            const BPMaps& maps, int n0, int cnt, const float* sp,
-                            cudaTextureObject_t tx, const BPOut& dst) {
-  // split launches: the second half's sums of each voxel in shared memory
-  const size_t sm = kSplit ? (size_t)(kSrc == kSrcBoth ? 2 : 1) * zc * 128 * sizeof(float) : 0;
-  if (zc == 8)
-    bp_kernel<kSrc, kZAff, 8, kSplit><<<grid, kBPThreads, sm, st>>>(bp, maps, n0, cnt, sp, tx, dst);
-  else if (zc == 4)
-    bp_kernel<kSrc, kZAff, 4, kSplit><<<grid, kBPThreads, sm, st>>>(bp, maps, n0, cnt, sp, tx, dst);
-  else
-    bp_kernel<kSrc, kZAff, 2, kSplit><<<grid, kBPThreads, sm, st>>>(bp, maps, n0, cnt, sp, tx, dst);
-}
-
-template <int kSrc, bool kZAff>
-static void launch_bp_zc(int zc, dim3 grid, cudaStream_t st, const BPParams& bp,
-                         const BPMaps& maps, int n0, int cnt, const float* sp,
-                         cudaTextureObject_t tx, const BPOut& dst) {
-  if (bp.vsplit == 2)
-    launch_bp_split<kSrc, kZAff, true>(zc, grid, st, bp, maps, n0, cnt, sp, tx, dst);
-  else
-    launch_bp_split<kSrc, kZAff, false>(zc, grid, st, bp, maps, n0, cnt, sp, tx, dst);
-}
-
-template <int kSrc>
-static void launch_bp_src(bool zaff, int zc, dim3 grid, cudaStream_t st, const BPParams& bp,
-                          const BPMaps& maps, int n0, int cnt, const float* sp,
-                          cudaTextureObject_t tx, const BPOut& dst) {
-  if (zaff) launch_bp_zc<kSrc, true>(zc, grid, st, bp, maps, n0, cnt, sp, tx, dst);
-  else launch_bp_zc<kSrc, false>(zc, grid, st, bp, maps, n0, cnt, sp, tx, dst);
-}
-
-static void launch_bp(int src, bool zaff, int zc, dim3 grid, cudaStream_t st, const BPParams& bp,
-                      const BPMaps& maps, int n0, int cnt, const float* sp, cudaTextureObject_t tx,
-                      const BPOut& dst) {
-  switch (src) {
-    case kSrcTex: launch_bp_src<kSrcTex>(zaff, zc, grid, st, bp, maps, n0, cnt, sp, tx, dst); break;
-    case kSrcQuad: launch_bp_src<kSrcQuad>(zaff, zc, grid, st, bp, maps, n0, cnt, sp, tx, dst); break;
-    case kSrcBoth: launch_bp_src<kSrcBoth>(zaff, zc, grid, st, bp, maps, n0, cnt, sp, tx, dst); break;
-    default: launch_bp_src<kSrcSoft>(zaff, zc, grid, st, bp, maps, n0, cnt, sp, tx, dst); break;
-  }
-}
-
-// Column tiles of 16 x 16, or of 16 x 8 where the plan splits its views.
-static int bp_tiles(const GeomParams& gp, int vsplit) {
-  const int th = vsplit == 2 ? kBPTile / 2 : kBPTile;
-  return ((gp.nx + kBPTile - 1) / kBPTile) * ((gp.ny + th - 1) / th);
-}
-
-// A volume whose 16 x 16 column tiles cannot give four blocks per SM even with
-// two slices per thread splits its views between two halves of each block
-// (twice the blocks, half the views each). A property of the plan's geometry
-// alone, so every launch of the plan sums its views in the same order.
-static int bp_vsplit(const GeomParams& gp) {
-  return gp.n_views >= 2 && (int64_t)bp_tiles(gp, 1) * ((gp.nz + 1) / 2) < kBPWantBlocks ? 2 : 1;
+static void launch_bp(int mode, const BPLaunch& l, bool zaff, const BPParams& bp,
+                      const BPMaps& maps, int n0, int cnt, const float4* recs,
+                      cudaTextureObject_t tex, const BPOut& dst) {
+  if (mode == kTex) launch_bp_mode<kTex>(l, zaff, bp, maps, n0, cnt, recs, tex, dst);
+  else if (mode == kBoth) launch_bp_mode<kBoth>(l, zaff, bp, maps, n0, cnt, recs, tex, dst);
+  else launch_bp_mode<kRec>(l, zaff, bp, maps, n0, cnt, recs, tex, dst);
 }
 
 static BPParams plan_bp_params(const Plan* p) {
@@ -380,14 +563,14 @@ static BPParams plan_bp_params(const Plan* p) {
   bp.power = gp.bp_power;
   bp.extent = gp.bp_extent;
   bp.scale = (float)gp.bp_scale;
-  bp.sino_pad_elems = (int64_t)(gp.nu + 2 * kPad) * (gp.nv + 2 * kPad);
+  bp.view_recs = (int64_t)(gp.nu + 2 * kPad) * (gp.nv + 2 * kPad);
   bp.warp = p->bp_warp;
-  bp.vsplit = bp_vsplit(gp);
+  bp.cull = p->bp_cull;
   return bp;
 }
 
 // Copies one batch item's sinogram into the plan's staged form: the layered
-// texture (texture plans), the quad records (exact plans) or the padded array.
+// texture (texture plans) or the records.
 static int stage_sino(Plan* p, const float* sino, cudaStream_t st) {
   const GeomParams& gp = p->gp;
   if (p->sino_tex != nullptr) {
@@ -398,45 +581,65 @@ static int stage_sino(Plan* p, const float* sino, cudaStream_t st) {
     cp.extent = make_cudaExtent(gp.nu, gp.nv, gp.n_views);
     cp.kind = cudaMemcpyDeviceToDevice;
     DTV_CUDA_TRY(cudaMemcpy3DAsync(&cp, st));
-  } else if (p->d_sino_quad != nullptr) {
-    dim3 qg((gp.nu + 1 + 31) / 32, (gp.nv + 1 + 7) / 8, gp.n_views);
-    stage_sino_quad_kernel<<<qg, 256, 0, st>>>(sino, p->d_sino_quad, gp.nu, gp.nv, gp.n_views);
-    note_launch();
-    DTV_LAUNCH_CHECK();
-  } else {
-    const int64_t per_item = (int64_t)gp.nu * gp.nv * gp.n_views;
-    stage_sino_pad_kernel<<<(int)std::min<int64_t>((per_item + 255) / 256, 148 * 16), 256, 0,
-                            st>>>(sino, p->d_sino_pad, gp.nu, gp.nv, gp.n_views);
-    note_launch();
-    DTV_LAUNCH_CHECK();
+    return DTV_OK;
   }
+  const int64_t warps = (int64_t)((gp.nu + 1 + 31) / 32) *
+                        ((gp.nv + 1 + kSinoRows - 1) / kSinoRows) * gp.n_views;
+  const int64_t blocks = (warps + 7) / 8;
+  DTV_CHECK(blocks < 2147483647LL, "sinogram too large for one staging launch");
+  stage_sino_kernel<<<(unsigned)blocks, 256, 0, st>>>(sino, p->d_sino_rec, gp.nu, gp.nv, warps);
+  note_launch();
+  DTV_LAUNCH_CHECK();
   return DTV_OK;
 }
 
-static dim3 bp_grid(const GeomParams& gp, int* zc_out) {
-  const int tiles = bp_tiles(gp, bp_vsplit(gp));
-  const int zc = bp_zc([&](int c) { return (int64_t)tiles * ((gp.nz + c - 1) / c); });
-  *zc_out = zc;
-  return dim3(tiles, (gp.nz + zc - 1) / zc);
+// Whether most (block, view) pairs miss the detector, over a sample of the
+// plan's blocks and views: then the blocks look for the views they meet first.
+// Of many-module scans, whose modules each see a slice of the fan, most pairs
+// go; where few do the test costs more than it saves (a circular scan whose
+// detector misses the volume's corners: 0.84 -> 0.86 ms through the texture
+// unit, 0.97 -> 1.14 ms through records), and a thread's own end tests skip
+// its views beside the detector anyway.
+int bp_cull_rule(const Plan* p) {
+  const GeomParams& gp = p->gp;
+  int missed = 0, total = 0;
+  const int vs = std::max(1, gp.n_views / 48);
+  for (int n = 0; n < gp.n_views; n += vs)
+    for (int c = 0; c < 18; ++c) {
+      const int n3[3] = {gp.nx, gp.ny, gp.nz}, e[3] = {kBPTile, kBPTile, kZC};
+      const int g3[3] = {c % 3, c / 3 % 3, c / 9};
+      float lo[3], hi[3];
+      for (int a = 0; a < 3; ++a) {
+        const int blocks = (n3[a] + e[a] - 1) / e[a];
+        const int b = (blocks - 1) * g3[a] / (a == 2 ? 1 : 2);
+        lo[a] = (float)(b * e[a]);
+        hi[a] = (float)(b * e[a] + e[a] - 1);
+      }
+      missed += !box_seen(p->h_bpv[n].m, lo[0], hi[0], lo[1], hi[1], lo[2], hi[2], (float)gp.nu,
+                          (float)gp.nv);
+      ++total;
+    }
+  return missed * 2 >= total ? 1 : 0;
 }
 
 // The views in chunks of kBPParamViews (their maps travel in the launch
 // parameters); later chunks add onto the first one's result.
-static int bp_view_chunks(const Plan* p, int src, const float* sp, cudaTextureObject_t tx,
-                          BPOut dst, cudaStream_t st) {
+static int bp_view_chunks(const Plan* p, int mode, const float4* recs, BPOut dst,
+                          cudaStream_t st) {
   const GeomParams& gp = p->gp;
   const BPParams bp = plan_bp_params(p);
-  int zc;
-  const dim3 grid = bp_grid(gp, &zc);
+  const cudaTextureObject_t tex = p->sino_tex ? p->sino_tex[0] : 0;
+  const int S = bp_split(gp);
+  const BPLaunch l{dim3(bp_tiles(gp, S), (gp.nz + kZC - 1) / kZC), S, st};
   BPMaps maps;
   for (int n0 = 0; n0 < gp.n_views; n0 += kBPParamViews) {
     const int cnt = std::min(kBPParamViews, gp.n_views - n0);
     for (int j = 0; j < cnt; ++j) memcpy(maps.m[j], p->h_bpv[n0 + j].m, sizeof(maps.m[j]));
     if (n0 > 0) {
       dst.base = dst.out;
-      dst.diff_base = dst.diff;
+      dst.diff_base = dst.diff;  // (kBoth only)
     }
-    launch_bp(src, p->bp_zaffine != 0, zc, grid, st, bp, maps, n0, cnt, sp, tx, dst);
+    launch_bp(mode, l, p->bp_zaffine != 0, bp, maps, n0, cnt, recs, tex, dst);
     note_launch();
     DTV_LAUNCH_CHECK();
   }
@@ -446,19 +649,13 @@ static int bp_view_chunks(const Plan* p, int src, const float* sp, cudaTextureOb
 int backward_impl(Plan* p, const float* sino, int batch, const float* base, float* out,
                   cudaStream_t st) {
   const GeomParams& gp = p->gp;
-  const bool tex = p->sino_tex != nullptr;      // allocated for the texture plans
-  const bool quad = p->d_sino_quad != nullptr;  // the exact plans
   const int64_t per_item = (int64_t)gp.nu * gp.nv * gp.n_views;
   const int64_t vox = (int64_t)gp.nx * gp.ny * gp.nz;
   for (int b = 0; b < batch; ++b) {
     int rc = stage_sino(p, sino + b * per_item, st);
     if (rc) return rc;
-    const cudaTextureObject_t tx = tex ? p->sino_tex[0] : 0;
-    const float* sp = tex ? nullptr
-                          : quad ? reinterpret_cast<const float*>(p->d_sino_quad) : p->d_sino_pad;
-    const int src = tex ? kSrcTex : quad ? kSrcQuad : kSrcSoft;
-    rc = bp_view_chunks(p, src, sp, tx, BPOut{out + b * vox, base ? base + b * vox : nullptr,
-                                              nullptr, nullptr}, st);
+    rc = bp_view_chunks(p, p->sino_tex ? kTex : kRec, p->d_sino_rec,
+                        BPOut{out + b * vox, base ? base + b * vox : nullptr, nullptr, nullptr}, st);
     if (rc) return rc;
   }
   return DTV_OK;
@@ -473,14 +670,15 @@ int backward_refresh_impl(Plan* fast, Plan* exact, const float* sino, int batch,
   const int64_t per_item = (int64_t)gp.nu * gp.nv * gp.n_views;
   const int64_t vox = (int64_t)gp.nx * gp.ny * gp.nz;
   for (int b = 0; b < batch; ++b) {
-    int rc = stage_sino(fast, sino + b * per_item, st);
+    int rc = stage_sino(exact, sino + b * per_item, st);
     if (rc) return rc;
-    rc = stage_sino(exact, sino + b * per_item, st);
+    // beyond a layered texture's views the fast plan samples records too: no difference
+    const bool both = fast->sino_tex != nullptr;
+    if (both && (rc = stage_sino(fast, sino + b * per_item, st))) return rc;
+    const BPOut dst{out + b * vox, nullptr, both ? e_b + b * vox : nullptr, nullptr};
+    rc = bp_view_chunks(fast, both ? kBoth : kRec, exact->d_sino_rec, dst, st);
     if (rc) return rc;
-    rc = bp_view_chunks(fast, kSrcBoth, reinterpret_cast<const float*>(exact->d_sino_quad),
-                        fast->sino_tex[0], BPOut{out + b * vox, nullptr, e_b + b * vox, nullptr},
-                        st);
-    if (rc) return rc;
+    if (!both) DTV_CUDA_TRY(cudaMemsetAsync(e_b + b * vox, 0, vox * sizeof(float), st));
   }
   return DTV_OK;
 }
@@ -490,11 +688,9 @@ int backward_refresh_impl(Plan* fast, Plan* exact, const float* sino, int batch,
 // its plan by the blocks' prefix offsets (kernel parameters, read uniformly).
 // The plans' maps travel in the launch parameters too, up to kBPManyViews
 // views per launch, so they are read through the constant cache as in the
-// single-plan launch (maps read from device memory go through the same L1
-// path as the texture fetches: 14% slower on 16 volumes of 96^3-256^3). A
-// plan with more views than that reads its maps from its device table.
-// Texture plans only; each item's sinogram is first copied into its plan's
-// layered array.
+// single-plan launch. A plan with more views than that reads its maps from its
+// device table. Texture plans only; each item's sinogram is first copied into
+// its plan's layered array.
 constexpr int kBPManyViews = 560;
 struct BPManyItem {
   BPParams bp;
@@ -519,8 +715,8 @@ struct RowMaps {
   __device__ __forceinline__ const float* row(int jn) const { return r[jn]; }
 };
 
-// Every item of one launch has the same bp.vsplit (kSplit).
-template <int ZC, bool kSplit>
+// Every item of one launch has the same S.
+template <int S>
 __global__ void __launch_bounds__(kBPThreads) bp_many_kernel(const __grid_constant__ BPMany m,
                                                              int accumulate) {
   int k = 0;
@@ -529,72 +725,54 @@ __global__ void __launch_bounds__(kBPThreads) bp_many_kernel(const __grid_consta
   const int local = (int)blockIdx.x - it.block0;
   const int tile = local % it.tiles, zc = local / it.tiles;
   const BPOut dst{it.out, accumulate ? it.out : nullptr, nullptr, nullptr};
+  const int nv = it.bp.n_views;
   if (it.map0 >= 0) {
     const RowMaps rows{m.m + it.map0};
-    if (it.zaffine)
-      bp_columns<kSrcTex, true, ZC, kSplit>(it.bp, rows, 0, it.bp.n_views, nullptr, it.tex, dst, tile, zc);
-    else
-      bp_columns<kSrcTex, false, ZC, kSplit>(it.bp, rows, 0, it.bp.n_views, nullptr, it.tex, dst, tile, zc);
-  } else if (it.zaffine) {
-    bp_columns<kSrcTex, true, ZC, kSplit>(it.bp, TableMaps{it.views}, 0, it.bp.n_views, nullptr, it.tex,
-                                  dst, tile, zc);
+    if (it.zaffine) bp_columns<kTex, true, S, false>(it.bp, rows, 0, nv, nullptr, it.tex, dst, tile, zc);
+    else bp_columns<kTex, false, S, false>(it.bp, rows, 0, nv, nullptr, it.tex, dst, tile, zc);
   } else {
-    bp_columns<kSrcTex, false, ZC, kSplit>(it.bp, TableMaps{it.views}, 0, it.bp.n_views, nullptr, it.tex,
-                                   dst, tile, zc);
+    const TableMaps rows{it.views};
+    if (it.zaffine) bp_columns<kTex, true, S, false>(it.bp, rows, 0, nv, nullptr, it.tex, dst, tile, zc);
+    else bp_columns<kTex, false, S, false>(it.bp, rows, 0, nv, nullptr, it.tex, dst, tile, zc);
   }
 }
 
 int backward_many_impl(Plan* const* plans, const float* const* sinos, float* const* outs, int count,
                        int accumulate, cudaStream_t st) {
   BPMany m;
-  // plans that split their views run in launches of their own
+  // plans of one view split share launches
   std::vector<int> ord;
-  for (int split = 1; split <= 2; ++split)
+  for (int S = 1; S <= kBPSplits; S *= 2)
     for (int k = 0; k < count; ++k)
-      if (bp_vsplit(plans[k]->gp) == split) ord.push_back(k);
+      if (bp_split(plans[k]->gp) == S) ord.push_back(k);
   int c0 = 0;
   while (c0 < count) {
     // this launch's plans: up to kManyItems of one split kind, whose maps fit
     // the parameters (a plan with more views than fit at all takes its maps
     // from its table)
-    const int kind = bp_vsplit(plans[ord[c0]]->gp);
+    const int S = bp_split(plans[ord[c0]]->gp);
     int cnt = 0, rows = 0;
     while (c0 + cnt < count && cnt < kManyItems) {
       const GeomParams& g = plans[ord[c0 + cnt]]->gp;
-      if (bp_vsplit(g) != kind) break;
+      if (bp_split(g) != S) break;
       const int nv = g.n_views;
       if (nv <= kBPManyViews && rows + nv > kBPManyViews) break;
       if (nv <= kBPManyViews) rows += nv;
       ++cnt;
     }
-    // one z-chunk length for the whole launch, from its total column tiles
-    const int zc = bp_zc([&](int c) {
-      int64_t b = 0;
-      for (int k = 0; k < cnt; ++k) {
-        const GeomParams& gp = plans[ord[c0 + k]]->gp;
-        b += (int64_t)bp_tiles(gp, bp_vsplit(gp)) * ((gp.nz + c - 1) / c);
-      }
-      return b;
-    });
     int64_t blocks = 0;
     int row = 0;
     for (int k = 0; k < cnt; ++k) {
       Plan* p = plans[ord[c0 + k]];
       const GeomParams& gp = p->gp;
-      cudaMemcpy3DParms cp;
-      memset(&cp, 0, sizeof(cp));
-      cp.srcPtr = make_cudaPitchedPtr((void*)sinos[ord[c0 + k]], gp.nu * sizeof(float), gp.nu, gp.nv);
-      cp.dstArray = p->sino_arrays[0];
-      cp.extent = make_cudaExtent(gp.nu, gp.nv, gp.n_views);
-      cp.kind = cudaMemcpyDeviceToDevice;
-      DTV_CUDA_TRY(cudaMemcpy3DAsync(&cp, st));
+      const int rc = stage_sino(p, sinos[ord[c0 + k]], st);
+      if (rc) return rc;
       BPManyItem& it = m.it[k];
       it.bp = plan_bp_params(p);
-      it.bp.sino_pad_elems = 0;
       it.views = p->d_bpv;
       it.tex = p->sino_tex[0];
       it.out = outs[ord[c0 + k]];
-      it.tiles = bp_tiles(gp, it.bp.vsplit);
+      it.tiles = bp_tiles(gp, S);
       it.block0 = (int)blocks;
       it.zaffine = p->bp_zaffine;
       it.map0 = -1;
@@ -603,21 +781,16 @@ int backward_many_impl(Plan* const* plans, const float* const* sinos, float* con
         for (int j = 0; j < gp.n_views; ++j) memcpy(m.m[row + j], p->h_bpv[j].m, sizeof(m.m[0]));
         row += gp.n_views;
       }
-      blocks += (int64_t)it.tiles * ((gp.nz + zc - 1) / zc);
+      blocks += (int64_t)it.tiles * ((gp.nz + kZC - 1) / kZC);
     }
     DTV_CHECK(blocks < 2147483647LL, "too many blocks for one launch");
     m.count = cnt;
     const unsigned nb = (unsigned)blocks;
-    if (kind == 2) {
-      const size_t sm = (size_t)zc * 128 * sizeof(float);
-      if (zc == 8) bp_many_kernel<8, true><<<nb, kBPThreads, sm, st>>>(m, accumulate);
-      else if (zc == 4) bp_many_kernel<4, true><<<nb, kBPThreads, sm, st>>>(m, accumulate);
-      else bp_many_kernel<2, true><<<nb, kBPThreads, sm, st>>>(m, accumulate);
-    } else {
-      if (zc == 8) bp_many_kernel<8, false><<<nb, kBPThreads, 0, st>>>(m, accumulate);
-      else if (zc == 4) bp_many_kernel<4, false><<<nb, kBPThreads, 0, st>>>(m, accumulate);
-      else bp_many_kernel<2, false><<<nb, kBPThreads, 0, st>>>(m, accumulate);
-    }
+    const size_t sm = bp_smem(kTex, S);
+    if (S == 8) bp_many_kernel<8><<<nb, kBPThreads, sm, st>>>(m, accumulate);
+    else if (S == 4) bp_many_kernel<4><<<nb, kBPThreads, sm, st>>>(m, accumulate);
+    else if (S == 2) bp_many_kernel<2><<<nb, kBPThreads, sm, st>>>(m, accumulate);
+    else bp_many_kernel<1><<<nb, kBPThreads, sm, st>>>(m, accumulate);
     note_launch();
     DTV_LAUNCH_CHECK();
     c0 += cnt;

@@ -65,6 +65,51 @@ __device__ __forceinline__ __half2 u32_as_half2(unsigned int w) {
                         __ushort_as_half((unsigned short)(w >> 16)));
 }
 
+// Packed FP32 pairs (Blackwell's two-lane FP32 arithmetic); each lane rounds as
+// the scalar instruction does.
+using f32x2_t = unsigned long long;
+__device__ __forceinline__ f32x2_t f32x2(float lo, float hi) {
+  f32x2_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ f32x2_t splat2(float v) { return f32x2(v, v); }
+__device__ __forceinline__ void unpack2(f32x2_t v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ f32x2_t add2(f32x2_t a, f32x2_t b) {
+  f32x2_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2_t add2_rm(f32x2_t a, f32x2_t b) {  // rounding down
+  f32x2_t r;
+  asm("add.rm.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2_t sub2(f32x2_t a, f32x2_t b) {
+  f32x2_t r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2_t mul2(f32x2_t a, f32x2_t b) {
+  f32x2_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2_t fma2(f32x2_t a, f32x2_t b, f32x2_t c) {
+  f32x2_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+// 1 / x by one Newton step r + r (1 - x r) on the approximate reciprocal.
+__device__ __forceinline__ float rcp_newton(float x) {
+  float r;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return fmaf(r, fmaf(-x, r, 1.f), r);
+}
+
 // Zero border of the exact sampler's records (texels on each side in x and y,
 // layers in z). The ray set-up keeps every sample within one step of (-1, n)
 // on each axis, so its cell corner lies in [-2, n] and a border of 3 leaves a
@@ -129,18 +174,17 @@ struct Plan {
   float4* d_vol_quads;
   int stage_dtype;    // DTV_F32 or DTV_F16
   int64_t pad_elems;  // elements of one padded volume
-  // soft bilinear staging: zero-padded sinogram of one batch item
-  float* d_sino_pad;
-  // exact plans: 16-byte records (2x2 detector values) of the padded sinogram
-  float4* d_sino_quad;
-  // texture sampler (DTV_PLAN_TEX): one 3-D array per batch item for the
-  // volume, one layered array for a sinogram
+  // backprojector: the sinogram of one batch item as 16-byte records (one
+  // bilinear detector cell each) or, texture plans, a layered array
+  float4* d_sino_rec;
+  cudaArray_t* sino_arrays;
+  cudaTextureObject_t* sino_tex;
+  int bp_cull;  // its blocks look for the views they meet first
+  // texture sampler (DTV_PLAN_TEX): one 3-D array per batch item
   cudaArray_t* vol_arrays;
   cudaTextureObject_t* vol_tex;      // host copy
   cudaTextureObject_t* vol_tex_dev;  // device copy (kernel argument)
   cudaSurfaceObject_t* vol_surf;     // staging writes into vol_arrays
-  cudaArray_t* sino_arrays;
-  cudaTextureObject_t* sino_tex;
   // z-pair sampler (DTV_PLAN_TEX_PAIRS): one layered half2 array per batch item
   cudaArray_t* pair_arrays;
   cudaTextureObject_t* pair_tex;
@@ -192,6 +236,7 @@ int forward_refresh_impl(Plan* fast, Plan* exact, const void* vol, int vol_dtype
                          cudaStream_t st);
 int backward_refresh_impl(Plan* fast, Plan* exact, const float* sino, int batch, float* out,
                           float* e_b, cudaStream_t st);
+int bp_cull_rule(const Plan* p);
 int adjoint_impl(Plan* p, const float* sino, int batch, float* out, cudaStream_t st);
 int encode_pair_maps(Plan* p);
 // several plans' projections in one launch (forward.cu, backward.cu)

@@ -69,13 +69,8 @@ struct QuadSampler {
   }
 };
 
-// Packed FP32 pairs (Blackwell's two-lane FP32 arithmetic): the z-pair
-// samplers interpolate both planes of a cell in one instruction.
-__device__ __forceinline__ unsigned long long f32x2(float lo, float hi) {
-  unsigned long long r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
+// a + w (b - a) per lane: the z-pair samplers interpolate both planes of a cell
+// in one instruction.
 __device__ __forceinline__ unsigned long long f32x2_lerp(unsigned long long w,
                                                          unsigned long long a,
                                                          unsigned long long b) {

@@ -63,8 +63,7 @@ void free_plan(Plan* p) {
   free(p->h_bpv);
   cudaFree(p->d_vol_pad);
   cudaFree(p->d_vol_quads);
-  cudaFree(p->d_sino_pad);
-  cudaFree(p->d_sino_quad);
+  cudaFree(p->d_sino_rec);
   delete p;
 }
 
@@ -197,13 +196,7 @@ int create_plan(const dtv_geometry* g, int max_batch, int flags, int device, Pla
       PLAN_CUDA(cudaMemset(p->d_vol_pad, 0, esz * p->pad_elems * max_batch));
     }
   }
-  const int64_t sino_pad = (int64_t)(gp.nu + 2 * kPad) * (gp.nv + 2 * kPad) * gp.n_views;
-  PLAN_CUDA(cudaMalloc(&p->d_sino_pad, sizeof(float) * sino_pad));
-  PLAN_CUDA(cudaMemset(p->d_sino_pad, 0, sizeof(float) * sino_pad));
-  if (flags & DTV_PLAN_PAIRS_EXACT) {
-    PLAN_CUDA(cudaMalloc(&p->d_sino_quad, sizeof(float4) * sino_pad));
-    PLAN_CUDA(cudaMemset(p->d_sino_quad, 0, sizeof(float4) * sino_pad));
-  }
+  p->bp_cull = bp_cull_rule(p);
 
   if (flags & DTV_PLAN_TEX) {
     p->vol_arrays = (cudaArray_t*)calloc(max_batch, sizeof(cudaArray_t));
@@ -285,7 +278,7 @@ int create_plan(const dtv_geometry* g, int max_batch, int flags, int device, Pla
   }
   if ((flags & (DTV_PLAN_TEX | DTV_PLAN_TEX_PAIRS)) && gp.n_views <= max_layers) {
     // backprojector: the sinogram as a layered texture (one layer per view);
-    // with more views than layers the backprojector samples in software
+    // with more views than layers the backprojector samples records
     p->sino_arrays = (cudaArray_t*)calloc(1, sizeof(cudaArray_t));
     p->sino_tex = (cudaTextureObject_t*)calloc(1, sizeof(cudaTextureObject_t));
     if (!p->sino_arrays || !p->sino_tex) {
@@ -300,6 +293,11 @@ int create_plan(const dtv_geometry* g, int max_batch, int flags, int device, Pla
       free_plan(p);
       return rc;
     }
+  } else {
+    // records: zero borders written once here, those that reach the view by each call
+    const int64_t recs = (int64_t)(gp.nu + 2 * kPad) * (gp.nv + 2 * kPad) * gp.n_views;
+    PLAN_CUDA(cudaMalloc(&p->d_sino_rec, sizeof(float4) * recs));
+    PLAN_CUDA(cudaMemset(p->d_sino_rec, 0, sizeof(float4) * recs));
   }
   if (flags & DTV_PLAN_ADJOINT) {
     const size_t n = (size_t)gp.n_views * gp.nu * gp.nv * 2;
