@@ -110,12 +110,6 @@ __device__ __forceinline__ float rcp_newton(float x) {
   return fmaf(r, fmaf(-x, r, 1.f), r);
 }
 
-// Zero border of the exact sampler's records (texels on each side in x and y,
-// layers in z). The ray set-up keeps every sample within one step of (-1, n)
-// on each axis, so its cell corner lies in [-2, n] and a border of 3 leaves a
-// whole texel of slack for the FP32 rounding of the sample positions.
-constexpr int kQuadPad = 3;
-
 inline int dtype_size(int dt) { return dt == DTV_F32 ? 4 : 2; }
 inline bool dtype_ok(int dt) { return dt == DTV_F32 || dt == DTV_F16 || dt == DTV_BF16; }
 
@@ -167,11 +161,11 @@ struct Plan {
   FPView* d_fpv;  // device
   BPView* d_bpv;  // device
   BPView* h_bpv;  // host copy (the backprojector passes the maps as launch parameters)
-  // soft sampler staging: zero-padded volumes (border kPad) of max_batch items
+  // FP16-staged soft plans: zero-padded volumes (border kPad) of max_batch items
   void* d_vol_pad;
-  // FP32 soft plans: quad records (x..x+1, y..y+1 of one plane) over the same
-  // padded grid, read by the forward projector instead of d_vol_pad
-  float4* d_vol_quads;
+  // FP32 soft and exact plans: 16-byte records of the x/y cells, z fastest, over
+  // the same padded grid (forward.cu RecSampler), read instead of d_vol_pad
+  float4* d_vol_rec;
   int stage_dtype;    // DTV_F32 or DTV_F16
   int64_t pad_elems;  // elements of one padded volume
   // backprojector: the sinogram of one batch item as 16-byte records (one
@@ -198,12 +192,6 @@ struct Plan {
   // (boxes for chunks along x and along y)
   unsigned int* d_pair_lin;
   int pair_pitch;
-  // exact z-pair sampler (DTV_PLAN_PAIRS_EXACT): per batch item, 16-byte
-  // records [L][Y][X] of the four x/y corner words of a z-pair cell, over the
-  // grid padded by kQuadPad zero texels on every side (X = x + 3, Y = y + 3,
-  // L = floor(z) + 3 holds (f[L-3], f[L-2]))
-  uint4* d_pair_quad;
-  int64_t pair_quad_elems;  // records per batch item
   int fp_tex_share;          // DTV_TUNE_FP_TEX_SHARE
   alignas(64) unsigned char tmap[2][128];
   int* d_status;             // device error bits

@@ -56,13 +56,12 @@ void free_plan(Plan* p) {
   cudaFree(p->d_rays);
   cudaFree(p->d_cells);
   cudaFree(p->d_pair_lin);
-  cudaFree(p->d_pair_quad);
   cudaFree(p->d_status);
   cudaFree(p->d_fpv);
   cudaFree(p->d_bpv);
   free(p->h_bpv);
   cudaFree(p->d_vol_pad);
-  cudaFree(p->d_vol_quads);
+  cudaFree(p->d_vol_rec);
   cudaFree(p->d_sino_rec);
   delete p;
 }
@@ -174,26 +173,22 @@ int create_plan(const dtv_geometry* g, int max_batch, int flags, int device, Pla
 
   p->stage_dtype = (flags & DTV_PLAN_STAGE_F16) ? DTV_F16 : DTV_F32;
   p->pad_elems = (int64_t)(gp.nx + 2 * kPad) * (gp.ny + 2 * kPad) * (gp.nz + 2 * kPad);
-  const size_t esz = p->stage_dtype == DTV_F16 ? 2 : 4;
-  // Staged volumes of the software sampler (FP32: quad records, FP16: the
+  // Staged volumes of the software samplers (16-byte records; FP16-staged: the
   // padded volume): zero border written once here, interiors by each call.
   if (flags & DTV_PLAN_PAIRS_EXACT) {
-    p->pair_quad_elems = (int64_t)(gp.nx + 2 * kQuadPad) * (gp.ny + 2 * kQuadPad) *
-                         (gp.nz + 2 * kQuadPad - 1);
-    if (p->pair_quad_elems >= (1LL << 31)) {
+    const int64_t most = (int64_t)(gp.nx + 6) * (gp.ny + 6) * (gp.nz + 5);
+    if (most >= (1LL << 31)) {
       free_plan(p);
       return fail(DTV_ERR_UNSUPPORTED, "volume too large for DTV_PLAN_PAIRS_EXACT");
     }
-    const size_t bytes = sizeof(uint4) * p->pair_quad_elems * max_batch;
-    PLAN_CUDA(cudaMalloc(&p->d_pair_quad, bytes));
-    PLAN_CUDA(cudaMemset(p->d_pair_quad, 0, bytes));  // records beyond the volume stay zero
-  } else if (!(flags & (DTV_PLAN_TEX | DTV_PLAN_TEX_PAIRS))) {
-    if (p->stage_dtype == DTV_F32) {
-      PLAN_CUDA(cudaMalloc(&p->d_vol_quads, sizeof(float4) * p->pad_elems * max_batch));
-      PLAN_CUDA(cudaMemset(p->d_vol_quads, 0, sizeof(float4) * p->pad_elems * max_batch));
+  }
+  if (!(flags & (DTV_PLAN_TEX | DTV_PLAN_TEX_PAIRS))) {
+    if (p->stage_dtype == DTV_F32 || (flags & DTV_PLAN_PAIRS_EXACT)) {
+      PLAN_CUDA(cudaMalloc(&p->d_vol_rec, sizeof(float4) * p->pad_elems * max_batch));
+      PLAN_CUDA(cudaMemset(p->d_vol_rec, 0, sizeof(float4) * p->pad_elems * max_batch));
     } else {
-      PLAN_CUDA(cudaMalloc(&p->d_vol_pad, esz * p->pad_elems * max_batch));
-      PLAN_CUDA(cudaMemset(p->d_vol_pad, 0, esz * p->pad_elems * max_batch));
+      PLAN_CUDA(cudaMalloc(&p->d_vol_pad, sizeof(__half) * p->pad_elems * max_batch));
+      PLAN_CUDA(cudaMemset(p->d_vol_pad, 0, sizeof(__half) * p->pad_elems * max_batch));
     }
   }
   p->bp_cull = bp_cull_rule(p);
@@ -323,9 +318,8 @@ int create_plan(const dtv_geometry* g, int max_batch, int flags, int device, Pla
     const double voxels = (double)gp.nx * gp.ny * gp.nz;
     double staged;
     if (flags & DTV_PLAN_TEX_PAIRS) staged = (double)gp.nx * gp.ny * (gp.nz + 3) * 4.0;
-    else if (flags & DTV_PLAN_PAIRS_EXACT) staged = (double)p->pair_quad_elems * 16.0;
     else if (flags & DTV_PLAN_TEX) staged = voxels * (p->stage_dtype == DTV_F16 ? 2.0 : 4.0);
-    else if (p->d_vol_quads) staged = (double)p->pad_elems * 16.0;
+    else if (p->d_vol_rec) staged = (double)p->pad_elems * 16.0;
     else staged = (double)p->pad_elems * 2.0;
     p->fp_band = staged > kBandAboveBytes ? kDefaultBand : 0;
   }
