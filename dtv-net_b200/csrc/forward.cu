@@ -875,94 +875,176 @@ __global__ void __launch_bounds__(kAdjThreads) adjoint_brick_kernel(
 
 // ---- the same transpose with vector atomics into cell records ---------------------------
 // Record (ix, iy, z) holds the four contributions of a trilinear cell to the
-// voxels (ix, iy, z), (ix+1, iy, z), (ix, iy+1, z), (ix+1, iy+1, z); x and y
-// run over [-1, n-1] (the cells whose corners reach the volume), z over
-// [0, nz-1]. A sample of base cell (ix, iy, iz) adds its bilinear weights
-// times (1 - az) to record (ix, iy, iz) and times az to record (ix, iy, iz+1):
-// two 16-byte vector reductions into L2 instead of eight scalar atomics. A
-// gather pass then sums each voxel's four record entries. Samples whose cell
-// lies wholly in the zero border are skipped, as their forward taps read zeros.
+// voxels (ix, iy, z), (ix+1, iy, z), (ix, iy+1, z), (ix+1, iy+1, z), z fastest
+// over the grid padded by kPad on every side (the padded grid of RecSampler,
+// so every sample's records exist). A sample of base cell (ix, iy, iz) adds its
+// bilinear weights times (1 - az) to record (ix, iy, iz) and times az to record
+// (ix, iy, iz+1): two 16-byte vector reductions into L2 instead of eight
+// scalar atomics. A gather pass then sums each voxel's four record entries.
+//
+// The L2 takes reductions by the 32-byte sector, and lanes of one record one
+// after the other: two reductions per sample bounded the scatter (2.61 ms for
+// 2 x 128^3 x 48 views of 192^2, 18.2 ms for 256^3 x 64 views of 384^2).
+// So the lanes of a warp run along v (one column of rays, whose samples of one
+// step fall into one (x, y) column at neighbouring z) and merge before they
+// reduce: lanes of one base record add up in the run's first lane, and a run's
+// upper-plane sums join the next run where that is the next record. With 1.3
+// rays per voxel along v, 64 reductions of 32 samples become 25 on consecutive
+// records: 1.29 and 9.5 ms, bound by instruction issue (117 per 32 samples, 91 %).
+//
+// kSlab: this launch takes the samples whose base y-cell is in [yb0, yb1).
+template <bool kSlab>
 __global__ void __launch_bounds__(256) adjoint_cells_kernel(RayParams rp,
                                                             const FPView* __restrict__ views,
                                                             const float4* __restrict__ rays,
                                                             const float* __restrict__ sino,
-                                                            float4* __restrict__ cells, int batch,
-                                                            int zb0, int zb1) {
-  const int64_t per = (int64_t)rp.n_views * rp.nu * rp.nv;
-  const int64_t total = per * batch;
-  const int cx = rp.nx + 1, cy = rp.ny + 1;
-  const int64_t cplane = (int64_t)cx * cy, citem = cplane * rp.nz;
-  for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < total;
-       r += (int64_t)gridDim.x * blockDim.x) {
-    const float val = __ldg(sino + r) * rp.scale;
-    if (val == 0.f) continue;
-    const int b = (int)(r / per);
-    const int64_t ray = r - b * per;
-    RaySetup rs;
-    if (rays) {
-      const float4 a = __ldg(rays + 2 * ray), c = __ldg(rays + 2 * ray + 1);
-      rs.p0[0] = a.x; rs.p0[1] = a.y; rs.p0[2] = a.z;
-      rs.count = __float_as_int(a.w);
-      rs.dp[0] = c.x; rs.dp[1] = c.y; rs.dp[2] = c.z;
-    } else {
-      const int u = (int)(ray % rp.nu);
-      const int64_t q = ray / rp.nu;
-      rs = setup_ray(rp, views[(int)(q / rp.nv)], u, (int)(q % rp.nv));
-    }
-    float4* cb = cells + b * citem;
-    // this launch takes the samples whose base z-cell is in [zb0, zb1): their
-    // k range from the ray's (monotone) z, widened by one, then tested exactly
-    int k0 = 0, k1 = rs.count;
-    if (rs.dp[2] != 0.f) {
-      const float inv = 1.f / rs.dp[2];
-      const float ka = ((float)zb0 - rs.p0[2]) * inv, kb = ((float)zb1 - rs.p0[2]) * inv;
-      const float cnt = (float)rs.count;  // clamp in float: the estimates may be huge
-      k0 = (int)fminf(fmaxf(floorf(fminf(ka, kb)) - 1.f, 0.f), cnt);
-      k1 = (int)fminf(fmaxf(ceilf(fmaxf(ka, kb)) + 1.f, 0.f), cnt);
-    }
-    for (int k = k0; k < k1; ++k) {
-      const float kf = (float)k;
-      const float x = fmaf(kf, rs.dp[0], rs.p0[0]), y = fmaf(kf, rs.dp[1], rs.p0[1]),
-                  z = fmaf(kf, rs.dp[2], rs.p0[2]);
-      const float fx = floorf(x), fy = floorf(y), fz = floorf(z);
-      const int ix = (int)fx, iy = (int)fy, iz = (int)fz;
-      if (iz < zb0 || iz >= zb1 || ix < -1 || ix > rp.nx - 1 || iy < -1 || iy > rp.ny - 1)
-        continue;
-      const float ax = x - fx, ay = y - fy, az = z - fz;
-      const float bx = 1.f - ax, by = 1.f - ay;
-      const int64_t cell = (int64_t)(iy + 1) * cx + (ix + 1);  // within a z-plane
-      if (iz >= 0) {
-        const float w = val * (1.f - az);
-        atomicAdd(cb + iz * cplane + cell,
-                  make_float4(w * bx * by, w * ax * by, w * bx * ay, w * ax * ay));
+                                                            float4* __restrict__ cells,
+                                                            int64_t pad_elems, int yb0, int yb1) {
+  constexpr unsigned int kAll = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  int u, v, n;
+  tile_pixel_v(rp, u, v, n);
+  // z grows with the lane: a detector whose rows run down takes them reversed
+  const int wv = 32 >> rp.lwu;
+  if (views[n].v[2] < 0.0) v += wv - 1 - 2 * (lane & (wv - 1));
+  const int b = blockIdx.z;
+  const int64_t per_view = (int64_t)rp.nu * rp.nv;
+  const int64_t ray = n * per_view + (int64_t)v * rp.nu + u;
+  float val = 0.f;
+  float4 a = make_float4(0.f, 0.f, 0.f, 0.f), c = a;
+  int k0 = 0, k1 = 0;
+  const float lo = (float)yb0, hi = (float)yb1;
+  const float fnx = (float)rp.nx, fny = (float)rp.ny, fnz = (float)rp.nz;
+  bool safe = true;
+  if (u < rp.nu && v < rp.nv) {
+    val = __ldg(sino + b * rp.n_views * per_view + ray) * rp.scale;
+    if (val != 0.f) {
+      a = __ldg(rays + 2 * ray);
+      c = __ldg(rays + 2 * ray + 1);
+      k1 = __float_as_int(a.w);
+      // the k range of the slab from the ray's (monotone) y, widened by one
+      if (kSlab && c.y != 0.f) {
+        const float inv = 1.f / c.y;
+        const float ka = (lo - a.y) * inv, kb = (hi - a.y) * inv;
+        const float cnt = (float)k1;  // clamp in float: the estimates may be huge
+        k0 = (int)fminf(fmaxf(floorf(fminf(ka, kb)) - 1.f, 0.f), cnt);
+        k1 = (int)fminf(fmaxf(ceilf(fmaxf(ka, kb)) + 1.f, 0.f), cnt);
       }
-      if (iz + 1 < rp.nz) {
-        const float w = val * az;
-        atomicAdd(cb + (iz + 1) * cplane + cell,
-                  make_float4(w * bx * by, w * ax * by, w * bx * ay, w * ax * ay));
+      // positions are monotone: the ends tell whether every record exists; else
+      // a sample outside (-1, n), whose forward taps read zeros, is left out
+      auto holds = [&](float k) {
+        const float x = fmaf(k, c.x, a.x), y = fmaf(k, c.y, a.y), z = fmaf(k, c.z, a.z);
+        return x >= -2.f && x < fnx + 1.f && y >= -2.f && y < fny + 1.f && z >= -2.f &&
+               z < fnz + 1.f;
+      };
+      safe = k0 < k1 && holds((float)k0) && holds((float)(k1 - 1));
+    }
+  }
+  const bool any = k0 < k1;
+  const int kmin = __reduce_min_sync(kAll, any ? k0 : 0x7fffffff);
+  const int kmax = __reduce_max_sync(kAll, any ? k1 : 0);
+  const unsigned int pz = (unsigned int)rp.nz + 2 * kPad, pxz = pz * (unsigned int)(rp.nx + 2 * kPad);
+  // record (0, 0, 0), biased by the magic bits (modulo 2^32; indices stay below 2^31)
+  const unsigned int origin = kPad * (pxz + pz + 1) - kIntMagicBits * (pxz + pz + 1);
+  float4* cb = cells + b * pad_elems;
+  const bool checked = !__all_sync(kAll, safe || !any);
+  const unsigned int len = (unsigned int)(any ? k1 - k0 : 0);
+  unsigned int j = (unsigned int)(kmin - k0);  // samples into this ray (wraps below its first)
+  float kf = (float)kmin;
+  for (int k = kmin; k < kmax; ++k, ++j, kf += 1.f) {
+    const float x = fmaf(kf, c.x, a.x), y = fmaf(kf, c.y, a.y), z = fmaf(kf, c.z, a.z);
+    const float tx = __fadd_rd(x, kIntMagic), ty = __fadd_rd(y, kIntMagic),
+                tz = __fadd_rd(z, kIntMagic);
+    const float fy = ty - kIntMagic;
+    bool live = j < len;
+    if (kSlab) live = live && fy >= lo && fy < hi;
+    if (checked)
+      live = live && (safe || (x >= -1.f && x < fnx && y >= -1.f && y < fny && z >= -1.f && z < fnz));
+    // idle lanes take markers that equal and adjoin no record
+    const unsigned int rec = live ? __float_as_uint(ty) * pxz + __float_as_uint(tx) * pz +
+                                        __float_as_uint(tz) + origin
+                                  : 0xffffff00u + 2u * lane;
+    const float ax = x - (tx - kIntMagic), ay = y - fy, az = z - (tz - kIntMagic);
+    const float w1 = val * az, w0 = val - w1;
+    const float q0 = w0 * ay, p0 = w0 - q0, q1 = w1 * ay, p1 = w1 - q1;
+    float A[4], B[4];
+    A[1] = p0 * ax; A[0] = p0 - A[1]; A[3] = q0 * ax; A[2] = q0 - A[3];
+    B[1] = p1 * ax; B[0] = p1 - B[1]; B[3] = q1 * ax; B[2] = q1 - B[3];
+    const unsigned int prec = __shfl_up_sync(kAll, rec, 1);
+    const bool first = lane == 0 || prec != rec;
+    const unsigned int firsts = __ballot_sync(kAll, first);
+    const bool last = lane == 31 || ((firsts >> lane >> 1) & 1);
+    // runs of one record: A sums into the run's first lane, B into its last
+    unsigned int rest = ~firsts;
+    if (rest) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float da = __shfl_down_sync(kAll, A[e], 1), db = __shfl_up_sync(kAll, B[e], 1);
+        if (!last) A[e] += da;
+        if (!first) B[e] += db;
+      }
+      rest &= rest << 1;  // runs longer than two
+      for (int o = 2; rest; o <<= 1) {
+        const unsigned int reach = (1u << o) - 1;  // lanes (l, l + o] start no run
+        const bool down = lane + o < 32 && ((firsts >> lane >> 1) & reach) == 0;
+        const bool up = lane >= o && ((firsts >> (lane - o + 1)) & reach) == 0;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float da = __shfl_down_sync(kAll, A[e], o), db = __shfl_up_sync(kAll, B[e], o);
+          if (down) A[e] += da;
+          if (up) B[e] += db;
+        }
+        rest &= rest << o;
       }
     }
+    // a run's upper plane joins the next run's lower one where that is the same record
+    const bool take = first && lane > 0 && prec + 1 == rec;
+    const unsigned int joins = __ballot_sync(kAll, take);
+    if (joins) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float d = __shfl_up_sync(kAll, B[e], 1);
+        if (take) A[e] += d;
+      }
+    }
+    float4* r = cb + rec;
+    if (live && first) atomicAdd(r, make_float4(A[0], A[1], A[2], A[3]));
+    if (live && last && !((joins >> lane >> 1) & 1))
+      atomicAdd(r + 1, make_float4(B[0], B[1], B[2], B[3]));
   }
 }
 
-__global__ void adjoint_gather_kernel(const float4* __restrict__ cells, float* __restrict__ out,
-                                      int nx, int ny, int nz, int batch) {
-  const int cx = nx + 1, cy = ny + 1;
-  const int64_t vox = (int64_t)nx * ny * nz, total = vox * batch;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const int b = (int)(i / vox);
-    const int64_t j = i - b * vox;
-    const int x = (int)(j % nx);
-    const int64_t q = j / nx;
-    const int y = (int)(q % ny), z = (int)(q / ny);
-    const float4* rz = cells + (int64_t)b * cx * cy * nz + (int64_t)z * cx * cy;
-    const float4* r11 = rz + (int64_t)(y + 1) * cx + (x + 1);  // cell (x, y)
-    const float4* r01 = r11 - 1;                                // cell (x-1, y)
-    const float4* r10 = r11 - cx;                               // cell (x, y-1)
-    const float4* r00 = r10 - 1;                                // cell (x-1, y-1)
-    out[i] = __ldg(&r11->x) + __ldg(&r01->y) + __ldg(&r10->z) + __ldg(&r00->w);
+// Each voxel's four record entries, summed. A warp owns 32 slices of one row
+// and marches x, reading records along z; the sums go through shared memory so
+// that the volume is written along x.
+__global__ void __launch_bounds__(256) adjoint_gather_kernel(const float4* __restrict__ cells,
+                                                             float* __restrict__ out, int nx,
+                                                             int ny, int nz, int ytiles,
+                                                             int64_t pad_elems) {
+  __shared__ float s[8][32][33];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int b = blockIdx.z / ytiles;
+  const int x0 = blockIdx.x * 32, z0 = blockIdx.y * 32;
+  const int y = (int)(blockIdx.z % ytiles) * 8 + w;
+  const int z = z0 + lane;
+  const int64_t pz = nz + 2 * kPad, px = nx + 2 * kPad;
+  const int xs = min(32, nx - x0);
+  if (y < ny && z < nz) {
+    // record (x - 1, y) and (x - 1, y - 1), then march
+    const float4* r = cells + b * pad_elems + ((int64_t)(y + kPad) * px + x0 - 1 + kPad) * pz + z + kPad;
+    const float4* q = r - px * pz;
+    float4 r0 = __ldg(r), q0 = __ldg(q);
+    for (int x = 0; x < xs; ++x) {
+      const float4 r1 = __ldg(r + (x + 1) * pz), q1 = __ldg(q + (x + 1) * pz);
+      s[w][lane][x] = r1.x + r0.y + q1.z + q0.w;
+      r0 = r1;
+      q0 = q1;
+    }
   }
+  __syncwarp();
+  if (y >= ny || lane >= xs) return;
+  float* o = out + ((int64_t)b * nz * ny + y) * nx + x0 + lane;
+  for (int k = 0; k < min(32, nz - z0); ++k) o[(int64_t)(z0 + k) * ny * nx] = s[w][k][lane];
 }
 
 int adjoint_impl(Plan* p, const float* sino, int batch, float* out, cudaStream_t st) {
@@ -970,23 +1052,37 @@ int adjoint_impl(Plan* p, const float* sino, int batch, float* out, cudaStream_t
   RayParams rp = make_ray_params(gp);
   const int64_t vox = (int64_t)gp.nx * gp.ny * gp.nz;
   if (p->adjoint_method == 1 && p->d_cells) {
-    const int64_t cells = (int64_t)(gp.nx + 1) * (gp.ny + 1) * gp.nz * batch;
-    DTV_CUDA_TRY(cudaMemsetAsync(p->d_cells, 0, cells * sizeof(float4), st));
-    const int64_t rays = (int64_t)gp.n_views * gp.nu * gp.nv * batch;
-    const int grid = (int)std::min<int64_t>((rays + 255) / 256, 148LL * 64);
-    // z-slabs of base cells whose records (at most 72 MB over the batch) stay
-    // resident in L2 while their samples scatter; base cells run over [-1, nz-1]
-    const int64_t plane_bytes = (int64_t)(gp.nx + 1) * (gp.ny + 1) * sizeof(float4) * batch;
-    const int slab = (int)std::max<int64_t>(1, (72LL << 20) / plane_bytes);
-    for (int zb0 = -1; zb0 < gp.nz; zb0 += slab) {
-      const int zb1 = std::min(zb0 + slab, gp.nz);
-      adjoint_cells_kernel<<<grid, 256, 0, st>>>(rp, p->d_fpv, p->d_rays, sino, p->d_cells, batch,
-                                                 zb0, zb1); note_launch();
+    DTV_CUDA_TRY(cudaMemsetAsync(p->d_cells, 0, p->pad_elems * batch * sizeof(float4), st));
+    // warps of 4 x 8 rays: 128^3 x 48 views 0.68 ms (1 x 32: 0.73, 2 x 16: 0.69;
+    // 97x113x61 x 33 views: 271, 334, 291 us)
+    rp.ltu = kRayTiles[3][0];
+    rp.ltv = kRayTiles[3][1];
+    rp.lwu = kRayTiles[3][2];
+    const int tiles = ((gp.nu + (1 << rp.ltu) - 1) >> rp.ltu) * ((gp.nv + (1 << rp.ltv) - 1) >> rp.ltv);
+    // y-slabs of base cells whose records (at most 160 MB over the batch) stay
+    // in L2 while their samples scatter; cells run over [-2, ny]. 256^3 x 64
+    // views of 384^2: 9.51 ms (slabs of 72 MB 9.80, none 10.63)
+    const int64_t row_bytes = (int64_t)(gp.nx + 2 * kPad) * (gp.nz + 2 * kPad) * sizeof(float4) * batch;
+    const int64_t rows = std::max<int64_t>(1, (160LL << 20) / row_bytes);
+    const int slabs = (int)((gp.ny + 3 + rows - 1) / rows);
+    const int slab = (gp.ny + 3 + slabs - 1) / slabs;
+    for (int yb = -2; yb <= gp.ny; yb += slab) {
+      const auto kernel = slabs > 1 ? adjoint_cells_kernel<true> : adjoint_cells_kernel<false>;
+      kernel<<<dim3(tiles, gp.n_views, batch), 256, 0, st>>>(rp, p->d_fpv, p->d_rays, sino, p->d_cells,
+                                                             p->pad_elems, yb,
+                                                             std::min(yb + slab, gp.ny + 1));
+      note_launch();
       DTV_LAUNCH_CHECK();
     }
-    const int ggrid = (int)std::min<int64_t>((vox * batch + 255) / 256, 148LL * 32);
-    adjoint_gather_kernel<<<ggrid, 256, 0, st>>>(p->d_cells, out, gp.nx, gp.ny, gp.nz, batch); note_launch();
-    DTV_LAUNCH_CHECK();
+    const int ytiles = (gp.ny + 7) / 8;
+    const int per = std::max(1, 65535 / ytiles);  // volumes per launch
+    for (int b = 0; b < batch; b += per) {
+      const dim3 grid((gp.nx + 31) / 32, (gp.nz + 31) / 32, ytiles * std::min(per, batch - b));
+      adjoint_gather_kernel<<<grid, 256, 0, st>>>(p->d_cells + b * p->pad_elems, out + b * vox,
+                                                  gp.nx, gp.ny, gp.nz, ytiles, p->pad_elems);
+      note_launch();
+      DTV_LAUNCH_CHECK();
+    }
     return DTV_OK;
   }
   const int bricks = ((gp.nx + kAB - 1) / kAB) * ((gp.ny + kAB - 1) / kAB) *

@@ -297,8 +297,7 @@ int create_plan(const dtv_geometry* g, int max_batch, int flags, int device, Pla
   if (flags & DTV_PLAN_ADJOINT) {
     const size_t n = (size_t)gp.n_views * gp.nu * gp.nv * 2;
     PLAN_CUDA(cudaMalloc(&p->d_rays, n * sizeof(float4)));
-    const size_t cells = (size_t)(gp.nx + 1) * (gp.ny + 1) * gp.nz * max_batch;
-    PLAN_CUDA(cudaMalloc(&p->d_cells, cells * sizeof(float4)));
+    PLAN_CUDA(cudaMalloc(&p->d_cells, (size_t)p->pad_elems * max_batch * sizeof(float4)));
     p->adjoint_method = 1;
     rc = build_ray_table(p, 0);
     if (!rc) {
