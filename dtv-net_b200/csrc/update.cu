@@ -1216,6 +1216,96 @@ __global__ void __launch_bounds__(256) tv_descent_kernel(const float* __restrict
   }
 }
 
+// The same step with every voxel's normalised gradient computed about once. A
+// warp owns 32 columns, of which the 30 inner ones are outputs, and a thread
+// marches kTVRows rows of its column along z: the x neighbour's term comes from
+// the next lane, the y neighbour's from the thread's previous row (one halo row
+// below), the z neighbour's from its previous slice. 1.25 x 1.07 gradients per
+// voxel instead of four: 143x129x77 27.9 -> 10.9 us, 256^3 177 -> 57 us, 315 ->
+// 85 instructions per voxel, bound by instruction issue.
+//
+// Rows are addressed through the flat index, so with the D_y wrap and X == Y
+// (offset Y is then one row) row -1 of a slice is the last row of the slice
+// before, and only the validity of the first and last rows differs.
+// For the clean D_y, or the wrap with X == Y; tv_descent_kernel does the rest.
+constexpr int kTVRows = 4, kTVCols = 30, kTVWarps = 4;
+template <bool kQuirk>
+__global__ void __launch_bounds__(32 * kTVWarps) tv_descent_rows_kernel(
+    const float* __restrict__ fin, float* __restrict__ fout, Dims d,
+    const float* __restrict__ davg) {
+  constexpr unsigned int kAll = 0xffffffffu;
+  constexpr int R = kTVRows;
+  const int lane = threadIdx.x;
+  const int x = (int)blockIdx.x * kTVCols + lane - 1;
+  const int y0 = ((int)blockIdx.y * kTVWarps + (int)threadIdx.y) * R;
+  const int zslabs = (d.Z + d.zs - 1) / d.zs;
+  const int z0 = (int)(blockIdx.z % zslabs) * d.zs;
+  const int z1 = min(z0 + d.zs, d.Z);
+  if (y0 >= d.Y) return;  // whole warps
+  const float step = davg[0];
+  const int64_t item = (int64_t)(blockIdx.z / zslabs) * d.N;
+  const unsigned int plane = (unsigned int)d.X * d.Y, N = (unsigned int)d.N;
+  const bool xin = x >= 0 && x < d.X, xv = x < d.X - 1, xl = x >= 1;
+  const bool store = lane >= 1 && lane <= kTVCols && xin;
+  const int zfirst = max(z0 - 1, 0);  // the slice below gives the z neighbours' terms
+  // flat index of row y0 - 1 in slice z (modulo 2^32: a row before the volume is
+  // beyond N, and so is one after it)
+  unsigned int i0 = (unsigned int)zfirst * plane + (unsigned int)(y0 - 1) * d.X + (unsigned int)x;
+  const float* p = fin + item + (int64_t)zfirst * plane + (int64_t)(y0 - 1) * d.X + x;
+  float* o = fout + (p - fin);
+  // f of rows y0 - 1 .. y0 + R of a slice; a row outside the volume reads zero
+  // (rows beyond a slice's own are other slices', read where the wrap joins them)
+  auto load = [&](const float* q, unsigned int i, bool slice, float (&v)[R + 2]) {
+#pragma unroll
+    for (int r = 0; r < R + 2; ++r) {
+      const bool in = kQuirk ? i + (unsigned int)(r * d.X) < N
+                             : slice && y0 - 1 + r >= 0 && y0 - 1 + r < d.Y;
+      v[r] = xin && in ? __ldg(q + r * d.X) : 0.f;
+    }
+  };
+  float cur[R + 2], nxt[R + 2], qz[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) qz[r] = 0.f;
+  load(p, i0, true, cur);
+  for (int z = zfirst; z < z1; ++z, p += plane, o += plane, i0 += plane) {
+    const bool zv = z < d.Z - 1;
+    load(p + plane, i0 + plane, zv, nxt);
+    float qyp = 0.f;  // the previous row's y term
+#pragma unroll
+    for (int r = 0; r <= R; ++r) {  // rows y0 - 1 (halo), y0 .. y0 + R - 1
+      const int y = y0 + r - 1;
+      const float fc = cur[r];
+      const unsigned int i = i0 + (unsigned int)(r * d.X);
+      const float fr = __shfl_down_sync(kAll, fc, 1);
+      const float gx = (xv ? fr : 0.f) - fc;
+      const bool yv = kQuirk ? i < N - (unsigned int)d.X : y < d.Y - 1;
+      const float gy = (yv ? cur[r + 1] : 0.f) - fc;
+      // a halo row of the slice before (wrap) has its z neighbour in this slice
+      const bool zn = kQuirk && r == 0 && y < 0 ? z >= 1 : zv;
+      const float gz = (zn ? nxt[r] : 0.f) - fc;
+      float nrm;
+      asm("sqrt.approx.f32 %0, %1;" : "=f"(nrm) : "f"(fmaf(gx, gx, fmaf(gy, gy, gz * gz))));
+      const float inv = rcp_newton(nrm + 1.f);
+      const float qx = gx * inv, qy = gy * inv, qzc = gz * inv;
+      if (r > 0) {
+        const float left = __shfl_up_sync(kAll, qx, 1);
+        // the order of the general kernel: x, y, z, own term then neighbour's
+        const bool yl = kQuirk ? i >= (unsigned int)d.X : y >= 1;
+        float grad = (xl ? left : 0.f) - qx;
+        grad -= qy;
+        grad += yl ? qyp : 0.f;
+        grad -= qzc;
+        grad += qz[r - 1];  // zero in the first slice
+        qz[r - 1] = qzc;
+        if (z >= z0 && store && y < d.Y) o[r * d.X] = fmaf(-step, grad, fc);
+      }
+      qyp = qy;
+    }
+#pragma unroll
+    for (int r = 0; r < R + 2; ++r) cur[r] = nxt[r];
+  }
+}
+
 __global__ void scale_scalar_kernel(const double* in, double scale, float* out) {
   if (threadIdx.x == 0) out[0] = (float)(in[0] * scale);
 }
@@ -1532,7 +1622,23 @@ int dtv_tv_descent(const float* f_in, float* f_out, const int32_t size[3], int32
   int rc = check_dims(size, batch);
   if (rc) return rc;
   Dims d = make_dims(size, quirk, batch);
-  tv_descent_kernel<<<grid3(d, batch), kBlock3, 0, as_stream(stream)>>>(f_in, f_out, d, davg); note_launch();
+  if (!quirk || d.X == d.Y) {
+    // slices per thread: 8, or 4 / 2 where that gives fewer than 16 warps per SM
+    // (143x129x77: 8 slices 14.9 us, 4 slices 10.9)
+    const int64_t warps = (int64_t)((d.X + kTVCols - 1) / kTVCols) * ((d.Y + kTVRows - 1) / kTVRows);
+    d.zs = 8;
+    while (d.zs > 2 && warps * ((d.Z + d.zs - 1) / d.zs) * batch < 148LL * 16 &&
+           (int64_t)((d.Z + d.zs / 2 - 1) / (d.zs / 2)) * batch <= 65535)
+      d.zs /= 2;
+    const dim3 grid((d.X + kTVCols - 1) / kTVCols,
+                    (d.Y + kTVRows * kTVWarps - 1) / (kTVRows * kTVWarps),
+                    ((d.Z + d.zs - 1) / d.zs) * batch);
+    const auto kernel = quirk ? tv_descent_rows_kernel<true> : tv_descent_rows_kernel<false>;
+    kernel<<<grid, dim3(32, kTVWarps), 0, as_stream(stream)>>>(f_in, f_out, d, davg);
+  } else {
+    tv_descent_kernel<<<grid3(d, batch), kBlock3, 0, as_stream(stream)>>>(f_in, f_out, d, davg);
+  }
+  note_launch();
   DTV_LAUNCH_CHECK();
   return DTV_OK;
 }
