@@ -51,12 +51,6 @@ constexpr int kZC = 8;
 // against an exact one).
 enum BPMode { kRec = 0, kTex = 1, kBoth = 2 };
 
-// Adding 1.5 * 2^23 leaves an integer in the sum's low bits; with rounding down
-// the sum is the floor. The float to integer conversions this replaces run at
-// a quarter rate (40 % of that pipe, and 2.4 x the instructions per sample).
-constexpr float kIntMagic = 12582912.f;
-constexpr unsigned int kIntMagicBits = 0x4B400000u;
-
 // Where a block's sums go: out = base + sum (out = sum when base is NULL; base
 // may be out). kBoth: out takes the record sum E, and
 // diff = diff_base + (E - T) with T the texture sum.

@@ -57,15 +57,13 @@ struct SoftSampler {
 // touches (four at least), and the rays of a warp that share a detector column
 // pass through one (x, y) column at neighbouring z. With the lanes of a quarter
 // warp along v they read consecutive records: 5.3 lines per load, against 11.2
-// with x fastest and lanes along u. 256^3 x 64 views of 384^2: 6.33 -> 3.67 ms,
+// with x fastest and lanes along u. 256^3 x 64 views of 384^2: 6.33 -> 3.48 ms,
 // 2.4 G samples, 80 % of the L1 data clocks busy (32 bytes per sample are 8
 // clocks per 32 samples at best).
 //
-// Floors come from rounding-down adds of 1.5 * 2^23, whose bits then address
-// the record with one 64-bit multiply-add per axis (float-to-integer
-// conversions run at a quarter rate); two samples go through packed FP32.
-constexpr float kIntMagic = 12582912.f;
-constexpr unsigned int kIntMagicBits = 0x4B400000u;
+// Floors come from rounding-down adds (kIntMagic), whose bits then address the
+// record with one 64-bit multiply-add per axis; two samples go through packed
+// FP32.
 
 // kFar: a row of records spans 4 GB or more (its pitch needs 64 bits).
 template <bool kFar>
@@ -243,8 +241,11 @@ __global__ void __launch_bounds__(kFPThreads) fp_soft_kernel(RayParams rp, const
   if (o.abs_sum) block_add_double((double)fabsf(res), o.abs_sum);
 }
 
+// Four blocks per SM: with the bound the compiler uses the 64 registers they
+// leave it (56 without: 3.71 -> 3.48 ms at 256^3 x 64 views); five or six blocks
+// spill (3.67, 4.29 ms).
 template <bool kFar>
-__global__ void __launch_bounds__(kFPThreads) fp_rec_kernel(RayParams rp,
+__global__ void __launch_bounds__(kFPThreads, 4) fp_rec_kernel(RayParams rp,
                                                             const FPView* __restrict__ views,
                                                             const float4* __restrict__ recs,
                                                             int64_t pad_elems, FPOut o) {
@@ -562,7 +563,8 @@ static bool rec_far(const GeomParams& g) {
 
 // `records`: the launch samples records, whose warps want 4 x 8 pixels: tile 0,
 // the default, then stands for shape 3 and the other way round. 256^3 x 64
-// views of 384^2: 4 x 8 3.67 ms, 8 x 4 4.07, 16 x 2 5.90, 32 x 1 9.34.
+// views of 384^2: 4 x 8 3.67 ms, 8 x 4 4.07, 16 x 2 5.90, 32 x 1 9.34; the
+// correction pass 4.94, 5.53, 7.27, 10.5.
 static RayParams plan_ray_params(const Plan* p, bool records) {
   RayParams rp = make_ray_params(p->gp);
   const int t = records && (p->fp_ray_tile == 0 || p->fp_ray_tile == 3) ? 3 - p->fp_ray_tile
