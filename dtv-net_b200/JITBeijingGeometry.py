@@ -17,7 +17,7 @@ _sys.path.insert(0, _os.path.dirname(_os.path.abspath(__file__)))
 import torch as _torch  # noqa: E402
 
 from dtvb200 import geometry as _geo  # noqa: E402
-from JITStandardGeometry import _check_len, _host_values, _SAMPLER  # noqa: E402
+from JITStandardGeometry import _check_len, _host_forms, _on_device, _SAMPLER  # noqa: E402
 
 _plans = {}
 
@@ -28,14 +28,12 @@ def _plan(volumeSize, detectorSize, projectVector, device, batch):
         raise RuntimeError("project vector's shape must be [angle's number, 12]")
     _check_len(volumeSize, 3, "volume size")
     _check_len(detectorSize, 2, "detector size")
-    ph, vh, dh = _host_values([projectVector, volumeSize, detectorSize])
-    pv = ph.astype("float32").reshape(-1, 12)
-    vs = [int(v) for v in vh]
-    ds = [int(v) for v in dh]
-    key = (pv.tobytes(), tuple(vs), tuple(ds), int(device))
+    (pv, raw), vs, ds = _host_forms((projectVector, volumeSize, detectorSize),
+                                    ("f32", "ints", "ints"))
+    key = (raw, vs, ds, int(device))
     p = _plans.get(key)
     if p is None or p.max_batch < batch:
-        g = _geo.vector(pv, vs, ds)
+        g = _geo.vector(pv.reshape(-1, 12), vs, ds)
         p = _geo.Plan(g, max_batch=max(batch, 1), sampler=_SAMPLER,
                       device=_torch.device("cuda", int(device)))
         _plans[key] = p
@@ -45,12 +43,10 @@ def _plan(volumeSize, detectorSize, projectVector, device, batch):
 def forward(volume, volumeSize, detectorSize, projectVector, device):
     _geo.check_input(volume, "volume")
     p = _plan(volumeSize, detectorSize, projectVector, device, volume.shape[0])
-    with _torch.cuda.device(p.device):
-        return p.forward(volume)
+    return _on_device(p, p.forward, volume)
 
 
 def backward(sino, volumeSize, detectorSize, projectVector, device):
     _geo.check_input(sino, "sino")
     p = _plan(volumeSize, detectorSize, projectVector, device, sino.shape[0])
-    with _torch.cuda.device(p.device):
-        return p.backward(sino)
+    return _on_device(p, p.backward, sino)

@@ -35,7 +35,10 @@ _SAMPLER = _os.environ.get("DTVB200_SAMPLER", "soft")
 _plans = {}
 
 
-_seen = {}  # id(tensor) -> (weakref, _version, host values)
+_seen = {}  # id(tensor) -> (weakref, _version, host values, their forms)
+# what a plan's key and geometry take the values as
+_FORMS = {"f32": lambda v: (lambda a: (a, a.tobytes()))(v.astype("float32")),
+          "ints": lambda v: tuple(int(x) for x in v)}
 
 
 def _check_len(t, n, name):
@@ -54,14 +57,37 @@ def _version(t):
         return None
 
 
+def _hit(t):
+    """The entry of a tensor already read, the same object and unmodified since."""
+    hit = _seen.get(id(t))
+    if hit is not None and hit[0]() is t and hit[1] is not None and hit[1] == _version(t):
+        return hit
+    return None
+
+
+def _host_forms(tensors, forms):
+    """The tensors' host values in the named forms; a read tensor's are kept
+    beside its values."""
+    hits = [_hit(t) for t in tensors]
+    if None in hits:
+        return [_FORMS[f](v) for f, v in zip(forms, _host_values(tensors))]
+    out = []
+    for hit, f in zip(hits, forms):
+        v = hit[3].get(f)
+        if v is None:
+            v = hit[3][f] = _FORMS[f](hit[2])
+        out.append(v)
+    return out
+
+
 def _host_values(tensors):
     """Host float64 copies of small geometry tensors: cached per tensor object
     and version, host tensors read directly, device tensors in one copy."""
     out = [None] * len(tensors)
     fetch = []
     for i, t in enumerate(tensors):
-        hit = _seen.get(id(t))
-        if hit is not None and hit[0]() is t and hit[1] is not None and hit[1] == _version(t):
+        hit = _hit(t)
+        if hit is not None:
             out[i] = hit[2]
         elif t.is_cuda:
             fetch.append(i)
@@ -81,7 +107,7 @@ def _host_values(tensors):
             if ver is not None:
                 k = id(tensors[i])
                 _seen[k] = (_weakref.ref(tensors[i], lambda _r, k=k: _seen.pop(k, None)), ver,
-                            out[i])
+                            out[i], {})
     return out
 
 
@@ -90,11 +116,8 @@ def _plan(angles, volumeSize, detectorSize, sid, sdd, device, batch):
         raise RuntimeError("angles must be a tensor")
     _check_len(volumeSize, 3, "volume size")
     _check_len(detectorSize, 2, "detector size")
-    ah, vh, dh = _host_values([angles, volumeSize, detectorSize])
-    a = ah.astype("float32")
-    vs = [int(v) for v in vh]
-    ds = [int(v) for v in dh]
-    key = (a.tobytes(), tuple(vs), tuple(ds), float(sid), float(sdd), int(device))
+    (a, raw), vs, ds = _host_forms((angles, volumeSize, detectorSize), ("f32", "ints", "ints"))
+    key = (raw, vs, ds, float(sid), float(sdd), int(device))
     p = _plans.get(key)
     if p is None or p.max_batch < batch:
         g = _geo.standard(a, vs, ds, sid, sdd)
@@ -104,15 +127,21 @@ def _plan(angles, volumeSize, detectorSize, sid, sdd, device, batch):
     return p
 
 
+def _on_device(p, op, x):
+    """op(x) with the plan's device current."""
+    if _torch.cuda.current_device() == p.device.index:
+        return op(x)
+    with _torch.cuda.device(p.device):
+        return op(x)
+
+
 def forward(volume, angles, volumeSize, detectorSize, sid, sdd, device):
     _geo.check_input(volume, "volume")
     p = _plan(angles, volumeSize, detectorSize, sid, sdd, device, volume.shape[0])
-    with _torch.cuda.device(p.device):
-        return p.forward(volume)
+    return _on_device(p, p.forward, volume)
 
 
 def backward(sino, angles, volumeSize, detectorSize, sid, sdd, device):
     _geo.check_input(sino, "sino")
     p = _plan(angles, volumeSize, detectorSize, sid, sdd, device, sino.shape[0])
-    with _torch.cuda.device(p.device):
-        return p.backward(sino)
+    return _on_device(p, p.backward, sino)

@@ -11,11 +11,14 @@ namespace dtv {
 
 namespace {
 
+// Makes `dev` current for the scope (nothing to set where it already is).
 struct DeviceGuard {
   int prev = -1;
   bool ok = false;
   explicit DeviceGuard(int dev) {
-    if (cudaGetDevice(&prev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess) ok = true;
+    if (cudaGetDevice(&prev) != cudaSuccess) return;
+    if (prev == dev) prev = -1;
+    ok = prev < 0 || cudaSetDevice(dev) == cudaSuccess;
   }
   ~DeviceGuard() {
     if (prev >= 0) cudaSetDevice(prev);

@@ -110,12 +110,13 @@ def circular(angles_deg, volume_size, voxel, detector_size, pitch, sod: float,
     return _finish(g, views)
 
 
-def _stream(device: torch.device) -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+def _stream(device: torch.device) -> int:
+    """The device's current stream, as the C ABI's argument type takes it."""
+    return torch.cuda.current_stream(device).cuda_stream
 
 
-def _ptr(t) -> ctypes.c_void_p:
-    return ctypes.c_void_p(0 if t is None else t.data_ptr())
+def _ptr(t) -> int:
+    return 0 if t is None else t.data_ptr()
 
 
 def check_input(t: torch.Tensor, name: str, shape=None, dtypes=(torch.float32,)):
@@ -126,7 +127,7 @@ def check_input(t: torch.Tensor, name: str, shape=None, dtypes=(torch.float32,))
         raise RuntimeError(f"{name} must be contiguous")
     if t.dtype not in dtypes:
         raise RuntimeError(f"{name} must have dtype in {dtypes}, got {t.dtype}")
-    if shape is not None and tuple(t.shape) != tuple(shape):
+    if shape is not None and t.shape != shape and tuple(t.shape) != tuple(shape):
         raise RuntimeError(f"{name} must have shape {tuple(shape)}, got {tuple(t.shape)}")
 
 
@@ -169,6 +170,8 @@ class Plan:
         self.max_batch = int(max_batch)
         self.sampler = sampler
         self.stage_f16 = bool(stage_f16)
+        self._vol_n = int(np.prod(geometry.vol_shape(1)))
+        self._sino_n = int(np.prod(geometry.sino_shape(1)))
         flags = {"soft": 0, "tex": _lib.DTV_PLAN_TEX, "pairs": _lib.DTV_PLAN_TEX_PAIRS,
                  "tma": _lib.DTV_PLAN_TEX_PAIRS | _lib.DTV_PLAN_TMA,
                  "exact": _lib.DTV_PLAN_PAIRS_EXACT}[sampler] | \
@@ -227,12 +230,12 @@ class Plan:
         (out = (out + sigma*(FP - g))/(1+sigma)). abs_sum (float64, 1 element)
         accumulates sum|FP - g| (or sum|FP| for STORE)."""
         check_input(vol, "volume", dtypes=tuple(_DT))
-        per = int(np.prod(self.vol_shape(1)))
-        b = self._batch_of(vol, per)
+        b = self._batch_of(vol, self._vol_n)
         shape = self.sino_shape(b)
         if out is None:
             out = torch.empty(shape, device=vol.device, dtype=torch.float32)
-        check_input(out, "out", shape)
+        else:
+            check_input(out, "out", shape)
         if g is not None:
             check_input(g, "g", shape)
         if abs_sum is not None:
@@ -247,12 +250,13 @@ class Plan:
         ``accumulate`` adds it to out; ``base`` (volume shaped, may be out)
         gives out = base + BP(sino)."""
         check_input(sino, "sino")
-        b = self._batch_of(sino, int(np.prod(self.sino_shape(1))))
+        b = self._batch_of(sino, self._sino_n)
         shape = self.vol_shape(b)
         if out is None:
             out = torch.empty(shape, device=sino.device, dtype=torch.float32)
             accumulate = False
-        check_input(out, "out", shape)
+        else:
+            check_input(out, "out", shape)
         if base is not None:
             check_input(base, "base", shape)
             call("dtv_backward_onto", self._h, _ptr(sino), b, _ptr(base), _ptr(out),
@@ -265,11 +269,12 @@ class Plan:
     def adjoint(self, sino: torch.Tensor, out: torch.Tensor = None) -> torch.Tensor:
         """Exact transpose of forward (STORE): A^T sino."""
         check_input(sino, "sino")
-        b = self._batch_of(sino, int(np.prod(self.sino_shape(1))))
+        b = self._batch_of(sino, self._sino_n)
         shape = self.vol_shape(b)
         if out is None:
             out = torch.empty(shape, device=sino.device, dtype=torch.float32)
-        check_input(out, "out", shape)
+        else:
+            check_input(out, "out", shape)
         call("dtv_backward_adjoint", self._h, _ptr(sino), b, _ptr(out), _stream(sino.device))
         return out
 
@@ -298,7 +303,7 @@ def forward_refresh(fast: Plan, exact: Plan, vol: torch.Tensor, g: torch.Tensor,
     fast projections of vol, g_eff = g + (a - e) and
     w = (w + sigma (e - g)) / (1 + sigma); abs_sum += sum|e - g|."""
     check_input(vol, "volume", dtypes=tuple(_DT))
-    b = fast._batch_of(vol, int(np.prod(fast.vol_shape(1))))
+    b = fast._batch_of(vol, fast._vol_n)
     shape = fast.sino_shape(b)
     for t, n in ((g, "g"), (w, "w"), (g_eff, "g_eff")):
         check_input(t, n, shape)
@@ -313,7 +318,7 @@ def backward_refresh(fast: Plan, exact: Plan, sino: torch.Tensor, out: torch.Ten
     """out = exact.backward(sino), e_b = out - fast.backward(sino), in one
     launch (the plans as for forward_refresh)."""
     check_input(sino, "sino")
-    b = fast._batch_of(sino, int(np.prod(fast.sino_shape(1))))
+    b = fast._batch_of(sino, fast._sino_n)
     shape = fast.vol_shape(b)
     check_input(out, "out", shape)
     check_input(e_b, "e_b", shape)

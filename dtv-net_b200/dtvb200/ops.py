@@ -32,6 +32,8 @@ class Projector:
         self.stage_f16 = stage_f16
         self.max_batch = max_batch
         self._plans = {}
+        self._vol_n = int(np.prod(geometry.vol_shape(1)))
+        self._sino_n = int(np.prod(geometry.sino_shape(1)))
 
     def plan(self, device: torch.device, batch: int = 1, sampler: str = None) -> Plan:
         sampler = sampler or self.sampler
@@ -46,8 +48,7 @@ class Projector:
         return p
 
     def batch_of(self, t: torch.Tensor, volume: bool) -> int:
-        per = int(np.prod(self.geometry.vol_shape(1) if volume else self.geometry.sino_shape(1)))
-        return max(1, t.numel() // per)
+        return max(1, t.numel() // (self._vol_n if volume else self._sino_n))
 
     def fp(self, x: torch.Tensor) -> torch.Tensor:
         x = x.contiguous()
