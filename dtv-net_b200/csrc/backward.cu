@@ -484,6 +484,24 @@ __global__ void __launch_bounds__(256) stage_sino_kernel(const float* __restrict
       o[(int64_t)k * pu] = make_float4(a[k], a[k + 1] - a[k], d[k], d[k + 1] - d[k]);
 }
 
+// The sinogram into its layered array, by surface writes: 3.9 MB (64^3 x 60 views)
+// 2.8 us, 37.7 MB 14.5 us, against 8.0 and 39.5 us for the 3-D copy.
+__global__ void __launch_bounds__(256) stage_sino_tex_kernel(const float* __restrict__ in,
+                                                             cudaSurfaceObject_t surf, int nu,
+                                                             int nv) {
+  const int u = blockIdx.x * 32 + (threadIdx.x & 31);
+  const int v0 = blockIdx.y * 32 + (threadIdx.x >> 5);
+  const int n = blockIdx.z;
+  if (u >= nu) return;
+  const float* s = in + (int64_t)n * nu * nv + u;
+  float x[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) x[k] = v0 + 8 * k < nv ? __ldg(s + (int64_t)(v0 + 8 * k) * nu) : 0.f;
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (v0 + 8 * k < nv) surf2DLayeredwrite(x[k], surf, u * 4, v0 + 8 * k, n);
+}
+
 // View groups per block: the least S of 1, 2, 4, 8 that gives the grid three
 // blocks per SM (8 voxels per thread throughout). A property of the plan's
 // geometry alone, so every launch of the plan sums its views in the same order.
@@ -568,13 +586,10 @@ static BPParams plan_bp_params(const Plan* p) {
 static int stage_sino(Plan* p, const float* sino, cudaStream_t st) {
   const GeomParams& gp = p->gp;
   if (p->sino_tex != nullptr) {
-    cudaMemcpy3DParms cp;
-    memset(&cp, 0, sizeof(cp));
-    cp.srcPtr = make_cudaPitchedPtr((void*)sino, gp.nu * sizeof(float), gp.nu, gp.nv);
-    cp.dstArray = p->sino_arrays[0];
-    cp.extent = make_cudaExtent(gp.nu, gp.nv, gp.n_views);
-    cp.kind = cudaMemcpyDeviceToDevice;
-    DTV_CUDA_TRY(cudaMemcpy3DAsync(&cp, st));
+    const dim3 grid((gp.nu + 31) / 32, (gp.nv + 31) / 32, gp.n_views);
+    stage_sino_tex_kernel<<<grid, 256, 0, st>>>(sino, p->sino_surf, gp.nu, gp.nv);
+    note_launch();
+    DTV_LAUNCH_CHECK();
     return DTV_OK;
   }
   const int64_t warps = (int64_t)((gp.nu + 1 + 31) / 32) *
@@ -592,7 +607,7 @@ static int stage_sino(Plan* p, const float* sino, cudaStream_t st) {
 // Of many-module scans, whose modules each see a slice of the fan, most pairs
 // go; where few do the test costs more than it saves (a circular scan whose
 // detector misses the volume's corners: 0.84 -> 0.86 ms through the texture
-// unit, 0.97 -> 1.14 ms through records), and a thread's own end tests skip
+// unit, 151x163x97 through records 118 -> 133 us), and a thread's own end tests skip
 // its views beside the detector anyway.
 int bp_cull_rule(const Plan* p) {
   const GeomParams& gp = p->gp;
@@ -600,12 +615,12 @@ int bp_cull_rule(const Plan* p) {
   const int vs = std::max(1, gp.n_views / 48);
   for (int n = 0; n < gp.n_views; n += vs)
     for (int c = 0; c < 18; ++c) {
+      // blocks at 1/6, 3/6, 5/6 of x and y and 1/4, 3/4 of z
       const int n3[3] = {gp.nx, gp.ny, gp.nz}, e[3] = {kBPTile, kBPTile, kZC};
-      const int g3[3] = {c % 3, c / 3 % 3, c / 9};
+      const int at[3] = {2 * (c % 3) + 1, 2 * (c / 3 % 3) + 1, 2 * (c / 9) + 1};
       float lo[3], hi[3];
       for (int a = 0; a < 3; ++a) {
-        const int blocks = (n3[a] + e[a] - 1) / e[a];
-        const int b = (blocks - 1) * g3[a] / (a == 2 ? 1 : 2);
+        const int b = (int)((int64_t)n3[a] * at[a] / (a == 2 ? 4 : 6)) / e[a];
         lo[a] = (float)(b * e[a]);
         hi[a] = (float)(b * e[a] + e[a] - 1);
       }

@@ -179,6 +179,7 @@ struct Plan {
   float4* d_sino_rec;
   cudaArray_t* sino_arrays;
   cudaTextureObject_t* sino_tex;
+  cudaSurfaceObject_t sino_surf;
   int bp_cull;  // its blocks look for the views they meet first
   // texture sampler (DTV_PLAN_TEX): one 3-D array per batch item
   cudaArray_t* vol_arrays;

@@ -50,6 +50,7 @@ void free_plan(Plan* p) {
       if (p->vol_arrays[b]) cudaFreeArray(p->vol_arrays[b]);
   }
   if (p->sino_tex && p->sino_tex[0]) cudaDestroyTextureObject(p->sino_tex[0]);
+  if (p->sino_surf) cudaDestroySurfaceObject(p->sino_surf);
   if (p->sino_arrays && p->sino_arrays[0]) cudaFreeArray(p->sino_arrays[0]);
   free(p->vol_tex);
   free(p->vol_arrays);
@@ -285,12 +286,17 @@ int create_plan(const dtv_geometry* g, int max_batch, int flags, int device, Pla
     }
     cudaChannelFormatDesc sd = cudaCreateChannelDesc<float>();
     PLAN_CUDA(cudaMalloc3DArray(&p->sino_arrays[0], &sd, make_cudaExtent(gp.nu, gp.nv, gp.n_views),
-                                cudaArrayLayered));
+                                cudaArrayLayered | cudaArraySurfaceLoadStore));
     rc = make_tex3d(p->sino_arrays[0], 1, &p->sino_tex[0]);
     if (rc) {
       free_plan(p);
       return rc;
     }
+    cudaResourceDesc rd;
+    memset(&rd, 0, sizeof(rd));
+    rd.resType = cudaResourceTypeArray;
+    rd.res.array.array = p->sino_arrays[0];
+    PLAN_CUDA(cudaCreateSurfaceObject(&p->sino_surf, &rd));
   } else {
     // records: zero borders written once here, those that reach the view by each call
     const int64_t recs = (int64_t)(gp.nu + 2 * kPad) * (gp.nv + 2 * kPad) * gp.n_views;
