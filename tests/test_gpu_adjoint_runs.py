@@ -29,13 +29,14 @@ def case(kind):
 
 @pytest.mark.parametrize("kind", ["long_runs", "one_per_voxel", "sparse_rays", "wide", "rows_down"])
 @pytest.mark.parametrize("holes", [False, True])
-def test_adjoint_runs(cuda, kind, holes):
+@pytest.mark.parametrize("batch", [1, 2, 3])  # pairs of items share threads, an odd one runs alone
+def test_adjoint_runs(cuda, kind, holes, batch):
     geo, og = case(kind)
     rng = np.random.default_rng(11)
-    y = rng.standard_normal((2, 1) + tuple(og.sino_shape)).astype(np.float32)
+    y = rng.standard_normal((batch, 1) + tuple(og.sino_shape)).astype(np.float32)
     if holes:
         y *= rng.random(y.shape) < 0.6
-    plan = dtvb200.Plan(geo, max_batch=2, device=cuda, adjoint=True)
+    plan = dtvb200.Plan(geo, max_batch=batch, device=cuda, adjoint=True)
     out = plan.adjoint(torch.from_numpy(y).to(cuda)).cpu().numpy()
     ref = O.adjoint(og, y).reshape(out.shape)
     assert np.abs(ref).max() > 0
