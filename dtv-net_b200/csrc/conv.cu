@@ -1,0 +1,706 @@
+// The forward pass of the unrolled networks' convolution block in BF16:
+// Conv3d(1, F) - ReLU - Conv3d(F, F) - ReLU - Conv3d(F, 1), 3x3x3 kernels, zero
+// padding (the shape of model/PDHG/RegularizationLayers/CNN.py:4-18), F = 16 or 32.
+// Activations are channels-last, [batch, z, y, x, F]. Each convolution sums in
+// FP32 and is rounded to BF16, then the BF16 bias is added and rounded again: the
+// roundings that autocast makes around a library convolution.
+// Measured at 2 x 128^3, F = 32: 0.50 ms (0.06 + 0.30 + 0.12 and the weights), where
+// three library convolutions with their layout conversions, bias additions and ReLUs
+// took 4.1 ms; F = 16: 0.37 ms.
+#include <cuda.h>
+#include <cuda_bf16.h>
+
+#include "common.cuh"
+
+namespace dtv {
+namespace {
+
+typedef __nv_bfloat16 bf16;
+
+struct ConvDims {
+  int X, Y, Z, B;
+};
+struct ConvW {  // a weight tensor [out, in, z, y, x] in elements
+  const bf16* w;
+  long long s[5];
+};
+
+__device__ __forceinline__ uint32_t conv_smem(const void* p) {
+  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+__device__ __forceinline__ float round_bf16(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
+// relu(bf16(bf16(sum) + bias)) of two channels; NaN stays NaN
+__device__ __forceinline__ unsigned conv_act(float lo, float hi, __nv_bfloat162 bias) {
+  const __nv_bfloat162 v =
+      __hmax2_nan(__hadd2(__floats2bfloat162_rn(lo, hi), bias), __nv_bfloat162(0.f, 0.f));
+  return *reinterpret_cast<const unsigned*>(&v);
+}
+// D[16 x 8] += A[16 x 16] B[16 x 8], BF16 in, FP32 out
+__device__ __forceinline__ void warp_mma(float (&d)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3,
+                                         unsigned b0, unsigned b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
+      "{%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// ---- F = 16, 32 middle convolution on the tensor cores -----------------------------------
+// A block marches down z over a column of 8 x 16 voxels (the 128 rows of a tile).
+// Each input plane is loaded once by TMA with its y halo, in three copies shifted
+// by -1, 0, 1 in x; a shift in y is then an offset of whole 8-row swizzle atoms, so
+// the nine (x, y) taps read their operands from the copies in place. The three z
+// taps of an (x, y) tap stand side by side in the B operand: one instruction of
+// 3F columns adds an input plane's share to the three output planes around it,
+// which lie side by side in a ring of kRing accumulators in tensor memory. Reading
+// A once for three planes is what makes the step arithmetic-bound: with F columns
+// an instruction waits on its 4 KB of A. 2 x 128^3, F = 32: 0.297 ms, 0.78 PFLOP/s
+// (0.63 ms while the issuing thread built each descriptor and one set of four warps
+// wrote; the library's kernel 1.03 ms).
+// Warp 0 loads, warp 1 issues, warps 2-5 and 6-9 write finished planes in turn.
+constexpr int kCX = 8, kCY = 16;   // column: rows of 8 voxels, one swizzle atom each
+constexpr int kRing = 16;          // accumulators
+constexpr int kStages = 4;         // input planes in flight
+constexpr int kMidThreads = 320;
+constexpr unsigned kConvWaitLimit = 1u << 20;  // polls of one wait
+
+template <int F>
+struct Mid {
+  static constexpr int kRow = F * 2;                        // bytes of a voxel
+  static constexpr int kCopy = kCX * (kCY + 2) * kRow;      // a shifted copy of a plane
+  static constexpr int kStage = 3 * kCopy;
+  static constexpr int kTap = 3 * F * kRow;                 // B operand of an (x, y) tap
+  static constexpr int kWeights = 9 * kTap;
+  static constexpr int kFirst = (kWeights + 1023) / 1024 * 1024;  // of the stages
+  static constexpr int kSmem = 1024 + kFirst + kStages * kStage;
+  static constexpr int kCols = F * kRing;                   // tensor-memory columns
+  static constexpr unsigned long long kLayout = F == 32 ? 4ull : 6ull;  // 64- / 32-byte swizzle
+};
+
+struct MidWork {
+  int tx, ty, nzc, zc;  // columns along x, y; z chunks and their length
+  long long items;
+};
+
+__device__ __forceinline__ bool conv_wait(uint32_t bar, uint32_t parity) {
+  for (unsigned i = 0; i < kConvWaitLimit; ++i) {
+    uint32_t done;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        " selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(done)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    if (done) return true;
+  }
+  return false;
+}
+__device__ __forceinline__ void conv_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void conv_expect(uint32_t bar, unsigned bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
+               : "memory");
+}
+// all matrix instructions issued so far arrive on bar when they are done
+__device__ __forceinline__ void conv_commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
+               : "memory");
+}
+// K-major operand descriptor, 8-row atoms one after another
+template <int F>
+__device__ __forceinline__ unsigned long long conv_desc(uint32_t addr) {
+  return (unsigned long long)((addr >> 4) & 0x3fffu) | (1ull << 16) |
+         ((unsigned long long)(8 * Mid<F>::kRow / 16) << 32) | (1ull << 46) |
+         (Mid<F>::kLayout << 61);
+}
+// D[128 x n] (+)= A[128 x 16] B[n x 16]^T, BF16 in, FP32 out
+__device__ __forceinline__ uint32_t conv_idesc(int n) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | (8u << 24);
+}
+__device__ __forceinline__ void conv_mma(uint32_t d, unsigned long long a, unsigned long long b,
+                                         uint32_t idesc, bool add) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.u32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
+      "l"(a), "l"(b), "r"(idesc), "r"((uint32_t)add)
+      : "memory");
+}
+
+// descriptor offsets of step k = (tap, 16 input channels) from the first step's
+template <int F>
+__device__ constexpr unsigned mid_a(int k) {
+  const int t = k / (F / 16), c = k % (F / 16);
+  return (t % 3 * Mid<F>::kCopy + t / 3 * 8 * Mid<F>::kRow + 32 * c) / 16;
+}
+template <int F>
+__device__ constexpr unsigned mid_b(int k) {
+  return (k / (F / 16) * Mid<F>::kTap + 32 * (k % (F / 16))) / 16;
+}
+
+struct MidItem {
+  int x0, y0, z0, z1, b;
+};
+__device__ __forceinline__ MidItem mid_item(const ConvDims& d, const MidWork& w, long long i) {
+  MidItem r;
+  r.x0 = (int)(i % w.tx) * kCX;
+  i /= w.tx;
+  r.y0 = (int)(i % w.ty) * kCY;
+  i /= w.ty;
+  r.z0 = (int)(i % w.nzc) * w.zc;
+  r.b = (int)(i / w.nzc);
+  r.z1 = min(d.Z, r.z0 + w.zc);
+  return r;
+}
+
+template <int F>
+__global__ void __launch_bounds__(kMidThreads, 1)
+    conv_mid_kernel(const __grid_constant__ CUtensorMap map, const unsigned char* __restrict__ wimg,
+                    const bf16* __restrict__ bias, bf16* __restrict__ out, ConvDims d, MidWork wk,
+                    int* status) {
+  typedef Mid<F> M;
+  extern __shared__ unsigned char conv_dyn[];
+  __shared__ __align__(8) unsigned long long bars[2 * kStages + 2 * kRing + 2];
+  __shared__ uint32_t tmem_slot;
+  const uint32_t base = (conv_smem(conv_dyn) + 1023u) & ~1023u;
+  const uint32_t wsm = base, stages = base + M::kFirst;
+  const uint32_t bar0 = conv_smem(bars);
+  const uint32_t full = bar0, empty = full + 8 * kStages, acc_full = empty + 8 * kStages,
+                 acc_empty = acc_full + 8 * kRing, wbar = acc_empty + 8 * kRing, drain = wbar + 8;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kStages; ++i) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(full + 8 * i) : "memory");
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(empty + 8 * i) : "memory");
+    }
+    for (int i = 0; i < kRing; ++i) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(acc_full + 8 * i) : "memory");
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;" ::"r"(acc_empty + 8 * i) : "memory");
+    }
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(wbar) : "memory");
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(drain) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     conv_smem(&tmem_slot)),
+                 "r"(M::kCols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = tmem_slot;
+  bool ok = true;
+
+  if (warp == 0 && lane == 0) {  // loads
+    conv_expect(wbar, M::kWeights);
+    asm volatile(
+        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(wsm),
+        "l"(wimg), "r"(M::kWeights), "r"(wbar)
+        : "memory");
+    long long n = 0;  // planes loaded
+    for (long long i = blockIdx.x; ok && i < wk.items; i += gridDim.x) {
+      const MidItem it = mid_item(d, wk, i);
+      for (int zi = it.z0 - 1; zi <= it.z1; ++zi, ++n) {
+        const int s = (int)(n % kStages);
+        if (n >= kStages && !(ok = conv_wait(empty + 8 * s, (uint32_t)((n / kStages - 1) & 1)))) break;
+        conv_expect(full + 8 * s, M::kStage);
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+          asm volatile(
+              "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+              " [%0], [%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(stages + s * M::kStage + c * M::kCopy),
+              "l"(&map), "r"(0), "r"(it.x0 + c - 1), "r"(it.y0 - 1), "r"(zi), "r"(it.b),
+              "r"(full + 8 * s)
+              : "memory");
+      }
+    }
+    // the last copies land before the block can end
+    for (long long k = n > kStages ? n - kStages : 0; k < n; ++k)
+      ok &= conv_wait(full + 8 * (int)(k % kStages), (uint32_t)((k / kStages) & 1));
+  } else if (warp == 1 && lane == 0) {  // matrix instructions
+    ok = conv_wait(wbar, 0);
+    long long n = 0, g = 0;  // input planes, output planes so far
+    for (long long i = blockIdx.x; ok && i < wk.items; i += gridDim.x) {
+      const MidItem it = mid_item(d, wk, i);
+      for (int zi = it.z0 - 1; zi <= it.z1; ++zi, ++n) {
+        const int s = (int)(n % kStages);
+        const int lo = max(it.z0, zi - 1), hi = min(it.z1 - 1, zi + 1);
+        if (hi == zi + 1) {  // a plane begins: its accumulator is drained
+          const long long u = g + (hi - it.z0);
+          if (u >= kRing &&
+              !(ok = conv_wait(acc_empty + 8 * (int)(u % kRing), (uint32_t)((u / kRing - 1) & 1))))
+            break;
+        }
+        if (!(ok = conv_wait(full + 8 * s, (uint32_t)((n / kStages) & 1)))) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const unsigned long long ad = conv_desc<F>(stages + s * M::kStage);
+        const unsigned long long bd = conv_desc<F>(wsm + (lo - zi + 1) * F * M::kRow);
+        constexpr unsigned kB = F * M::kRow / 16;  // one plane's rows of B
+        const int slot = (int)((g + (lo - it.z0)) % kRing), n1 = min(hi - lo + 1, kRing - slot),
+                  n2 = hi - lo + 1 - n1;
+        const uint32_t d1 = tmem + slot * F;
+        // the first step one plane at a time: the plane that begins is overwritten
+        for (int j = 0; j < n1 + n2; ++j)
+          conv_mma(j < n1 ? d1 + j * F : tmem + (j - n1) * F, ad, bd + j * kB, conv_idesc(F),
+                   lo + j != zi + 1);
+        const uint32_t i1 = conv_idesc(n1 * F), i2 = conv_idesc(n2 * F);
+        if (n2 == 0) {
+#pragma unroll
+          for (int k = 1; k < 9 * (F / 16); ++k)
+            conv_mma(d1, ad + mid_a<F>(k), bd + mid_b<F>(k), i1, true);
+        } else {  // the planes wrap round the ring
+#pragma unroll
+          for (int k = 1; k < 9 * (F / 16); ++k) {
+            conv_mma(d1, ad + mid_a<F>(k), bd + mid_b<F>(k), i1, true);
+            conv_mma(tmem, ad + mid_a<F>(k), bd + mid_b<F>(k) + n1 * kB, i2, true);
+          }
+        }
+        conv_commit(empty + 8 * s);
+        if (zi - 1 >= it.z0) conv_commit(acc_full + 8 * (int)((g + (zi - 1 - it.z0)) % kRing));
+      }
+      g += it.z1 - it.z0;
+    }
+    conv_commit(drain);  // nothing in flight when the tensor memory is given back
+    ok &= conv_wait(drain, 0);
+  } else if (warp >= 2) {  // finished planes
+    const int q = warp & 3;  // the quarter of the lanes this warp may read
+    const int turn = (warp - 2) >> 2;
+    __nv_bfloat162 bs[F / 2];
+#pragma unroll
+    for (int c = 0; c < F / 2; ++c) bs[c] = __nv_bfloat162(bias[2 * c], bias[2 * c + 1]);
+    long long g = 0;
+    for (long long i = blockIdx.x; ok && i < wk.items; i += gridDim.x) {
+      const MidItem it = mid_item(d, wk, i);
+      const int x = it.x0 + (lane & 7), y = it.y0 + q * 4 + (lane >> 3);
+      const bool in = x < d.X && y < d.Y;
+      for (int z = it.z0; z < it.z1; ++z, ++g) {
+        if ((int)(g & 1) != turn) continue;
+        const int slot = (int)(g % kRing);
+        ok = __all_sync(0xffffffffu, conv_wait(acc_full + 8 * slot, (uint32_t)((g / kRing) & 1)));
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        uint32_t r[F];
+        const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16) + slot * F;
+#pragma unroll
+        for (int c = 0; c < F; c += 16)
+          asm volatile(
+              "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, "
+              "%11, %12, %13, %14, %15}, [%16];"
+              : "=r"(r[c]), "=r"(r[c + 1]), "=r"(r[c + 2]), "=r"(r[c + 3]), "=r"(r[c + 4]),
+                "=r"(r[c + 5]), "=r"(r[c + 6]), "=r"(r[c + 7]), "=r"(r[c + 8]), "=r"(r[c + 9]),
+                "=r"(r[c + 10]), "=r"(r[c + 11]), "=r"(r[c + 12]), "=r"(r[c + 13]), "=r"(r[c + 14]),
+                "=r"(r[c + 15])
+              : "r"(ta + c));
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) conv_arrive(acc_empty + 8 * slot);
+        if (in) {
+          uint4* o = reinterpret_cast<uint4*>(
+              out + ((((long long)it.b * d.Z + z) * d.Y + y) * d.X + x) * F);
+#pragma unroll
+          for (int c = 0; c < F; c += 8) {
+            unsigned p[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              p[j] = conv_act(__uint_as_float(r[c + 2 * j]), __uint_as_float(r[c + 2 * j + 1]),
+                              bs[c / 2 + j]);
+            o[c / 8] = make_uint4(p[0], p[1], p[2], p[3]);
+          }
+        }
+      }
+    }
+  }
+  __syncwarp();
+  if (!ok) *status = 1;
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  if (warp == 1)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(M::kCols));
+}
+
+// The weights as the three kernels read them: the B operands of the middle one's nine
+// (x, y) taps in their swizzled shared-memory layout (rows (output plane zi - 1, zi,
+// zi + 1; output channel), input channels along K), and the fragments of the first and
+// the last one's B operands, lane by lane.
+template <int F>
+struct ConvWs {
+  static constexpr int kIn = Mid<F>::kWeights;     // bytes before the first one's fragments
+  static constexpr int kInWords = F / 2;           // per lane
+  static constexpr int kOut = kIn + 32 * kInWords * 4;
+  static constexpr int kOutWords = F / 2;
+  static constexpr int kStatus = kOut + 32 * kOutWords * 4;
+};
+
+__device__ __forceinline__ bf16 conv_weight(const ConvW& w, int co, int ci, int kz, int ky, int kx) {
+  return w.w[co * w.s[0] + ci * w.s[1] + kz * w.s[2] + ky * w.s[3] + kx * w.s[4]];
+}
+
+template <int F>
+__global__ void conv_weights_kernel(ConvW w1, ConvW w2, ConvW w3, unsigned char* ws) {
+  typedef ConvWs<F> W;
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0) *reinterpret_cast<int*>(ws + W::kStatus) = 0;
+  if (i < 27 * F * F) {
+    const int ci = i % F, n = (i / F) % (3 * F), t = i / (3 * F * F);
+    const int sw = F == 32 ? (n >> 1) & 3 : (n >> 2) & 1;
+    reinterpret_cast<bf16*>(ws)[(t * Mid<F>::kTap + n * Mid<F>::kRow + (((ci >> 3) ^ sw) << 4)) / 2 + (ci & 7)] =
+        conv_weight(w2, n % F, ci, 2 - n / F, t / 3, t % 3);
+    return;
+  }
+  i -= 27 * F * F;
+  // element e of word j of a lane: column n = lane / 4, k pair lane % 4
+  if (i < 32 * W::kInWords * 2) {
+    const int e = i & 1, j = (i >> 1) % W::kInWords, lane = (i >> 1) / W::kInWords;
+    const int half = j & 1, ks = (j >> 1) & 1, t = j >> 2, n = lane >> 2, q = lane & 3;
+    const int tap = ks * 16 + 2 * q + 8 * half + e, c = F / 4 * (n >> 1) + 2 * t + (n & 1);
+    reinterpret_cast<bf16*>(ws + W::kIn)[i] =
+        tap < 27 ? conv_weight(w1, c, 0, tap / 9, tap / 3 % 3, tap % 3) : __float2bfloat16_rn(0.f);
+    return;
+  }
+  i -= 32 * W::kInWords * 2;
+  if (i < 32 * W::kOutWords * 2) {
+    const int e = i & 1, j = (i >> 1) % W::kOutWords, lane = (i >> 1) / W::kOutWords;
+    const int half = j & 1, ks = (j >> 1) % (F / 16), t = (j >> 1) / (F / 16), n = lane >> 2, q = lane & 3;
+    const int tap = 8 * t + n, c = F / 4 * q + 4 * ks + 2 * half + e;
+    reinterpret_cast<bf16*>(ws + W::kOut)[i] =
+        tap < 27 ? conv_weight(w3, 0, c, tap / 9, tap / 3 % 3, tap % 3) : __float2bfloat16_rn(0.f);
+  }
+}
+template <int F>
+constexpr int conv_weight_items() { return 27 * F * F + 32 * F * 2; }
+
+// F / 2 consecutive words of a lane
+template <int F>
+__device__ __forceinline__ void load_frags(unsigned (&r)[F / 2], const unsigned char* p, int lane) {
+  const uint4* q = reinterpret_cast<const uint4*>(p) + lane * (F / 8);
+#pragma unroll
+  for (int i = 0; i < F / 8; ++i) {
+    const uint4 v = q[i];
+    r[4 * i] = v.x; r[4 * i + 1] = v.y; r[4 * i + 2] = v.z; r[4 * i + 3] = v.w;
+  }
+}
+// F / 4 channels of a voxel: 8 or 16 bytes
+template <int F>
+struct Quarter {
+  unsigned w[F / 8];
+};
+template <int F>
+__device__ __forceinline__ Quarter<F> load_quarter(const bf16* p) {
+  Quarter<F> r;
+  if (F == 32) {
+    const uint4 v = __ldg(reinterpret_cast<const uint4*>(p));
+    r.w[0] = v.x; r.w[1] = v.y; r.w[F / 16] = v.z; r.w[F / 8 - 1] = v.w;
+  } else {
+    const uint2 v = __ldg(reinterpret_cast<const uint2*>(p));
+    r.w[0] = v.x; r.w[1] = v.y;
+  }
+  return r;
+}
+template <int F>
+__device__ __forceinline__ void store_quarter(bf16* p, const Quarter<F>& r) {
+  if (F == 32)
+    *reinterpret_cast<uint4*>(p) = make_uint4(r.w[0], r.w[1], r.w[F / 16], r.w[F / 8 - 1]);
+  else
+    *reinterpret_cast<uint2*>(p) = make_uint2(r.w[0], r.w[1]);
+}
+
+// ---- first convolution: one channel to F ----------------------------------------------
+// 27 taps padded to K = 32 and F columns: eight small matrix instructions per 16
+// voxels of a row leave the kernel to its writes of 2 F bytes per voxel (27 F FP32
+// multiply-adds per voxel took 0.26 ms at 2 x 128^3, this 0.060). The columns are permuted so
+// that a lane ends with F / 4 adjacent channels. A warp takes a row of 16 voxels and
+// walks along z.
+constexpr int kInX = 16, kInY = 8, kInZ = 16;
+
+template <int F>
+__global__ void __launch_bounds__(256) conv_in_kernel(const bf16* __restrict__ x,
+                                                      const unsigned char* __restrict__ wf,
+                                                      const bf16* __restrict__ bias,
+                                                      bf16* __restrict__ out, ConvDims d) {
+  constexpr int kPX = kInX + 2, kNT = F / 8;
+  __shared__ unsigned short in[(kInZ + 2) * (kInY + 2) * kPX];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, row = lane >> 2, q = lane & 3;
+  unsigned w[F / 2];
+  load_frags<F>(w, wf, lane);
+  __nv_bfloat162 bs[kNT];
+#pragma unroll
+  for (int t = 0; t < kNT; ++t) {
+    const int c = F / 4 * q + 2 * t;
+    bs[t] = __nv_bfloat162(bias[c], bias[c + 1]);
+  }
+  const int tx = (d.X + kInX - 1) / kInX, ty = (d.Y + kInY - 1) / kInY, tz = (d.Z + kInZ - 1) / kInZ;
+  long long id = blockIdx.x;
+  const int x0 = (int)(id % tx) * kInX;
+  id /= tx;
+  const int y0 = (int)(id % ty) * kInY;
+  id /= ty;
+  const int z0 = (int)(id % tz) * kInZ, b = (int)(id / tz);
+  const unsigned short* xs = reinterpret_cast<const unsigned short*>(x) + (long long)b * d.Z * d.Y * d.X;
+  for (int i = threadIdx.x; i < (kInZ + 2) * (kInY + 2) * kPX; i += 256) {
+    const int ix = i % kPX, iy = i / kPX % (kInY + 2), iz = i / (kPX * (kInY + 2));
+    const int gx = x0 + ix - 1, gy = y0 + iy - 1, gz = z0 + iz - 1;
+    in[i] = gx >= 0 && gx < d.X && gy >= 0 && gy < d.Y && gz >= 0 && gz < d.Z
+                ? xs[((long long)gz * d.Y + gy) * d.X + gx]
+                : (unsigned short)0;
+  }
+  // this lane's taps (2 per word; the padding's weights are zero)
+  int off[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const int tap = min((j >> 2) * 16 + 2 * q + (j >> 1 & 1) * 8 + (j & 1), 26);
+    off[j] = (tap / 9 * (kInY + 2) + tap / 3 % 3) * kPX + tap % 3 + warp * kPX + row;
+  }
+  __syncthreads();
+  const int gy = y0 + warp;
+  if (gy >= d.Y) return;
+  const bool in0 = x0 + row < d.X, in1 = x0 + row + 8 < d.X;
+  bf16* o = out + ((((long long)b * d.Z + z0) * d.Y + gy) * d.X + x0 + row) * F + F / 4 * q;
+  const int nz = min(kInZ, d.Z - z0);
+  for (int k = 0; k < nz; ++k, o += (long long)d.Y * d.X * F) {
+    const unsigned short* s = in + k * (kInY + 2) * kPX;
+    unsigned a[2][4];
+#pragma unroll
+    for (int ks = 0; ks < 2; ++ks)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {  // (row, row + 8) x (low, high half of k)
+        const unsigned short* r = s + (j & 1) * 8;
+        const int u = ks * 4 + (j >> 1) * 2;
+        a[ks][j] = (unsigned)r[off[u]] | (unsigned)r[off[u + 1]] << 16;
+      }
+    Quarter<F> r0, r1;
+#pragma unroll
+    for (int t = 0; t < kNT; ++t) {
+      float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int ks = 0; ks < 2; ++ks)
+        warp_mma(acc, a[ks][0], a[ks][1], a[ks][2], a[ks][3], w[(t * 2 + ks) * 2], w[(t * 2 + ks) * 2 + 1]);
+      r0.w[t] = conv_act(acc[0], acc[1], bs[t]);
+      r1.w[t] = conv_act(acc[2], acc[3], bs[t]);
+    }
+    if (in0) store_quarter<F>(o, r0);
+    if (in1) store_quarter<F>(o + 8 * F, r1);
+  }
+}
+
+// ---- last convolution: F channels to one ----------------------------------------------
+// Read once: the 27 products of a voxel's F channels with the taps' weights are a
+// matrix product of K = F and 32 columns; each output then adds 27 of them from
+// shared memory. A block walks down z over 16 x 16 outputs, with the products of one
+// plane's 18 x 18 voxels in shared memory (two planes, written and read in turn), its
+// next plane's voxels on their way in registers, and three outputs in progress.
+// 2 x 128^3, F = 32: 0.124 ms (0.38 with FP32 multiply-adds from a BF16 tile).
+constexpr int kOutT = 16, kOutM = (kOutT + 2) * (kOutT + 2);  // kOutM = 4 mod 16: no bank conflicts
+constexpr int kOutTiles = (kOutM + 15) / 16, kOutPerWarp = (kOutTiles + 7) / 8;
+constexpr int kOutSmem = 2 * 27 * kOutM * 4;
+
+template <int F>
+__global__ void __launch_bounds__(256) conv_out_kernel(const bf16* __restrict__ h,
+                                                       const unsigned char* __restrict__ wf,
+                                                       const bf16* __restrict__ bias,
+                                                       bf16* __restrict__ out, ConvDims d, int zc,
+                                                       const int* status) {
+  constexpr int kKS = F / 16;
+  extern __shared__ __align__(16) unsigned char conv_dyn[];
+  float* prod = reinterpret_cast<float*>(conv_dyn);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, row = lane >> 2, q = lane & 3;
+  unsigned w[F / 2];
+  load_frags<F>(w, wf, lane);
+  const int tx = (d.X + kOutT - 1) / kOutT, ty = (d.Y + kOutT - 1) / kOutT, tz = (d.Z + zc - 1) / zc;
+  long long id = blockIdx.x;
+  const int x0 = (int)(id % tx) * kOutT;
+  id /= tx;
+  const int y0 = (int)(id % ty) * kOutT;
+  id /= ty;
+  const int z0 = (int)(id % tz) * zc, z1 = min(d.Z, z0 + zc), b = (int)(id / tz);
+  const long long plane = (long long)d.X * d.Y;
+  const bf16* hb = h + (long long)b * d.Z * plane * F + F / 4 * q;
+  // this lane's voxels of a plane, -1 outside the volume
+  int off[kOutPerWarp][2];
+#pragma unroll
+  for (int i = 0; i < kOutPerWarp; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int m = (warp + 8 * i) * 16 + row + 8 * j;
+      const int gx = x0 + m % (kOutT + 2) - 1, gy = y0 + m / (kOutT + 2) - 1;
+      off[i][j] = m < kOutM && gx >= 0 && gx < d.X && gy >= 0 && gy < d.Y ? gy * d.X + gx : -1;
+    }
+  Quarter<F> a[kOutPerWarp][2];
+  const auto fetch = [&](int z) {
+#pragma unroll
+    for (int i = 0; i < kOutPerWarp; ++i)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        if (off[i][j] >= 0 && z >= 0 && z < d.Z) {
+          a[i][j] = load_quarter<F>(hb + (z * plane + off[i][j]) * F);
+        } else {
+#pragma unroll
+          for (int c = 0; c < F / 8; ++c) a[i][j].w[c] = 0u;
+        }
+      }
+  };
+  fetch(z0 - 1);
+  const int lx = threadIdx.x % kOutT, ly = threadIdx.x / kOutT;
+  const int gx = x0 + lx, gy = y0 + ly;
+  const bool in = gx < d.X && gy < d.Y, bad = *status != 0;  // a wait of the middle one ran out
+  const float bs = __bfloat162float(bias[0]);
+  bf16* o = out + (long long)b * d.Z * plane + (long long)gy * d.X + gx;
+  float s0 = 0.f, s1 = 0.f;  // outputs z - 1 and z
+  for (int z = z0 - 1; z <= z1; ++z) {
+    float* p = prod + ((z - z0 + 1) & 1) * 27 * kOutM;
+#pragma unroll
+    for (int i = 0; i < kOutPerWarp; ++i) {
+      const int m = (warp + 8 * i) * 16 + row;
+      if (warp + 8 * i < kOutTiles) {
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+          for (int ks = 0; ks < kKS; ++ks)
+            warp_mma(acc, a[i][0].w[2 * ks], a[i][1].w[2 * ks], a[i][0].w[2 * ks + 1],
+                     a[i][1].w[2 * ks + 1], w[(t * kKS + ks) * 2], w[(t * kKS + ks) * 2 + 1]);
+          const int tap = 8 * t + 2 * q;
+          if (tap < 27) {
+            float* r = p + tap * kOutM + m;
+            if (m < kOutM) r[0] = acc[0];
+            if (m + 8 < kOutM) r[8] = acc[2];
+            if (tap + 1 < 27) {
+              if (m < kOutM) r[kOutM] = acc[1];
+              if (m + 8 < kOutM) r[kOutM + 8] = acc[3];
+            }
+          }
+        }
+      }
+    }
+    if (z < z1) fetch(z + 1);
+    __syncthreads();
+    float t[3] = {0.f, 0.f, 0.f};
+    const float* r = p + ly * (kOutT + 2) + lx;
+#pragma unroll
+    for (int kz = 0; kz < 3; ++kz)
+#pragma unroll
+      for (int k = 0; k < 9; ++k)
+        t[kz] += r[(kz * 9 + k) * kOutM + k / 3 * (kOutT + 2) + k % 3];
+    const float done = s0 + t[2];  // output z - 1
+    s0 = s1 + t[1];
+    s1 = t[0];
+    if (in && z - 1 >= z0)
+      o[(z - 1) * plane] = __float2bfloat16_rn(bad ? __int_as_float(0x7fffffff) : round_bf16(done) + bs);
+  }
+}
+
+typedef CUresult (*ConvEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
+                                 const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                                 const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                 CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+template <int F>
+int conv_block(const bf16* x, const ConvW* w, const bf16* const* bias, bf16* h1, bf16* h2, bf16* y,
+               unsigned char* ws, const ConvDims& d, cudaStream_t st) {
+  typedef Mid<F> M;
+  static const ConvEncodeFn enc = [] {
+    void* ptr = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess)
+      ptr = nullptr;
+    return reinterpret_cast<ConvEncodeFn>(ptr);
+  }();
+  if (!enc) return fail(DTV_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
+  CUtensorMap map;
+  const cuuint64_t row = M::kRow;
+  const cuuint64_t dims[5] = {(cuuint64_t)F, (cuuint64_t)d.X, (cuuint64_t)d.Y, (cuuint64_t)d.Z,
+                              (cuuint64_t)d.B};
+  const cuuint64_t strides[4] = {row, row * d.X, row * d.X * d.Y, row * d.X * d.Y * d.Z};
+  const cuuint32_t box[5] = {F, kCX, kCY + 2, 1, 1}, es[5] = {1, 1, 1, 1, 1};
+  const CUresult r =
+      enc(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, h1, dims, strides, box, es,
+          CU_TENSOR_MAP_INTERLEAVE_NONE,
+          F == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B,
+          CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(DTV_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
+  DTV_CUDA_TRY(cudaFuncSetAttribute(conv_mid_kernel<F>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    M::kSmem));
+  DTV_CUDA_TRY(cudaFuncSetAttribute(conv_out_kernel<F>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    kOutSmem));
+  int dev = 0, sms = 0;
+  DTV_CUDA_TRY(cudaGetDevice(&dev));
+  DTV_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  int* status = reinterpret_cast<int*>(ws + ConvWs<F>::kStatus);
+
+  conv_weights_kernel<F><<<(conv_weight_items<F>() + 255) / 256, 256, 0, st>>>(w[0], w[1], w[2], ws);
+  note_launch();
+  DTV_LAUNCH_CHECK();
+
+  const auto up = [](int n, int t) { return (long long)((n + t - 1) / t); };
+  const long long nin = up(d.X, kInX) * up(d.Y, kInY) * up(d.Z, kInZ) * d.B;
+  const long long columns = up(d.X, kOutT) * up(d.Y, kOutT) * d.B;
+  // z chunks of the last convolution: four blocks or so for each of an SM's places
+  const int zc = (int)std::max<long long>(4, std::min<long long>(32, d.Z * columns / (sms * 12)));
+  const long long nout = columns * up(d.Z, zc);
+  DTV_CHECK(nin < (1ll << 31) && nout < (1ll << 31), "volume too large");
+  conv_in_kernel<F><<<(unsigned)nin, 256, 0, st>>>(x, ws + ConvWs<F>::kIn, bias[0], h1, d);
+  note_launch();
+  DTV_LAUNCH_CHECK();
+
+  // z chunks: a block pays two halo planes per chunk; the length with the fewest
+  // planes in the longest block
+  MidWork wk;
+  wk.tx = (int)up(d.X, kCX);
+  wk.ty = (int)up(d.Y, kCY);
+  long long best = -1;
+  for (int c = 1; c <= d.Z && c <= 64; ++c) {
+    const int len = (d.Z + c - 1) / c, chunks = (d.Z + len - 1) / len;
+    const long long items = (long long)wk.tx * wk.ty * d.B * chunks;
+    const long long cost = (items + sms - 1) / sms * (len + 2);
+    if (best < 0 || cost < best) {
+      best = cost;
+      wk.zc = len;
+      wk.nzc = chunks;
+      wk.items = items;
+    }
+  }
+  conv_mid_kernel<F><<<(unsigned)std::min<long long>(wk.items, sms), kMidThreads, M::kSmem, st>>>(
+      map, ws, bias[1], h2, d, wk, status);
+  note_launch();
+  DTV_LAUNCH_CHECK();
+  conv_out_kernel<F><<<(unsigned)nout, 256, kOutSmem, st>>>(h2, ws + ConvWs<F>::kOut, bias[2], y, d, zc,
+                                                            status);
+  note_launch();
+  DTV_LAUNCH_CHECK();
+  return DTV_OK;
+}
+
+}  // namespace
+}  // namespace dtv
+
+using namespace dtv;
+
+int64_t dtv_conv_block_workspace_bytes(int32_t features) {
+  return (int64_t)27 * features * features * 2 + 32 * features * 4 + 16;
+}
+
+int dtv_conv_block(const void* x, const void* const weights[3], const int64_t strides[15],
+                   const void* const biases[3], void* h1, void* h2, void* y, const int32_t size[3],
+                   int32_t batch, int32_t features, void* workspace, void* stream) {
+  DTV_CHECK(x && weights && strides && biases && h1 && h2 && y && size && workspace, "NULL argument");
+  DTV_CHECK(size[0] > 0 && size[1] > 0 && size[2] > 0 && batch > 0, "empty volume");
+  DTV_CHECK(features == 16 || features == 32, "features must be 16 or 32");
+  ConvW w[3];
+  const bf16* bias[3];
+  for (int i = 0; i < 3; ++i) {
+    DTV_CHECK(weights[i] && biases[i], "NULL argument");
+    w[i].w = static_cast<const bf16*>(weights[i]);
+    for (int k = 0; k < 5; ++k) w[i].s[k] = strides[5 * i + k];
+    bias[i] = static_cast<const bf16*>(biases[i]);
+  }
+  DTV_CHECK(((uintptr_t)h1 | (uintptr_t)h2 | (uintptr_t)workspace) % 16 == 0, "buffers must be 16-byte aligned");
+  const ConvDims d{size[0], size[1], size[2], batch};
+  return (features == 32 ? conv_block<32> : conv_block<16>)(
+      static_cast<const bf16*>(x), w, bias, static_cast<bf16*>(h1), static_cast<bf16*>(h2),
+      static_cast<bf16*>(y), static_cast<unsigned char*>(workspace), d, static_cast<cudaStream_t>(stream));
+}

@@ -1,0 +1,122 @@
+"""The convolution block Conv3d(1, f) - ReLU - Conv3d(f, f) - ReLU - Conv3d(f, 1) in
+BF16 through the library's kernels (csrc/conv.cu)."""
+from __future__ import annotations
+
+import ctypes
+
+import torch
+import torch.nn as nn
+import torch.nn.functional as F
+
+from . import _lib
+from .geometry import _ptr, _stream
+
+_CONVS = (0, 2, 4)  # of the block's modules
+
+
+def _plain(m: nn.Module, kind) -> bool:
+    """A module of exactly this class whose call runs its class's forward alone."""
+    return (type(m) is kind and "forward" not in m.__dict__ and not m._forward_hooks
+            and not m._forward_pre_hooks and not m._backward_hooks and not m._backward_pre_hooks)
+
+
+def _special_modes() -> bool:
+    """Whether something watches or transforms the calls made here: tracing, functorch,
+    forward-mode differentiation, dispatch and function modes, global module hooks."""
+    return (torch.compiler.is_compiling() or torch.jit.is_tracing()
+            or torch._C._functorch.peek_interpreter_stack() is not None
+            or torch.autograd.forward_ad._current_level >= 0
+            or torch._C._len_torch_dispatch_stack() > 0
+            or torch._C._len_torch_function_stack() > 0
+            or torch.nn.modules.module._has_any_global_hook())
+
+
+def supported(body: nn.Sequential, x: torch.Tensor) -> bool:
+    """Whether the block's call is one that the kernels compute: FP32 input and weights
+    on a GPU under BF16 autocast, 16 or 32 features (the weights of all taps stay in
+    shared memory), the block as it was built."""
+    if not (type(x) is torch.Tensor and x.is_cuda and x.dtype == torch.float32 and x.dim() == 5
+            and x.shape[1] == 1 and x.numel() > 0 and torch.is_autocast_enabled("cuda")
+            and torch.get_autocast_dtype("cuda") == torch.bfloat16):
+        return False
+    if _special_modes() or not _plain(body, nn.Sequential) or len(body) != 5:
+        return False
+    f = body[0].out_channels if type(body[0]) is nn.Conv3d else 0
+    if f not in (16, 32) or not (_plain(body[1], nn.ReLU) and _plain(body[3], nn.ReLU)):
+        return False
+    if max(x.shape) >= 1 << 24 or x.numel() >= 1 << 32:
+        return False
+    for i, (ci, co) in zip(_CONVS, ((1, f), (f, f), (f, 1))):
+        m = body[i]
+        if not (_plain(m, nn.Conv3d) and m.kernel_size == (3, 3, 3) and m.stride == (1, 1, 1)
+                and m.padding == (1, 1, 1) and m.dilation == (1, 1, 1) and m.groups == 1
+                and m.padding_mode == "zeros" and m.bias is not None):
+            return False
+        for p, shape in ((m.weight, (co, ci, 3, 3, 3)), (m.bias, (co,))):
+            if not (type(p) in (torch.Tensor, nn.Parameter) and p.dtype == torch.float32
+                    and p.device == x.device and p.shape == shape):
+                return False
+    return True
+
+
+def _reference(x, w1, b1, w2, b2, w3, b3):
+    h = F.relu(F.conv3d(x, w1, b1, padding=1))
+    h = F.relu(F.conv3d(h, w2, b2, padding=1))
+    return F.conv3d(h, w3, b3, padding=1)
+
+
+def _conv_grads(g, x, w, need):
+    return torch.ops.aten.convolution_backward(g, x, w, [w.shape[0]], [1] * 3, [1] * 3, [1] * 3,
+                                               False, [0] * 3, 1, need)
+
+
+class _Block(torch.autograd.Function):
+    """x, weights and biases in BF16."""
+
+    @staticmethod
+    def forward(ctx, x, *params):
+        x_ = x.contiguous()
+        w = [p.detach() for p in params[0::2]]
+        b = [p.detach().contiguous() for p in params[1::2]]
+        B, _, Z, Y, X = x.shape
+        f = w[0].shape[0]
+        new = dict(dtype=torch.bfloat16, device=x.device, memory_format=torch.channels_last_3d)
+        h1, h2 = torch.empty((B, f, Z, Y, X), **new), torch.empty((B, f, Z, Y, X), **new)
+        y = torch.empty((B, 1, Z, Y, X), **new)
+        ws = torch.empty(_lib.load().dtv_conv_block_workspace_bytes(f), dtype=torch.uint8,
+                         device=x.device)
+        strides = (ctypes.c_int64 * 15)(*[s for t in w for s in t.stride()])
+        with torch.cuda.device(x.device):
+            _lib.call("dtv_conv_block", _ptr(x_), (ctypes.c_void_p * 3)(*[t.data_ptr() for t in w]),
+                      strides, (ctypes.c_void_p * 3)(*[t.data_ptr() for t in b]), _ptr(h1), _ptr(h2),
+                      _ptr(y), _lib.ivec((X, Y, Z)), B, f, _ptr(ws), _stream(x.device))
+        ctx.save_for_backward(x, *params, h1, h2)
+        return y
+
+    @staticmethod
+    def backward(ctx, gy):
+        x, w1, b1, w2, b2, w3, b3, h1, h2 = ctx.saved_tensors
+        need = ctx.needs_input_grad
+        if torch.is_grad_enabled():  # a differentiable gradient was asked for
+            with torch.autocast("cuda", enabled=False):
+                args = [x, w1, b1, w2, b2, w3, b3]
+                y = _reference(*args)
+                wanted = [a for a, n in zip(args, need) if n]
+                got = iter(torch.autograd.grad(y, wanted, gy, create_graph=True, allow_unused=True))
+            return tuple(next(got) if n else None for n in need)
+        low = any(need[:5])  # anything below the last convolution
+        g, gw3, gb3 = _conv_grads(gy, h2, w3, [low, need[5], need[6]])
+        gx = gw1 = gb1 = gw2 = gb2 = None
+        if low:
+            g = torch.ops.aten.threshold_backward(g, h2, 0)
+            low = any(need[:3])
+            g, gw2, gb2 = _conv_grads(g, h1, w2, [low, need[3], need[4]])
+            if low:
+                g = torch.ops.aten.threshold_backward(g, h1, 0)
+                gx, gw1, gb1 = _conv_grads(g, x, w1, list(need[:3]))
+        return gx, gw1, gb1, gw2, gb2, gw3, gb3
+
+
+def conv_block(body: nn.Sequential, x: torch.Tensor) -> torch.Tensor:
+    params = [p.to(torch.bfloat16) for i in _CONVS for p in (body[i].weight, body[i].bias)]
+    return _Block.apply(x.to(torch.bfloat16), *params)

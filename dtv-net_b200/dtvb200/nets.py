@@ -31,6 +31,7 @@ import torch
 import torch.nn as nn
 from torch.utils.checkpoint import checkpoint
 
+from . import conv
 from .ops import Projector, make_functions
 from .tv import diff
 
@@ -238,7 +239,9 @@ class LEARN(_Cascades):
 
 class ConvBlock(nn.Module):
     """Conv3d(1, f) - ReLU - Conv3d(f, f) - ReLU - Conv3d(f, 1), 3x3x3 kernels
-    (the shape of model/PDHG/RegularizationLayers/CNN.py:4-18 with three layers)."""
+    (the shape of model/PDHG/RegularizationLayers/CNN.py:4-18 with three layers).
+    Under BF16 autocast on a GPU the library's kernels compute it where they can
+    (conv.supported)."""
 
     def __init__(self, features: int = 32):
         super().__init__()
@@ -248,6 +251,8 @@ class ConvBlock(nn.Module):
             nn.Conv3d(features, 1, 3, padding=1))
 
     def forward(self, x):
+        if conv.supported(self.body, x):
+            return conv.conv_block(self.body, x)
         return self.body(x)
 
 

@@ -456,6 +456,17 @@ DTV_API int dtv_axpy_l1(float* f, const float* bp, float beta, double* l1, int64
 DTV_API int dtv_tv_descent(const float* f_in, float* f_out, const int32_t size[3], int32_t batch,
                    int32_t quirk, const float* davg, void* stream);
 
+/* Forward pass of the convolution block Conv3d(1,F) - ReLU - Conv3d(F,F) - ReLU -
+ * Conv3d(F,1) (3x3x3, zero padding; model/PDHG/RegularizationLayers/CNN.py:4-18) in
+ * BF16 with FP32 sums, F = features = 16 or 32. x, y: [batch, Z, Y, X]; h1, h2 (the
+ * activations after each ReLU, 16-byte aligned): [batch, Z, Y, X, F]; weights[i]:
+ * [out, in, 3, 3, 3] with element strides strides[5i..5i+4]. workspace: device memory,
+ * 16-byte aligned, of dtv_conv_block_workspace_bytes(F). */
+DTV_API int64_t dtv_conv_block_workspace_bytes(int32_t features);
+DTV_API int dtv_conv_block(const void* x, const void* const weights[3], const int64_t strides[15],
+                   const void* const biases[3], void* h1, void* h2, void* y, const int32_t size[3],
+                   int32_t batch, int32_t features, void* workspace, void* stream);
+
 /* out[0] = (float)(in[0] * scale) on the device (scalar glue that keeps
  * data-dependent step sizes such as davg = alpha * dp on the GPU, ASDPOCS.py:35). */
 DTV_API int dtv_scale_scalar(const double* in, double scale, float* out, void* stream);
