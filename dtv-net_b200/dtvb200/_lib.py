@@ -115,6 +115,10 @@ SIGNATURES = {
     "dtv_conv_block_workspace_bytes": [_I],
     "dtv_conv_block": [_P, ctypes.POINTER(_P), ctypes.POINTER(_L), ctypes.POINTER(_P), _P, _P, _P,
                        _IP, _I, _I, _P, _P],
+    "dtv_conv_block_backward_workspace_bytes": [_IP, _I, _I],
+    "dtv_conv_block_backward": [_P, _P, ctypes.POINTER(_P), ctypes.POINTER(_L), _P, _P, _P, _P, _P,
+                                ctypes.POINTER(_P), ctypes.POINTER(_L), ctypes.POINTER(_P), _IP, _I,
+                                _I, _P, _P],
     "dtv_tv_descent": [_P, _P, _IP, _I, _I, _P, _P],
     "dtv_scale_scalar": [_P, _D, _P, _P],
     "dtv_l1_distance": [_P, _P, _L, _P, _P],
@@ -129,6 +133,7 @@ _RESTYPES = {
     "dtv_error_string": ctypes.c_char_p,
     "dtv_last_error_message": ctypes.c_char_p,
     "dtv_conv_block_workspace_bytes": ctypes.c_int64,
+    "dtv_conv_block_backward_workspace_bytes": ctypes.c_int64,
     "dtv_l1ball_workspace_bytes": ctypes.c_int64,
     "dtv_launch_count": ctypes.c_int64,
     "dtv_pdhg_workspace_bytes": ctypes.c_int64,

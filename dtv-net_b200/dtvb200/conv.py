@@ -65,9 +65,12 @@ def _reference(x, w1, b1, w2, b2, w3, b3):
     return F.conv3d(h, w3, b3, padding=1)
 
 
-def _conv_grads(g, x, w, need):
-    return torch.ops.aten.convolution_backward(g, x, w, [w.shape[0]], [1] * 3, [1] * 3, [1] * 3,
-                                               False, [0] * 3, 1, need)
+def _pointers(ts):
+    return (ctypes.c_void_p * 3)(*[None if t is None else t.data_ptr() for t in ts])
+
+
+def _strides(ts):
+    return (ctypes.c_int64 * 15)(*[s for t in ts for s in t.stride()])
 
 
 class _Block(torch.autograd.Function):
@@ -85,11 +88,9 @@ class _Block(torch.autograd.Function):
         y = torch.empty((B, 1, Z, Y, X), **new)
         ws = torch.empty(_lib.load().dtv_conv_block_workspace_bytes(f), dtype=torch.uint8,
                          device=x.device)
-        strides = (ctypes.c_int64 * 15)(*[s for t in w for s in t.stride()])
         with torch.cuda.device(x.device):
-            _lib.call("dtv_conv_block", _ptr(x_), (ctypes.c_void_p * 3)(*[t.data_ptr() for t in w]),
-                      strides, (ctypes.c_void_p * 3)(*[t.data_ptr() for t in b]), _ptr(h1), _ptr(h2),
-                      _ptr(y), _lib.ivec((X, Y, Z)), B, f, _ptr(ws), _stream(x.device))
+            _lib.call("dtv_conv_block", _ptr(x_), _pointers(w), _strides(w), _pointers(b), _ptr(h1),
+                      _ptr(h2), _ptr(y), _lib.ivec((X, Y, Z)), B, f, _ptr(ws), _stream(x.device))
         ctx.save_for_backward(x, *params, h1, h2)
         return y
 
@@ -104,17 +105,28 @@ class _Block(torch.autograd.Function):
                 wanted = [a for a, n in zip(args, need) if n]
                 got = iter(torch.autograd.grad(y, wanted, gy, create_graph=True, allow_unused=True))
             return tuple(next(got) if n else None for n in need)
-        low = any(need[:5])  # anything below the last convolution
-        g, gw3, gb3 = _conv_grads(gy, h2, w3, [low, need[5], need[6]])
-        gx = gw1 = gb1 = gw2 = gb2 = None
-        if low:
-            g = torch.ops.aten.threshold_backward(g, h2, 0)
-            low = any(need[:3])
-            g, gw2, gb2 = _conv_grads(g, h1, w2, [low, need[3], need[4]])
-            if low:
-                g = torch.ops.aten.threshold_backward(g, h1, 0)
-                gx, gw1, gb1 = _conv_grads(g, x, w1, list(need[:3]))
-        return gx, gw1, gb1, gw2, gb2, gw3, gb3
+        B, _, Z, Y, X = x.shape
+        f = w1.shape[0]
+        last = dict(memory_format=torch.channels_last_3d)
+        h1, h2 = h1.contiguous(**last), h2.contiguous(**last)
+        gy, x_ = gy.contiguous(), x.contiguous()
+        w = [w1, w2, w3]
+        gw = [torch.empty_like(t) if n else None for t, n in zip(w, need[1::2])]
+        gb = [torch.empty_like(t) if n else None for t, n in zip((b1, b2), need[2:5:2])]
+        gx = torch.empty_like(x_) if need[0] else None
+        g2 = torch.empty_like(h2) if any(need[:5]) else None
+        g1 = torch.empty_like(h1) if any(need[:3]) else None
+        size = _lib.ivec((X, Y, Z))
+        with torch.cuda.device(x.device):
+            ws = torch.empty(_lib.load().dtv_conv_block_backward_workspace_bytes(size, B, f),
+                             dtype=torch.uint8, device=x.device)
+            _lib.call("dtv_conv_block_backward", _ptr(gy), _ptr(x_), _pointers(w), _strides(w), _ptr(h1),
+                      _ptr(h2), None if g1 is None else _ptr(g1), None if g2 is None else _ptr(g2),
+                      None if gx is None else _ptr(gx), _pointers(gw),
+                      _strides([t if g is None else g for t, g in zip(w, gw)]), _pointers(gb + [None]),
+                      size, B, f, _ptr(ws), _stream(x.device))
+        gb3 = gy.sum((0, 2, 3, 4)) if need[6] else None
+        return gx, gw[0], gb[0], gw[1], gb[1], gw[2], gb3
 
 
 def conv_block(body: nn.Sequential, x: torch.Tensor) -> torch.Tensor:

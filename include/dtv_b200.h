@@ -467,6 +467,19 @@ DTV_API int dtv_conv_block(const void* x, const void* const weights[3], const in
                    const void* const biases[3], void* h1, void* h2, void* y, const int32_t size[3],
                    int32_t batch, int32_t features, void* workspace, void* stream);
 
+/* Gradients of dtv_conv_block: from gy, that of y, those of x (gx), of the weights
+ * (grad_weights[i] with strides as for weights) and of the first two biases
+ * (grad_biases[2] must be NULL: it is the sum of gy). NULL leaves one out. g1, g2: room
+ * for the gradients before the ReLUs, like h1 and h2; g2 may be NULL if only
+ * grad_weights[2] is wanted, g1 if nothing of the first convolution is. */
+DTV_API int64_t dtv_conv_block_backward_workspace_bytes(const int32_t size[3], int32_t batch,
+                   int32_t features);
+DTV_API int dtv_conv_block_backward(const void* gy, const void* x, const void* const weights[3],
+                   const int64_t strides[15], const void* h1, const void* h2, void* g1, void* g2,
+                   void* gx, void* const grad_weights[3], const int64_t grad_strides[15],
+                   void* const grad_biases[3], const int32_t size[3], int32_t batch,
+                   int32_t features, void* workspace, void* stream);
+
 /* out[0] = (float)(in[0] * scale) on the device (scalar glue that keeps
  * data-dependent step sizes such as davg = alpha * dp on the GPU, ASDPOCS.py:35). */
 DTV_API int dtv_scale_scalar(const double* in, double scale, float* out, void* stream);

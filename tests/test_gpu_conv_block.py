@@ -70,6 +70,27 @@ def test_block(cuda, size, features, batch, last):
         assert g.dtype == r.dtype and _rel(g, r) < 2.0 ** -6
 
 
+@pytest.mark.parametrize("wanted", [("x",), ("body.4.weight",), ("body.4.bias",), ("body.2.bias",),
+                                    ("body.2.weight", "body.4.bias"), ("body.0.bias", "x"),
+                                    ("body.0.weight",)])
+def test_some_gradients(cuda, wanted):
+    """Any subset of the gradients has the bits it has among all of them."""
+    torch.manual_seed(4)
+    block = ConvBlock(16).to(cuda)
+    x = torch.randn(1, 1, 9, 18, 20, device=cuda, requires_grad=True)
+    named = {"x": x, **dict(block.named_parameters())}
+    with torch.autocast("cuda", dtype=bf):
+        y = block(x)
+    gy = torch.randn_like(y)
+    full = dict(zip(named, torch.autograd.grad(y, list(named.values()), gy)))
+    for k, t in named.items():
+        t.requires_grad_(k in wanted)
+    with torch.autocast("cuda", dtype=bf), torch.autograd.graph.save_on_cpu():
+        y = block(x)
+    for k, g in zip(wanted, torch.autograd.grad(y, [named[k] for k in wanted], gy)):
+        assert torch.equal(g, full[k]), k
+
+
 def test_what_stays_general(cuda):
     block = ConvBlock(16).to(cuda)
     x = torch.randn(1, 1, 6, 5, 7, device=cuda)
