@@ -4,9 +4,9 @@
 // Activations are channels-last, [batch, z, y, x, F]. Each convolution sums in
 // FP32 and is rounded to BF16, then the BF16 bias is added and rounded again: the
 // roundings that autocast makes around a library convolution.
-// Measured at 2 x 128^3, F = 32: 0.50 ms (0.06 + 0.30 + 0.12 and the weights), where
+// Measured at 2 x 128^3, F = 32: 0.42 ms (0.06 + 0.22 + 0.12 and the weights), where
 // three library convolutions with their layout conversions, bias additions and ReLUs
-// took 4.1 ms; F = 16: 0.37 ms. Backward, all gradients: 1.2 ms, the library's 8.4.
+// took 4.1 ms; F = 16: 0.28 ms. Backward, all gradients: 1.05 ms, the library's 8.4.
 // Gradients are rounded to BF16 where autocast's are: the data gradients after each
 // convolution, the weight and bias gradients once summed. Sums are FP32 in an order
 // fixed by the sizes and the number of SMs.
@@ -63,14 +63,20 @@ __device__ __forceinline__ void warp_mma(float (&d)[4], unsigned a0, unsigned a1
 // 3F columns adds an input plane's share to the three output planes around it,
 // which lie side by side in a ring of kRing accumulators in tensor memory. Reading
 // A once for three planes is what makes the step arithmetic-bound: with F columns
-// an instruction waits on its 4 KB of A. 2 x 128^3, F = 32: 0.297 ms, 0.78 PFLOP/s
-// (0.63 ms while the issuing thread built each descriptor and one set of four warps
-// wrote; the library's kernel 1.03 ms).
-// Warp 0 loads, warp 1 issues, warps 2-5 and 6-9 write finished planes in turn.
+// an instruction waits on its 4 KB of A. 2 x 128^3, F = 32: 0.223 ms, 1.04 PFLOP/s
+// (F = 16: 0.120); the library's kernel 1.03 ms. On the way: 0.63 ms while one thread
+// built each descriptor, 0.30 with them precomputed, 0.28 with the whole warp in the
+// loop and one lane elected per instruction. Not faster: one unswizzled copy of a
+// plane addressed at odd offsets (cp.async, a third of the loads; 0.30), two
+// accumulators per plane (0.32).
+// Two columns at a time, each with a warp that loads, one that issues and four that
+// write finished planes: the issue of a plane's instructions and its waits take longer
+// than the tensor core takes for them.
 constexpr int kCX = 8, kCY = 16;   // column: rows of 8 voxels, one swizzle atom each
-constexpr int kRing = 16;          // accumulators
-constexpr int kStages = 4;         // input planes in flight
-constexpr int kMidThreads = 320;
+constexpr int kPipes = 2;          // columns a block works on
+constexpr int kRing = 8;           // accumulators of a column
+constexpr int kStages = 3;         // input planes in flight of a column
+constexpr int kMidThreads = kPipes * (64 + 128);
 constexpr unsigned kConvWaitLimit = 1u << 20;  // polls of one wait
 
 template <int F>
@@ -81,8 +87,8 @@ struct Mid {
   static constexpr int kTap = 3 * F * kRow;                 // B operand of an (x, y) tap
   static constexpr int kWeights = 9 * kTap;
   static constexpr int kFirst = (kWeights + 1023) / 1024 * 1024;  // of the stages
-  static constexpr int kSmem = 1024 + kFirst + kStages * kStage;
-  static constexpr int kCols = F * kRing;                   // tensor-memory columns
+  static constexpr int kSmem = 1024 + kFirst + kPipes * kStages * kStage;
+  static constexpr int kCols = kPipes * F * kRing;          // tensor-memory columns
   static constexpr unsigned long long kLayout = F == 32 ? 4ull : 6ull;  // 64- / 32-byte swizzle
 };
 
@@ -112,9 +118,22 @@ __device__ __forceinline__ void conv_expect(uint32_t bar, unsigned bytes) {
                : "memory");
 }
 // all matrix instructions issued so far arrive on bar when they are done
-__device__ __forceinline__ void conv_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
-               : "memory");
+__device__ __forceinline__ void conv_commit(uint32_t bar, uint32_t elected) {
+  asm volatile(
+      "{\n .reg .pred e;\n setp.ne.u32 e, %1, 0;\n"
+      " @e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(bar),
+      "r"(elected)
+      : "memory");
+}
+// one lane of the warp, the same at each call
+__device__ __forceinline__ uint32_t conv_elect() {
+  uint32_t e;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(e));
+  return e;
+}
+// the whole warp waits
+__device__ __forceinline__ bool conv_wait_all(uint32_t bar, uint32_t parity) {
+  return __all_sync(0xffffffffu, conv_wait(bar, parity));
 }
 // K-major operand descriptor, 8-row atoms one after another
 template <int F>
@@ -128,11 +147,11 @@ __device__ __forceinline__ uint32_t conv_idesc(int n) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | (8u << 24);
 }
 __device__ __forceinline__ void conv_mma(uint32_t d, unsigned long long a, unsigned long long b,
-                                         uint32_t idesc, bool add) {
+                                         uint32_t idesc, bool add, uint32_t elected) {
   asm volatile(
-      "{\n .reg .pred p;\n setp.ne.u32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
-      "l"(a), "l"(b), "r"(idesc), "r"((uint32_t)add)
+      "{\n .reg .pred p, e;\n setp.ne.u32 p, %4, 0;\n setp.ne.u32 e, %5, 0;\n"
+      " @e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
+      "l"(a), "l"(b), "r"(idesc), "r"((uint32_t)add), "r"(elected)
       : "memory");
 }
 
@@ -145,6 +164,17 @@ __device__ constexpr unsigned mid_a(int k) {
 template <int F>
 __device__ constexpr unsigned mid_b(int k) {
   return (k / (F / 16) * Mid<F>::kTap + 32 * (k % (F / 16))) / 16;
+}
+
+// 16 columns of this warp's lanes
+__device__ __forceinline__ void tmem_load16(uint32_t* r, uint32_t addr) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, "
+      "%13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
+        "=r"(r[15])
+      : "r"(addr));
 }
 
 struct MidItem {
@@ -167,19 +197,22 @@ __device__ __forceinline__ MidItem mid_item(const ConvDims& d, const MidWork& w,
 template <int F, bool kMask>
 __global__ void __launch_bounds__(kMidThreads, 1)
     conv_mid_kernel(const __grid_constant__ CUtensorMap map, const unsigned char* __restrict__ wimg,
-                    const bf16* __restrict__ bias, const bf16* __restrict__ act, bf16* __restrict__ out, ConvDims d, MidWork wk,
-                    int* status) {
+                    const bf16* __restrict__ bias, const bf16* __restrict__ act, bf16* __restrict__ out,
+                    ConvDims d, MidWork wk, int* status) {
   typedef Mid<F> M;
   extern __shared__ unsigned char conv_dyn[];
-  __shared__ __align__(8) unsigned long long bars[2 * kStages + 2 * kRing + 2];
+  __shared__ __align__(8) unsigned long long bars[kPipes * (2 * kStages + 2 * kRing + 1) + 1];
   __shared__ uint32_t tmem_slot;
   const uint32_t base = (conv_smem(conv_dyn) + 1023u) & ~1023u;
-  const uint32_t wsm = base, stages = base + M::kFirst;
-  const uint32_t bar0 = conv_smem(bars);
+  // (the shuffle tells the compiler that a warp's number is the same in all its lanes)
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int pipe = warp < 2 * kPipes ? warp >> 1 : (warp - 2 * kPipes) >> 2;
+  const uint32_t wsm = base, stages = base + M::kFirst + pipe * kStages * M::kStage;
+  const uint32_t wbar = conv_smem(bars), bar0 = wbar + 8 + pipe * 8 * (2 * kStages + 2 * kRing + 1);
   const uint32_t full = bar0, empty = full + 8 * kStages, acc_full = empty + 8 * kStages,
-                 acc_empty = acc_full + 8 * kRing, wbar = acc_empty + 8 * kRing, drain = wbar + 8;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (threadIdx.x == 0) {
+                 acc_empty = acc_full + 8 * kRing, drain = acc_empty + 8 * kRing;
+  if (threadIdx.x == 0) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(wbar) : "memory");
+  if (warp < 2 * kPipes && (threadIdx.x & 63) == 0) {
     for (int i = 0; i < kStages; ++i) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(full + 8 * i) : "memory");
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(empty + 8 * i) : "memory");
@@ -188,7 +221,6 @@ __global__ void __launch_bounds__(kMidThreads, 1)
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(acc_full + 8 * i) : "memory");
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;" ::"r"(acc_empty + 8 * i) : "memory");
     }
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(wbar) : "memory");
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(drain) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -202,39 +234,45 @@ __global__ void __launch_bounds__(kMidThreads, 1)
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = tmem_slot;
+  const uint32_t tmem = tmem_slot + pipe * F * kRing;
+  const long long first = (long long)blockIdx.x * kPipes + pipe, step = (long long)gridDim.x * kPipes;
   bool ok = true;
 
-  if (warp == 0 && lane == 0) {  // loads
-    conv_expect(wbar, M::kWeights);
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(wsm),
-        "l"(wimg), "r"(M::kWeights), "r"(wbar)
-        : "memory");
-    long long n = 0;  // planes loaded
-    for (long long i = blockIdx.x; ok && i < wk.items; i += gridDim.x) {
-      const MidItem it = mid_item(d, wk, i);
-      for (int zi = it.z0 - 1; zi <= it.z1; ++zi, ++n) {
-        const int s = (int)(n % kStages);
-        if (n >= kStages && !(ok = conv_wait(empty + 8 * s, (uint32_t)((n / kStages - 1) & 1)))) break;
-        conv_expect(full + 8 * s, M::kStage);
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-          asm volatile(
-              "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-              " [%0], [%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(stages + s * M::kStage + c * M::kCopy),
-              "l"(&map), "r"(0), "r"(it.x0 + c - 1), "r"(it.y0 - 1), "r"(zi), "r"(it.b),
-              "r"(full + 8 * s)
-              : "memory");
+  if (warp < 2 * kPipes && !(warp & 1)) {  // loads
+    if (lane == 0) {
+      if (pipe == 0) {
+        conv_expect(wbar, M::kWeights);
+        asm volatile(
+            "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(wsm),
+            "l"(wimg), "r"(M::kWeights), "r"(wbar)
+            : "memory");
       }
+      long long n = 0;  // planes loaded
+      for (long long i = first; ok && i < wk.items; i += step) {
+        const MidItem it = mid_item(d, wk, i);
+        for (int zi = it.z0 - 1; zi <= it.z1; ++zi, ++n) {
+          const int s = (int)(n % kStages);
+          if (n >= kStages && !(ok = conv_wait(empty + 8 * s, (uint32_t)((n / kStages - 1) & 1)))) break;
+          conv_expect(full + 8 * s, M::kStage);
+#pragma unroll
+          for (int c = 0; c < 3; ++c)
+            asm volatile(
+                "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+                " [%0], [%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(stages + s * M::kStage + c * M::kCopy),
+                "l"(&map), "r"(0), "r"(it.x0 + c - 1), "r"(it.y0 - 1), "r"(zi), "r"(it.b),
+                "r"(full + 8 * s)
+                : "memory");
+        }
+      }
+      // the last copies land before the block can end
+      for (long long k = n > kStages ? n - kStages : 0; k < n; ++k)
+        ok &= conv_wait(full + 8 * (int)(k % kStages), (uint32_t)((k / kStages) & 1));
     }
-    // the last copies land before the block can end
-    for (long long k = n > kStages ? n - kStages : 0; k < n; ++k)
-      ok &= conv_wait(full + 8 * (int)(k % kStages), (uint32_t)((k / kStages) & 1));
-  } else if (warp == 1 && lane == 0) {  // matrix instructions
-    ok = conv_wait(wbar, 0);
+  } else if (warp < 2 * kPipes) {  // matrix instructions
+    const uint32_t e1 = conv_elect();
+    ok = conv_wait_all(wbar, 0);
     long long n = 0, g = 0;  // input planes, output planes so far
-    for (long long i = blockIdx.x; ok && i < wk.items; i += gridDim.x) {
+    for (long long i = first; ok && i < wk.items; i += step) {
       const MidItem it = mid_item(d, wk, i);
       for (int zi = it.z0 - 1; zi <= it.z1; ++zi, ++n) {
         const int s = (int)(n % kStages);
@@ -242,10 +280,10 @@ __global__ void __launch_bounds__(kMidThreads, 1)
         if (hi == zi + 1) {  // a plane begins: its accumulator is drained
           const long long u = g + (hi - it.z0);
           if (u >= kRing &&
-              !(ok = conv_wait(acc_empty + 8 * (int)(u % kRing), (uint32_t)((u / kRing - 1) & 1))))
+              !(ok = conv_wait_all(acc_empty + 8 * (int)(u % kRing), (uint32_t)((u / kRing - 1) & 1))))
             break;
         }
-        if (!(ok = conv_wait(full + 8 * s, (uint32_t)((n / kStages) & 1)))) break;
+        if (!(ok = conv_wait_all(full + 8 * s, (uint32_t)((n / kStages) & 1)))) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const unsigned long long ad = conv_desc<F>(stages + s * M::kStage);
         const unsigned long long bd = conv_desc<F>(wsm + (lo - zi + 1) * F * M::kRow);
@@ -256,40 +294,38 @@ __global__ void __launch_bounds__(kMidThreads, 1)
         // the first step one plane at a time: the plane that begins is overwritten
         for (int j = 0; j < n1 + n2; ++j)
           conv_mma(j < n1 ? d1 + j * F : tmem + (j - n1) * F, ad, bd + j * kB, conv_idesc(F),
-                   lo + j != zi + 1);
+                   lo + j != zi + 1, e1);
         const uint32_t i1 = conv_idesc(n1 * F), i2 = conv_idesc(n2 * F);
         if (n2 == 0) {
 #pragma unroll
           for (int k = 1; k < 9 * (F / 16); ++k)
-            conv_mma(d1, ad + mid_a<F>(k), bd + mid_b<F>(k), i1, true);
+            conv_mma(d1, ad + mid_a<F>(k), bd + mid_b<F>(k), i1, true, e1);
         } else {  // the planes wrap round the ring
 #pragma unroll
           for (int k = 1; k < 9 * (F / 16); ++k) {
-            conv_mma(d1, ad + mid_a<F>(k), bd + mid_b<F>(k), i1, true);
-            conv_mma(tmem, ad + mid_a<F>(k), bd + mid_b<F>(k) + n1 * kB, i2, true);
+            conv_mma(d1, ad + mid_a<F>(k), bd + mid_b<F>(k), i1, true, e1);
+            conv_mma(tmem, ad + mid_a<F>(k), bd + mid_b<F>(k) + n1 * kB, i2, true, e1);
           }
         }
-        conv_commit(empty + 8 * s);
-        if (zi - 1 >= it.z0) conv_commit(acc_full + 8 * (int)((g + (zi - 1 - it.z0)) % kRing));
+        conv_commit(empty + 8 * s, e1);
+        if (zi - 1 >= it.z0) conv_commit(acc_full + 8 * (int)((g + (zi - 1 - it.z0)) % kRing), e1);
       }
       g += it.z1 - it.z0;
     }
-    conv_commit(drain);  // nothing in flight when the tensor memory is given back
-    ok &= conv_wait(drain, 0);
-  } else if (warp >= 2) {  // finished planes
+    conv_commit(drain, e1);  // nothing in flight when the tensor memory is given back
+    ok &= conv_wait_all(drain, 0);
+  } else {  // finished planes
     const int q = warp & 3;  // the quarter of the lanes this warp may read
-    const int turn = (warp - 2) >> 2;
     __nv_bfloat162 bs[F / 2];
 #pragma unroll
     for (int c = 0; c < F / 2; ++c)
       if (!kMask) bs[c] = __nv_bfloat162(bias[2 * c], bias[2 * c + 1]);
     long long g = 0;
-    for (long long i = blockIdx.x; ok && i < wk.items; i += gridDim.x) {
+    for (long long i = first; ok && i < wk.items; i += step) {
       const MidItem it = mid_item(d, wk, i);
       const int x = it.x0 + (lane & 7), y = it.y0 + q * 4 + (lane >> 3);
       const bool in = x < d.X && y < d.Y;
       for (int z = it.z0; z < it.z1; ++z, ++g) {
-        if ((int)(g & 1) != turn) continue;
         const int slot = (int)(g % kRing);
         const long long vox = ((((long long)it.b * d.Z + z) * d.Y + y) * d.X + x) * F;
         uint4 m[F / 8];
@@ -302,17 +338,9 @@ __global__ void __launch_bounds__(kMidThreads, 1)
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         uint32_t r[F];
-        const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16) + slot * F;
 #pragma unroll
         for (int c = 0; c < F; c += 16)
-          asm volatile(
-              "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, "
-              "%11, %12, %13, %14, %15}, [%16];"
-              : "=r"(r[c]), "=r"(r[c + 1]), "=r"(r[c + 2]), "=r"(r[c + 3]), "=r"(r[c + 4]),
-                "=r"(r[c + 5]), "=r"(r[c + 6]), "=r"(r[c + 7]), "=r"(r[c + 8]), "=r"(r[c + 9]),
-                "=r"(r[c + 10]), "=r"(r[c + 11]), "=r"(r[c + 12]), "=r"(r[c + 13]), "=r"(r[c + 14]),
-                "=r"(r[c + 15])
-              : "r"(ta + c));
+          tmem_load16(r + c, tmem + ((uint32_t)(q * 32) << 16) + slot * F + c);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
@@ -340,7 +368,7 @@ __global__ void __launch_bounds__(kMidThreads, 1)
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   if (warp == 1)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(M::kCols));
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_slot), "r"(M::kCols));
 }
 
 // The weights as the three kernels read them: the B operands of the middle one's nine
@@ -763,7 +791,8 @@ __global__ void __launch_bounds__(256) wgrad_edge_kernel(const bf16* __restrict_
 // ignored), B = g with columns (x tap, co) from three copies shifted in x, one set of
 // columns in tensor memory per z tap. The sums stay in tensor memory over all the
 // columns a block marches through; each block leaves its own in `part`.
-// 2 x 128^3, F = 32: 0.323 ms (the library's 1.4), 0.72 PFLOP/s of wanted products.
+// 2 x 128^3, F = 32: 0.288 ms (the library's 1.4), 0.81 PFLOP/s of wanted products;
+// loading through cp.async without the copies of g in global reads took 0.54 ms.
 template <int F>
 struct Wgrad {
   static constexpr int kRow = F * 2;
@@ -849,37 +878,41 @@ __global__ void __launch_bounds__(192, 1)
       ok &= conv_wait(a_full + 8 * (int)(k % W::kAStages), (uint32_t)((k / W::kAStages) & 1));
     for (long long k = nb > W::kBStages ? nb - W::kBStages : 0; k < nb; ++k)
       ok &= conv_wait(b_full + 8 * (int)(k % W::kBStages), (uint32_t)((k / W::kBStages) & 1));
-  } else if (warp == 1 && lane == 0) {  // matrix instructions
+  } else if (warp == 1) {  // matrix instructions
+    const uint32_t e1 = conv_elect();
     const uint32_t idesc = conv_idesc(3 * F) | (1u << 15) | (1u << 16);  // both operands MN-major
     long long na = 0, nb = 0;  // plane z - 1 of h, plane z of g
     for (long long i = blockIdx.x; ok && i < wk.items; i += gridDim.x) {
       const MidItem it = mid_item(d, wk, i);
       for (int z = it.z0; ok && z < it.z1; ++z, ++na, ++nb) {
         for (int k = z == it.z0 ? 0 : 2; ok && k < 3; ++k)
-          ok = conv_wait(a_full + 8 * (int)((na + k) % W::kAStages), (uint32_t)(((na + k) / W::kAStages) & 1));
+          ok = conv_wait_all(a_full + 8 * (int)((na + k) % W::kAStages), (uint32_t)(((na + k) / W::kAStages) & 1));
         const int t = (int)(nb % W::kBStages);
-        if (!ok || !(ok = conv_wait(b_full + 8 * t, (uint32_t)((nb / W::kBStages) & 1)))) break;
+        if (!ok || !(ok = conv_wait_all(b_full + 8 * t, (uint32_t)((nb / W::kBStages) & 1)))) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const unsigned long long bd = wgrad_desc<F>(sb + t * W::kB, W::kCopy);
+        unsigned long long ad[3];
 #pragma unroll
-        for (int kz = 0; kz < 3; ++kz) {
-          const unsigned long long ad =
-              wgrad_desc<F>(sa + (int)((na + kz) % W::kAStages) * W::kA, 8 * W::kRow);
+        for (int kz = 0; kz < 3; ++kz)
+          ad[kz] = wgrad_desc<F>(sa + (int)((na + kz) % W::kAStages) * W::kA, 8 * W::kRow);
+        // 16 voxels, two rows of the column, at a time; the z taps in turn, since an
+        // instruction waits for the last one on its accumulator
 #pragma unroll
-          for (int k = 0; k < 8; ++k)  // 16 voxels: two rows of the column
-            conv_mma(tmem + kz * 3 * F, ad + k * W::kRow, bd + k * W::kRow, idesc, nb > 0 || k > 0);
-        }
-        conv_commit(b_empty + 8 * t);
-        conv_commit(a_empty + 8 * (int)(na % W::kAStages));
+        for (int k = 0; k < 8; ++k)
+#pragma unroll
+          for (int kz = 0; kz < 3; ++kz)
+            conv_mma(tmem + kz * 3 * F, ad[kz] + k * W::kRow, bd + k * W::kRow, idesc, nb > 0 || k > 0, e1);
+        conv_commit(b_empty + 8 * t, e1);
+        conv_commit(a_empty + 8 * (int)(na % W::kAStages), e1);
         if (z == it.z1 - 1) {  // the item's last two planes of h
-          conv_commit(a_empty + 8 * (int)((na + 1) % W::kAStages));
-          conv_commit(a_empty + 8 * (int)((na + 2) % W::kAStages));
+          conv_commit(a_empty + 8 * (int)((na + 1) % W::kAStages), e1);
+          conv_commit(a_empty + 8 * (int)((na + 2) % W::kAStages), e1);
         }
       }
       na += 2;
     }
-    conv_commit(done);
-    ok &= conv_wait(done, 0);
+    conv_commit(done, e1);
+    ok &= conv_wait_all(done, 0);
   }
   __syncwarp();
   // every warp sees the sums complete; readers of tensor memory are warps 2-5
@@ -891,13 +924,7 @@ __global__ void __launch_bounds__(192, 1)
     const int q = warp & 3;
     for (int c = 0; c < W::kCols; c += 16) {
       uint32_t r[16];
-      asm volatile(
-          "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, "
-          "%11, %12, %13, %14, %15}, [%16];"
-          : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-            "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-            "=r"(r[14]), "=r"(r[15])
-          : "r"(tmem + ((uint32_t)(q * 32) << 16) + c));
+      tmem_load16(r, tmem + ((uint32_t)(q * 32) << 16) + c);
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
       if (q * 32 + lane < 3 * F) {
 #pragma unroll
@@ -1051,8 +1078,8 @@ int launch_mid(const bf16* in, unsigned char* ws, const bf16* bias, const bf16* 
   if (const int rc = conv_map<F>(&map, in, d, kCY + 2)) return rc;
   DTV_CUDA_TRY(cudaFuncSetAttribute(conv_mid_kernel<F, kMask>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     Mid<F>::kSmem));
-  const MidWork wk = mid_work(d, sms);
-  conv_mid_kernel<F, kMask><<<(unsigned)std::min<long long>(wk.items, sms), kMidThreads, Mid<F>::kSmem, st>>>(
+  const MidWork wk = mid_work(d, sms * kPipes);
+  conv_mid_kernel<F, kMask><<<(unsigned)std::min<long long>((wk.items + kPipes - 1) / kPipes, sms), kMidThreads, Mid<F>::kSmem, st>>>(
       map, ws, bias, act, out, d, wk, reinterpret_cast<int*>(ws + ConvWs<F>::kStatus));
   note_launch();
   DTV_LAUNCH_CHECK();
