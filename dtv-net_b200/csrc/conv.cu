@@ -38,11 +38,11 @@ __device__ __forceinline__ unsigned conv_act(float lo, float hi, __nv_bfloat162 
       __hmax2_nan(__hadd2(__floats2bfloat162_rn(lo, hi), bias), __nv_bfloat162(0.f, 0.f));
   return *reinterpret_cast<const unsigned*>(&v);
 }
-// bf16(sum) of two channels where the activations of the forward pass are positive
+// bf16(sum) of two channels where the activations of the forward pass are positive (or NaN)
 __device__ __forceinline__ unsigned conv_masked(float lo, float hi, unsigned act) {
   const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   const __nv_bfloat162 h = *reinterpret_cast<const __nv_bfloat162*>(&act);
-  return *reinterpret_cast<const unsigned*>(&v) & __hgt2_mask(h, __nv_bfloat162(0.f, 0.f));
+  return *reinterpret_cast<const unsigned*>(&v) & ~__hle2_mask(h, __nv_bfloat162(0.f, 0.f));
 }
 // D[16 x 8] += A[16 x 16] B[16 x 8], BF16 in, FP32 out
 __device__ __forceinline__ void warp_mma(float (&d)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3,
@@ -501,7 +501,9 @@ __global__ void __launch_bounds__(256) conv_in_kernel(const bf16* __restrict__ x
                 ? xs[((long long)gz * d.Y + gy) * d.X + gx]
                 : (unsigned short)0;
   }
-  // this lane's taps (2 per word; the padding's weights are zero)
+  // this lane's taps, 2 per word; the last word's beyond 26 are padding, zero on both
+  // sides (an infinite voxel times a zero weight would be NaN)
+  const unsigned keep = q == 0 ? 0xffffffffu : q == 1 ? 0xffffu : 0u;
   int off[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
@@ -531,6 +533,7 @@ __global__ void __launch_bounds__(256) conv_in_kernel(const bf16* __restrict__ x
         const unsigned short* r = s + (j & 1) * 8;
         const int u = ks * 4 + (j >> 1) * 2;
         a[ks][j] = (unsigned)r[off[u]] | (unsigned)r[off[u + 1]] << 16;
+        if (u == 6) a[ks][j] &= keep;
       }
     Quarter<F> r0, r1;
 #pragma unroll
@@ -728,6 +731,12 @@ __global__ void __launch_bounds__(256) wgrad_edge_kernel(const bf16* __restrict_
     }
     __syncthreads();
     const int gy = y0 + warp, nz = gy < d.Y ? min(kInZ, d.Z - z0) : 0;
+    unsigned have[2];  // this lane's voxels inside the volume
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int x = x0 + 2 * q + 8 * j;
+      have[j] = (x < d.X ? 0xffffu : 0u) | (x + 1 < d.X ? 0xffff0000u : 0u);
+    }
     const bf16* tp = T + ((((long long)b * d.Z + z0) * d.Y + gy) * d.X + x0) * F + F / 8 * g;
     for (int k = 0; k < nz; ++k, tp += (long long)d.Y * d.X * F) {
       unsigned v[4][F / 16];  // voxels 2q, 2q + 1, 2q + 8, 2q + 9
@@ -753,7 +762,7 @@ __global__ void __launch_bounds__(256) wgrad_edge_kernel(const bf16* __restrict_
 #pragma unroll
         for (int j = 0; j < 4; ++j) {  // (tap, tap + 8) x (voxels 2q.., 2q + 8..)
           const unsigned short* r = s + off[2 * i + (j & 1)] + (j >> 1) * 8;
-          a[i][j] = (unsigned)r[0] | (unsigned)r[1] << 16;
+          a[i][j] = ((unsigned)r[0] | (unsigned)r[1] << 16) & have[j >> 1];
         }
       if (tap3 == 27) a[1][1] = a[1][3] = 0x3f803f80u;  // ones
 #pragma unroll

@@ -251,8 +251,9 @@ class ConvBlock(nn.Module):
             nn.Conv3d(features, 1, 3, padding=1))
 
     def forward(self, x):
-        if conv.supported(self.body, x):
-            return conv.conv_block(self.body, x)
+        if not torch.jit.is_scripting():  # (a script keeps the modules, and so does a compiler)
+            if not torch.compiler.is_compiling() and conv.supported(self.body, x):
+                return conv.conv_block(self.body, x)
         return self.body(x)
 
 

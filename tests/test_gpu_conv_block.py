@@ -91,6 +91,42 @@ def test_some_gradients(cuda, wanted):
         assert torch.equal(g, full[k]), k
 
 
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan")])
+@pytest.mark.parametrize("at", [(0, 0, 0), (4, 9, 12), (8, 17, 19)])
+def test_not_finite(cuda, value, at):
+    """One infinite or NaN voxel reaches the outputs that the module's own layers let
+    it reach, and one such output gradient the same input gradients."""
+    torch.manual_seed(5)
+    block = ConvBlock(32).to(cuda)
+    x = torch.randn(1, 1, 9, 18, 20, device=cuda)
+    gy = torch.randn(1, 1, 9, 18, 20, device=cuda).to(bf)
+    bad_x, bad_gy = x.clone(), gy.clone()
+    bad_x[0, 0][at] = value
+    bad_gy[0, 0][at] = value
+    for xi, g in ((bad_x, None), (x, bad_gy)):
+        got = []
+        for f in (block, block.body):
+            xi = xi.detach().requires_grad_()
+            with torch.autocast("cuda", dtype=bf):
+                y = f(xi)
+            if g is not None:
+                y, = torch.autograd.grad(y, xi, g)
+            got.append(y.detach().float())
+        assert torch.equal(torch.isnan(got[0]), torch.isnan(got[1]))
+        assert torch.equal(torch.isinf(got[0]), torch.isinf(got[1]))
+
+
+@pytest.mark.parametrize("mode", [torch.inference_mode, torch.no_grad])
+def test_without_gradients(cuda, mode):
+    block = ConvBlock(16).to(cuda)
+    x = torch.randn(2, 1, 5, 6, 7, device=cuda)
+    with torch.autocast("cuda", dtype=bf):
+        y = block(x)
+        with mode():
+            z = block(x)
+    assert torch.equal(y, z)
+
+
 def test_what_stays_general(cuda):
     block = ConvBlock(16).to(cuda)
     x = torch.randn(1, 1, 6, 5, 7, device=cuda)
