@@ -687,10 +687,11 @@ __global__ void __launch_bounds__(256) conv_out_kernel(const bf16* __restrict__ 
 // one-channel and an F-channel tensor; tap 27 stands for the sum of T alone. 32 rows
 // of taps, F columns, voxels along K: eight small matrix instructions per 16 voxels,
 // so that the kernel takes little more than the time of reading T (2 x 128^3, F = 32:
-// 0.106 ms; the library's 0.47-0.70). The columns are permuted so that a lane loads
+// 0.090 ms; the library's 0.47-0.70; 0.134 with the two blocks per SM that its 92
+// registers allowed unbounded). The columns are permuted so that a lane loads
 // F / 8 adjacent channels. Each block leaves its sums in `part`.
 template <int F>
-__global__ void __launch_bounds__(256) wgrad_edge_kernel(const bf16* __restrict__ s_in,
+__global__ void __launch_bounds__(256, 3) wgrad_edge_kernel(const bf16* __restrict__ s_in,
                                                          const bf16* __restrict__ T, ConvDims d,
                                                          long long tiles, float* __restrict__ part) {
   constexpr int kPX = kInX + 2, kNT = F / 8, kCells = (kInZ + 2) * (kInY + 2) * kPX;
@@ -1123,9 +1124,9 @@ int conv_block(const bf16* x, const ConvW* w, const bf16* const* bias, bf16* h1,
   return rc;
 }
 
-// blocks of the one-channel weight gradients: five fit an SM
+// blocks of the one-channel weight gradients: three fit an SM
 int edge_blocks(const ConvDims& d, int sms) {
-  return (int)std::min<long long>(conv_tiles(d, kInX, kInY, kInZ), 5LL * sms);
+  return (int)std::min<long long>(conv_tiles(d, kInX, kInY, kInZ), 3LL * sms);
 }
 
 // bytes of the blocks' sums, shared by the kernels that leave some
