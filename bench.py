@@ -800,9 +800,10 @@ def run_train(args):
     launches = L.dtv_launch_count() - n0
     plan = proj.plan(dev, 2)
     fp_units = 2 * plan.fp_samples()  # per forward projection of the batch
-    # the exact adjoint alone: each sample adds two 16-byte vector reductions
-    # into L2-resident cell records, so its bound is the L2's rate of those
-    # reductions, measured here with a kernel that does nothing else
+    # the exact adjoint alone: each sample adds to two 16-byte cell records in L2.
+    # Against the L2's rate of 16-byte reductions, measured here with a kernel that
+    # does nothing else; the adjoint merges the additions of a warp's neighbouring
+    # rays first, so it can exceed one reduction per addition
     adj_in = torch.rand(plan.sino_shape(2), device=dev)
     adj_out = torch.empty(plan.vol_shape(2), device=dev)
     plan.adjoint(adj_in, out=adj_out)
@@ -831,9 +832,9 @@ def run_train(args):
             "scattered_peak": v4_scatter,
             "adjoint_ms": t_adj * 1e3,
             "reductions_per_launch": 2 * fp_units,
-            "note": ("two reductions per forward-projector sample of the batch (samples whose "
-                     "cell lies wholly in the zero border add none, so achieved is an upper "
-                     "bound)")},
+            "note": ("two additions per forward-projector sample of the batch, merged within a "
+                     "warp before they reduce: a fraction above 1 means fewer reductions than "
+                     "additions (samples whose cell lies wholly in the zero border add none)")},
         "gpu_launches": launches,
         "clocks": clk.summary(),
     }

@@ -142,15 +142,14 @@ class Plan:
     bilinear fetch per sample, z interpolated in FP32) or "tma" (the same
     z-pairs streamed by the Tensor Memory Accelerator into shared memory per
     ray tile and interpolated there with FP32 weights; a tunable share of the
-    tiles still uses the texture unit) or "exact" (the same FP16 z-pairs in a
-    zero-bordered linear copy read through L1, FP32 x/y/z weights, and the
-    software FP32-weight backprojector: no 8-bit texture weights anywhere,
+    tiles still uses the texture unit) or "exact" ("soft" on the
+    FP16-rounded volume: no 8-bit texture weights anywhere,
     whose error 100-iteration reconstructions amplify past 1e-3 of FP64).
     The backprojector samples the sinogram through a texture for "tex",
     "pairs" and "tma".
     ``stage_f16`` stages projected volumes as FP16 ("soft"/"tex").
     ``adjoint`` keeps a per-ray table (32 bytes per ray and view) and cell
-    records (16 bytes per voxel) that speed up :meth:`adjoint`.
+    records (16 bytes per voxel of the grid padded by two) that speed up :meth:`adjoint`.
 
     A plan stages its input in buffers of its own, so its calls are ordered
     on the stream they are made on; calls of one plan from two streams at once

@@ -72,7 +72,7 @@ extern "C" {
  * as DTV_PLAN_TEX. Needs nz + 3 <= the device's layered-texture layer limit. */
 #define DTV_PLAN_TEX_PAIRS 0x4
 /* Keep a table of every ray's sample range (32 bytes per ray and view) and
- * (nx+1)(ny+1)nz 16-byte cell records per batch item for
+ * (nx+4)(ny+4)(nz+4) 16-byte cell records per batch item for
  * dtv_backward_adjoint, which otherwise rebuilds each ray for every 16^3
  * brick it crosses (see DTV_TUNE_ADJOINT). */
 #define DTV_PLAN_ADJOINT 0x8
@@ -84,12 +84,10 @@ extern "C" {
  * trilinear of the FP16 volume). DTV_TUNE_FP_TEX_SHARE sends a share of the
  * tiles through the texture unit instead, so both pipes work at once. */
 #define DTV_PLAN_TMA 0x10
-/* Exact interpolation weights in both directions. Forward projector: the FP16
- * z pairs of DTV_PLAN_TEX_PAIRS staged in a linear array with a two-texel
- * zero border, read through L1 (four 4-byte loads per sample) and
- * interpolated with FP32 x/y/z weights (exact trilinear of the FP16-rounded
- * volume). Backprojector: software bilinear with FP32 weights, as
- * DTV_PLAN_SOFT. The texture filter's 8-bit weights, whose error iterative
+/* Exact interpolation weights in both directions, on the FP16-rounded volume:
+ * the forward projector of DTV_PLAN_SOFT (16-byte records of the x/y cells, z
+ * fastest, two loads per sample, FP32 x/y/z weights) with the volume rounded
+ * to FP16 as it is staged, and its backprojector. The texture filter's 8-bit weights, whose error iterative
  * reconstructions amplify, are not used. Exclusive with DTV_PLAN_TEX,
  * DTV_PLAN_TEX_PAIRS and DTV_PLAN_TMA. */
 #define DTV_PLAN_PAIRS_EXACT 0x20
@@ -209,7 +207,8 @@ DTV_API int dtv_plan_destroy(dtv_plan* plan);
  *   4 consecutive lanes: 0 = 16 x 2 (quads 4 x 1), 1 = 8 x 4 (4 x 1),
  *   2 = 4 x 8 (4 x 1), 3 = 8 x 4 (2 x 2), 4 = 4 x 8 (2 x 2, default). The
  *   texture unit serves a quad in fewer wavefronts when its four footprints
- *   are close. No counterpart in the reference. */
+ *   are close. Plans whose blocks split their views (small volumes) use 4 x 8
+ *   throughout. No counterpart in the reference. */
 #define DTV_TUNE_BP_WARP 5
 DTV_API int dtv_plan_set_tuning(dtv_plan* plan, int32_t key, int32_t value);
 DTV_API int dtv_plan_get_tuning(const dtv_plan* plan, int32_t key, int32_t* value);
