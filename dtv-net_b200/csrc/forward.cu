@@ -55,10 +55,10 @@ struct SoftSampler {
 //
 // Why this layout: a 16-byte warp load costs one L1 clock per 128-byte line it
 // touches (four at least), and the rays of a warp that share a detector column
-// pass through one (x, y) column at neighbouring z. With the lanes of a quarter
-// warp along v they read consecutive records: 5.3 lines per load, against 11.2
-// with x fastest and lanes along u. 256^3 x 64 views of 384^2: 6.33 -> 3.48 ms,
-// 2.4 G samples, 80 % of the L1 data clocks busy (32 bytes per sample are 8
+// pass through one (x, y) column at neighbouring z. With the lanes of a half
+// warp along v they read consecutive records: 5.0 lines per load, against 11.2
+// with x fastest and lanes along u. 256^3 x 64 views of 384^2: 6.33 -> 3.28 ms,
+// 2.4 G samples, 84 % of the L1 data clocks busy (32 bytes per sample are 8
 // clocks per 32 samples at best).
 //
 // Floors come from rounding-down adds (kIntMagic), whose bits then address the
@@ -208,15 +208,15 @@ __device__ __forceinline__ void tile_pixel(const RayParams& rp, int& u, int& v, 
 }
 
 // The pixel of this thread with a warp's lanes along v first (record samplers:
-// consecutive lanes then read consecutive records of one column).
-__device__ __forceinline__ void tile_pixel_v(const RayParams& rp, int& u, int& v, int& n) {
+// consecutive lanes then read consecutive records of one column), 2^lwu columns.
+__device__ __forceinline__ void tile_pixel_v(const RayParams& rp, int lwu, int& u, int& v, int& n) {
   const int t = threadIdx.x, w = t >> 5, l = t & 31;
   const int tiles_u = (rp.nu + (1 << rp.ltu) - 1) >> rp.ltu;
   int tile;
   block_tile_view(rp, tile, n);
   const int tu = tile % tiles_u, tv = tile / tiles_u;
-  const int lwpr = rp.ltu - rp.lwu, lwv = 5 - rp.lwu;
-  u = (tu << rp.ltu) + ((w & ((1 << lwpr) - 1)) << rp.lwu) + (l >> lwv);
+  const int lwpr = rp.ltu - lwu, lwv = 5 - lwu;
+  u = (tu << rp.ltu) + ((w & ((1 << lwpr) - 1)) << lwu) + (l >> lwv);
   v = (tv << rp.ltv) + ((w >> lwpr) << lwv) + (l & ((1 << lwv) - 1));
 }
 
@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(kFPThreads) fp_soft_kernel(RayParams rp, const
 }
 
 // Four blocks per SM: with the bound the compiler uses the 64 registers they
-// leave it (56 without: 3.71 -> 3.48 ms at 256^3 x 64 views); five or six blocks
+// leave it (56 without: 3.71 -> 3.48 ms at 256^3 x 64 views, in warps of 4 x 8); five or six blocks
 // spill (3.67, 4.29 ms).
 template <bool kFar>
 __global__ void __launch_bounds__(kFPThreads, 4) fp_rec_kernel(RayParams rp,
@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(kFPThreads, 4) fp_rec_kernel(RayParams rp,
                                                             const float4* __restrict__ recs,
                                                             int64_t pad_elems, FPOut o) {
   int u, v, n;
-  tile_pixel_v(rp, u, v, n);
+  tile_pixel_v(rp, rp.lwu, u, v, n);
   const int b = blockIdx.z;
   float res = 0.f;
   if (u < rp.nu && v < rp.nv) {
@@ -299,8 +299,8 @@ __global__ void __launch_bounds__(kFPThreads) fp_pair_kernel(RayParams rp, const
 //   abs_sum += |E f - g|.
 // Each sum has the bits of fp_pair_kernel / fp_rec_kernel for the ray. The
 // texture unit wants a quad's lanes on one layer (along u), the records want
-// lanes along v: a thread sums one ray of its warp's tile through each, in its
-// own order, and a shuffle brings the two sums of a ray together.
+// lanes along v: a thread sums one ray of its block's tile through each, in each
+// one's order, and the record sums change hands in shared memory.
 struct RefreshOut {
   const float* g;
   float* w;
@@ -314,10 +314,12 @@ __global__ void __launch_bounds__(kFPThreads, 4) fp_refresh_kernel(RayParams rp,
                                                                 const FPView* __restrict__ views,
                                                                 const cudaTextureObject_t* texs,
                                                                 const float4* __restrict__ recs,
-                                                                int64_t pad_elems, RefreshOut o) {
+                                                                int64_t pad_elems, int rec_lwu,
+                                                                RefreshOut o) {
+  __shared__ float sums[288];  // of the tile's rays, rows padded by one
   int u, v, n, ue, ve;
   tile_pixel(rp, u, v, n);
-  tile_pixel_v(rp, ue, ve, n);
+  tile_pixel_v(rp, rec_lwu, ue, ve, n);
   const int b = blockIdx.z;
   float sf = 0.f, se = 0.f;
   if (u < rp.nu && v < rp.nv) {
@@ -330,9 +332,10 @@ __global__ void __launch_bounds__(kFPThreads, 4) fp_refresh_kernel(RayParams rp,
     const RecSampler<kFar> exact(rp, recs + b * pad_elems);
     if (rs.count > 0) se = exact.sum(rs);
   }
-  // lane (u, v) of the texture order takes its record sum from lane (v, u)
-  const int l = threadIdx.x & 31, wu = 1 << rp.lwu;
-  se = __shfl_sync(0xffffffffu, se, ((l & (wu - 1)) << (5 - rp.lwu)) + (l >> rp.lwu));
+  const int mu = (1 << rp.ltu) - 1, mv = (1 << rp.ltv) - 1;
+  sums[(ve & mv) * (mu + 2) + (ue & mu)] = se;
+  __syncthreads();
+  se = sums[(v & mv) * (mu + 2) + (u & mu)];
   float res = 0.f;
   if (u < rp.nu && v < rp.nv) {
     const float a = sf * rp.scale, e = se * rp.scale;
@@ -565,17 +568,19 @@ static bool rec_far(const GeomParams& g) {
   return (int64_t)(g.nx + 2 * kPad) * (g.nz + 2 * kPad) * 16 >= (1LL << 32);
 }
 
-// `records`: the launch samples records, whose warps want 4 x 8 pixels: tile 0,
-// the default, then stands for shape 3 and the other way round. 256^3 x 64
-// views of 384^2: 4 x 8 3.67 ms, 8 x 4 4.07, 16 x 2 5.90, 32 x 1 9.34; the
-// correction pass 4.94, 5.53, 7.27, 10.5.
+// `records`: the launch samples records, whose warps want two columns of 16 pixels
+// (tile 0, the default, then stands for those). A half warp's rays pass one (x, y)
+// column and read its records once; four columns of 8 touch more 128-byte lines, and
+// one of 32 needs blocks of 32 rows, which cross more of the volume at a time. 256^3 x
+// 64 views of 384^2: 2 x 16 3.28 ms, 4 x 8 3.49, 1 x 32 3.45, 8 x 4 4.07, 16 x 2 5.90;
+// 151x163x97 x 45 views of 231x149: 0.366, 0.387, 0.357 (1 x 32).
 static RayParams plan_ray_params(const Plan* p, bool records) {
+  static const int kRecTile[3] = {4, 4, 1};
   RayParams rp = make_ray_params(p->gp);
-  const int t = records && (p->fp_ray_tile == 0 || p->fp_ray_tile == 3) ? 3 - p->fp_ray_tile
-                                                                        : p->fp_ray_tile;
-  rp.ltu = kRayTiles[t][0];
-  rp.ltv = kRayTiles[t][1];
-  rp.lwu = kRayTiles[t][2];
+  const int* t = records && p->fp_ray_tile == 0 ? kRecTile : kRayTiles[p->fp_ray_tile];
+  rp.ltu = t[0];
+  rp.ltv = t[1];
+  rp.lwu = t[2];
   rp.band = p->fp_band;
   return rp;
 }
@@ -622,7 +627,9 @@ int forward_refresh_impl(Plan* fast, Plan* exact, const void* vol, int vol_dtype
   if (rc) return rc;
   rc = stage_volume(exact, vol, vol_dtype, batch, st);
   if (rc) return rc;
-  RayParams rp = plan_ray_params(fast, true);
+  RayParams rp = plan_ray_params(fast, false);
+  // the record order's columns per warp: two where the tile has 16 rows
+  const int rec_lwu = std::max(1, 5 - rp.ltv);
   // band-major plans march bands of one tile row here: with the exact
   // sampler's records beside the z-pairs, the narrower slab keeps more of both
   // in L2 (5.66 ms against 5.74 ms with the plan's 4 rows at 256^3 x 64 views)
@@ -632,10 +639,10 @@ int forward_refresh_impl(Plan* fast, Plan* exact, const void* vol, int vol_dtype
   const RefreshOut o{g, w, g_eff, sigma, abs_sum};
   if (rec_far(gp))
     fp_refresh_kernel<true><<<grid, kFPThreads, 0, st>>>(rp, fast->d_fpv, fast->pair_tex_dev,
-                                                         exact->d_vol_rec, exact->pad_elems, o);
+                                                         exact->d_vol_rec, exact->pad_elems, rec_lwu, o);
   else
     fp_refresh_kernel<false><<<grid, kFPThreads, 0, st>>>(rp, fast->d_fpv, fast->pair_tex_dev,
-                                                          exact->d_vol_rec, exact->pad_elems, o);
+                                                          exact->d_vol_rec, exact->pad_elems, rec_lwu, o);
   note_launch();
   DTV_LAUNCH_CHECK();
   return DTV_OK;
@@ -912,7 +919,7 @@ __global__ void __launch_bounds__(256) adjoint_cells_kernel(RayParams rp,
   constexpr unsigned int kAll = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   int u, v, n;
-  tile_pixel_v(rp, u, v, n);
+  tile_pixel_v(rp, rp.lwu, u, v, n);
   // z grows with the lane: a detector whose rows run down takes them reversed
   const int wv = 32 >> rp.lwu;
   if (views[n].v[2] < 0.0) v += wv - 1 - 2 * (lane & (wv - 1));
