@@ -426,8 +426,11 @@ static int grid_for(int64_t n, int threads = 256) {
 // reach the volume only, x and y in [-1, n-1], z in [0, nz-1]; the others keep
 // the plan's initial zeros. A block transposes a tile of 32 x 4 x 32 records
 // through shared memory: x runs along the lanes when it reads the volume, z
-// when it writes the records, so the pass is bound by its 16-byte writes
-// (256^3: 95 us). kRound: the exact plans' FP16-rounded volume.
+// when it writes the records. All loads of a thread are in flight together, and
+// a column's values serve the records on both sides of it, so that the pass is
+// bound by its 16-byte writes: 256^3 62 us (load by load and four shared loads per
+// record: 93), 128^3 8.9 (14.6), 24x20x12 2.3 (6.1). kRound: the exact plans'
+// FP16-rounded volume.
 constexpr int kRecX = 32, kRecY = 4, kRecZ = 32;
 template <class Tin, bool kRound>
 __global__ void __launch_bounds__(256) stage_rec_kernel(const Tin* __restrict__ in,
@@ -439,33 +442,51 @@ __global__ void __launch_bounds__(256) stage_rec_kernel(const Tin* __restrict__ 
             z0 = (int)(blockIdx.z % ztiles) * kRecZ;
   const Tin* vol = in + (int64_t)b * nx * ny * nz;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  // rows (y, z) of the tile, a warp each: 33 values from x0
-  for (int r = w; r < (kRecY + 1) * kRecZ; r += 8) {
-    const int yy = r / kRecZ, zz = r % kRecZ;
-    const int y = y0 + yy, z = z0 + zz;
-    const bool row = y >= 0 && y < ny && z < nz;
-    const Tin* p = vol + ((int64_t)z * ny + y) * nx;
-    auto at = [&](int x) {
-      float f = row && x >= 0 && x < nx ? load_as_float(p, x) : 0.f;
+  // rows (y, z) of the tile, 33 values from x0: a warp takes four of each y, and its
+  // first four lanes their last values; all loads before the first store
+  const int64_t zrow = (int64_t)nx * ny;
+  float v[kRecY + 1][4], e[kRecY + 1];
+#pragma unroll
+  for (int yy = 0; yy <= kRecY; ++yy) {
+    const int y = y0 + yy;
+    const bool yin = y >= 0 && y < ny;
+    auto at = [&](int x, int z) {
+      float f = yin && z < nz && x >= 0 && x < nx ? load_as_float(vol + z * zrow + (int64_t)y * nx, x) : 0.f;
       if constexpr (kRound) f = __half2float(__float2half_rn(f));
       return f;
     };
-    s[yy][lane][zz] = at(x0 + lane);
-    if (lane == 0) s[yy][kRecX][zz] = at(x0 + kRecX);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[yy][j] = at(x0 + lane, z0 + w + 8 * j);
+    e[yy] = lane < 4 ? at(x0 + kRecX, z0 + w + 8 * lane) : 0.f;
+  }
+#pragma unroll
+  for (int yy = 0; yy <= kRecY; ++yy) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) s[yy][lane][w + 8 * j] = v[yy][j];
+    if (lane < 4) s[yy][kRecX][w + 8 * lane] = e[yy];
   }
   __syncthreads();
   const int z = z0 + lane;
   if (z >= nz) return;
-  const int64_t pz = nz + 2 * kPad, px = nx + 2 * kPad;
-  float4* out = rec + b * pad_elems + z + kPad;
-  for (int c = w; c < kRecX * kRecY; c += 8) {
-    const int xx = c % kRecX, yy = c / kRecX;
-    const int x = x0 + xx, y = y0 + yy;
-    if (x >= nx || y >= ny) continue;
-    const float f00 = s[yy][xx][lane], f10 = s[yy][xx + 1][lane];
-    const float f01 = s[yy + 1][xx][lane], f11 = s[yy + 1][xx + 1][lane];
-    const float B = f10 - f00;
-    out[((int64_t)(y + kPad) * px + x + kPad) * pz] = make_float4(f00, f01 - f00, B, (f11 - f01) - B);
+  const int64_t pz = nz + 2 * kPad, py = pz * (nx + 2 * kPad);
+  // four columns of x per warp, from one to the next
+  float f0[kRecY + 1], f1[kRecY + 1];
+#pragma unroll
+  for (int yy = 0; yy <= kRecY; ++yy) f0[yy] = s[yy][w * 4][lane];
+  float4* out = rec + b * pad_elems + (y0 + kPad) * py + (x0 + w * 4 + kPad) * pz + z + kPad;
+#pragma unroll
+  for (int k = 0; k < 4; ++k, out += pz) {
+    if (x0 + w * 4 + k >= nx) return;
+#pragma unroll
+    for (int yy = 0; yy <= kRecY; ++yy) f1[yy] = s[yy][w * 4 + k + 1][lane];
+#pragma unroll
+    for (int yy = 0; yy < kRecY; ++yy) {
+      const float B = f1[yy] - f0[yy];
+      if (y0 + yy < ny)
+        out[yy * py] = make_float4(f0[yy], f0[yy + 1] - f0[yy], B, (f1[yy + 1] - f0[yy + 1]) - B);
+    }
+#pragma unroll
+    for (int yy = 0; yy <= kRecY; ++yy) f0[yy] = f1[yy];
   }
 }
 
