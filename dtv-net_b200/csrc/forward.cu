@@ -927,11 +927,14 @@ __global__ void __launch_bounds__(kAdjThreads) adjoint_brick_kernel(
 // records: 1.29 and 9.5 ms, bound by instruction issue (117 per 32 samples, 91 %).
 //
 // A thread takes NB batch items through the same samples: the positions, records
-// and runs are theirs alike (2 x 128^3: 1.32 -> 1.18 ms).
+// and runs are theirs alike (2 x 128^3: 1.32 -> 1.17 ms).
+//
+// Five blocks per SM: the bound gives the compiler a few registers more than it took
+// (47 against 43; 256^3 9.45 -> 8.98 ms, 128^3 0.697 -> 0.680); six spill (9.48).
 //
 // kSlab: this launch takes the samples whose base y-cell is in [yb0, yb1).
 template <bool kSlab, int NB>
-__global__ void __launch_bounds__(256) adjoint_cells_kernel(RayParams rp,
+__global__ void __launch_bounds__(256, 5) adjoint_cells_kernel(RayParams rp,
                                                             const FPView* __restrict__ views,
                                                             const float4* __restrict__ rays,
                                                             const float* __restrict__ sino,
