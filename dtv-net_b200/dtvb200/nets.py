@@ -261,7 +261,8 @@ class UnrolledPDHG(nn.Module):
     """x_{s+1} = x_s - lamb_s * A^T (A x_s - p) - tau_s * R_s(x_s), s < stages
     (LEARN.py:15-22 with the matched adjoint A^T). ``share_weights`` reuses one
     block for every stage, as the reference's ``nn.ModuleList([m] * n)`` does
-    (LEARN.py:11, FISTAnet.py:12-13). The blocks run channels-last 3-D, the
+    (LEARN.py:11, FISTAnet.py:12-13). The blocks run on the library's BF16
+    kernels where those apply (ConvBlock), and otherwise channels-last 3-D, the
     layout cuDNN's tensor-core convolutions take without transposes."""
 
     def __init__(self, projector: Projector, stages: int = 10, features: int = 32,
