@@ -19,8 +19,8 @@
 // its outputs: per tap it loads one new pair on each side and the tap, for kOut
 // packed adds and FMAs. Taps run from the farthest in, so that the small terms
 // add up first. (One output per thread needed 2.5 shared loads per tap, which
-// bounded it: 6144 rows of 1680 columns, 1.21 ms; now 0.37 ms, bound by
-// the FP32 pipe at 60 % of its rate. 24576 rows of 384: 0.26 -> 0.14 ms.) The weighted sequences sit in shared memory between their
+// bounded it: 6144 rows of 1680 columns, 1.21 ms; now 0.36 ms, bound by
+// the FP32 pipe at 60 % of its rate. 24576 rows of 384: 0.26 -> 0.16 ms.) The weighted sequences sit in shared memory between their
 // zero paddings, one pair of skew per kOut, so that lanes kOut apart read
 // different banks. The taps are built once per block in FP64 and rounded to
 // FP32 as the reference's float32 kernel array holds them. The transpose (for
@@ -28,6 +28,7 @@
 // after.
 #include <algorithm>
 #include <atomic>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -73,7 +74,9 @@ static size_t filt_smem(const FiltShape& f) {
   return sizeof(float) * ((size_t)f.taps + 2 * (size_t)f.seq * f.rows);
 }
 
-__global__ void __launch_bounds__(kFiltThreads) fbp_filter_kernel(const float* __restrict__ in,
+// At most 72 registers: rows of 1680 columns then have four blocks of 224 threads per
+// SM (unbounded the compiler takes 80; 6144 x 1680: 411 us, with the bound 362).
+__global__ void __maxnreg__(72) fbp_filter_kernel(const float* __restrict__ in,
                                                                   float* __restrict__ out, int64_t rows,
                                                                   int rows_per_view, int width,
                                                                   FiltShape f, float sdd, float mid_i,
@@ -123,19 +126,26 @@ __global__ void __launch_bounds__(kFiltThreads) fbp_filter_kernel(const float* _
       rw[(e + kOut - 1) % kOut] = right[filt_off(kOut - 1 + e)];
       lw[(e + 1) % kOut] = left[filt_off(e - kOut)];
     }
-    for (int j = f.taps - kOut; j >= 0; j -= kOut) {
+    // kOut taps from j; those beyond the last of the width (kLast) meet columns whose
+    // infinities or NaN do not belong to the sum
+    auto group = [&](int j, auto last) {
+      constexpr bool kLast = decltype(last)::value;
 #pragma unroll
       for (int q = kOut - 1; q >= 0; --q) {
         const f32x2_t t = splat2(taps[j + q]);
+        if (!kLast || j + q < used) {
 #pragma unroll
-        for (int e = 0; e < kOut; ++e)
-          acc[e] = fma2(t, add2(rw[(e + q) % kOut], lw[(e - q + kOut) % kOut]), acc[e]);
+          for (int e = 0; e < kOut; ++e)
+            acc[e] = fma2(t, add2(rw[(e + q) % kOut], lw[(e - q + kOut) % kOut]), acc[e]);
+        }
         rw[(q + kOut - 1) % kOut] = right[filt_off(q - 1)];
         lw[(kOut - q) % kOut] = left[filt_off(kOut - 1 - q)];
       }
       right -= kOut + 1;
       left += kOut + 1;
-    }
+    };
+    group(f.taps - kOut, std::true_type{});
+    for (int j = f.taps - 2 * kOut; j >= 0; j -= kOut) group(j, std::false_type{});
     const int64_t r = r0 + rr;
     const float row = adjoint ? row_term(r) : 0.f;
 #pragma unroll
