@@ -109,11 +109,14 @@ __device__ __forceinline__ f32x2_t fma2(f32x2_t a, f32x2_t b, f32x2_t c) {
 constexpr float kIntMagic = 12582912.f;
 constexpr unsigned int kIntMagicBits = 0x4B400000u;
 
-// 1 / x by one Newton step r + r (1 - x r) on the approximate reciprocal.
+// 1 / x by one Newton step r + r (1 - x r) on the approximate reciprocal. kAny: x may
+// be zero or infinite, where 1 - x r is no remainder and r, infinite or zero, stands.
+template <bool kAny>
 __device__ __forceinline__ float rcp_newton(float x) {
   float r;
   asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return fmaf(r, fmaf(-x, r, 1.f), r);
+  const float e = fmaf(-x, r, 1.f);
+  return kAny && !(fabsf(e) < 1.f) ? r : fmaf(r, e, r);
 }
 
 inline int dtype_size(int dt) { return dt == DTV_F32 ? 4 : 2; }
