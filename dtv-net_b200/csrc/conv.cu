@@ -6,7 +6,7 @@
 // roundings that autocast makes around a library convolution.
 // Measured at 2 x 128^3, F = 32: 0.42 ms (0.06 + 0.22 + 0.12 and the weights), where
 // three library convolutions with their layout conversions, bias additions and ReLUs
-// took 4.1 ms; F = 16: 0.28 ms. Backward, all gradients: 1.05 ms, the library's 8.4.
+// took 4.1 ms; F = 16: 0.28 ms. Backward, all gradients: 1.06 ms, the library's 8.4.
 // Gradients are rounded to BF16 where autocast's are: the data gradients after each
 // convolution, the weight and bias gradients once summed. Sums are FP32 in an order
 // fixed by the sizes and the number of SMs.
@@ -381,6 +381,7 @@ struct ConvWs {
   static constexpr int kInWords = F / 2;           // per lane
   static constexpr int kOut = kIn + 32 * kInWords * 4;
   static constexpr int kOutWords = F / 2;
+  // 16 bytes: a wait ran out; the last, the middle one's weight gradient is not finite
   static constexpr int kStatus = kOut + 32 * kOutWords * 4;
 };
 
@@ -392,7 +393,7 @@ template <int F>
 __global__ void conv_weights_kernel(ConvW w1, ConvW w2, ConvW w3, unsigned char* ws) {
   typedef ConvWs<F> W;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i == 0) *reinterpret_cast<int*>(ws + W::kStatus) = 0;
+  if (i == 0) *reinterpret_cast<int4*>(ws + W::kStatus) = make_int4(0, 0, 0, 0);
   if (i < 27 * F * F) {
     const int ci = i % F, n = (i / F) % (3 * F), t = i / (3 * F * F);
     const int sw = F == 32 ? (n >> 1) & 3 : (n >> 2) & 1;
@@ -951,11 +952,61 @@ __global__ void __launch_bounds__(192, 1)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(W::kAlloc));
 }
 
+// A weight gradient voxel by voxel, dW[co][ci][k] = sum_v g[v][co] h[v + k - 1][ci] with
+// h zero beyond the volume. The kernels above also multiply zeros in the place of
+// gradients beyond it with activations inside, and the last convolution's leaves the
+// zeros beyond h out: the same sums, but not where a factor is infinite or NaN. An
+// infinity or NaN anywhere shows in the centre tap, whose pairs all lie inside; only
+// then (`odd`) does this kernel do its work, on the FP32 pipe, and its sums replace
+// theirs. One tap and one run of rows per block. 2 x 128^3, F = 32: all gradients 1.05
+// -> 1.06 ms with nothing to do, 44 ms with an infinite voxel.
+template <int F, int G>
+__global__ void __launch_bounds__(256) wgrad_plain_kernel(const bf16* __restrict__ g, const bf16* __restrict__ h,
+                                                          ConvDims d, float* __restrict__ part,
+                                                          const int* odd) {
+  constexpr int kOuts = F * G, kPer = kOuts >= 256 ? kOuts / 256 : 1;  // outputs, of a thread
+  constexpr int kSub = kOuts >= 256 ? 1 : 256 / kOuts;                 // threads of an output
+  __shared__ float red[256];
+  if (!*odd) return;
+  const int tap = blockIdx.x, t = threadIdx.x, ci = t % F, co = t / F % G, sub = t / kOuts;
+  const int dz = tap / 9 - 1, dy = tap / 3 % 3 - 1, dx = tap % 3 - 1;
+  const long long rows = (long long)d.B * d.Z * d.Y;
+  float acc[kPer];
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) acc[j] = 0.f;
+  for (long long r = rows * blockIdx.y / gridDim.y; r < rows * (blockIdx.y + 1) / gridDim.y; ++r) {
+    const int y = (int)(r % d.Y) + dy, z = (int)(r / d.Y % d.Z) + dz;
+    const bool in = y >= 0 && y < d.Y && z >= 0 && z < d.Z;
+    const bf16* gr = g + r * d.X * G + co;
+    const bf16* hr = h + (r + (long long)dz * d.Y + dy) * d.X * F + ci;
+    for (int x = sub; x < d.X; x += kSub) {
+      const bool ok = in && x + dx >= 0 && x + dx < d.X;
+      const float hv = ok ? __bfloat162float(hr[(long long)(x + dx) * F]) : 0.f;
+#pragma unroll
+      for (int j = 0; j < kPer; ++j)
+        acc[j] = fmaf(__bfloat162float(gr[(long long)x * G + j * (256 / F)]), hv, acc[j]);
+    }
+  }
+  float* p = part + ((long long)blockIdx.y * 27 + tap) * kOuts + ci;
+  if (kSub == 1) {
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) p[(co + j * (256 / F)) * F] = acc[j];
+    return;
+  }
+  red[t] = acc[0];
+  __syncthreads();
+  if (t >= kOuts) return;
+#pragma unroll
+  for (int i = 1; i < kSub; ++i) acc[0] += red[t + i * kOuts];
+  p[co * F] = acc[0];
+}
+
 // Adds the blocks' sums, element by element in a fixed order, and writes them to a
 // weight gradient [out, in, z, y, x] or a bias gradient in BF16. kind 0: rows of F
 // sums to a bias. 1, 2: rows [28][F] of wgrad_edge_kernel, to a weight whose one
 // channel is the input (1; tap 27 to the bias) or the output (2: the taps run
-// backwards). 3: rows [9 F][3 F] of wgrad_mid_kernel.
+// backwards). 3: rows [9 F][3 F] of wgrad_mid_kernel. 2 and 3 note in `odd` a
+// centre tap that is not finite.
 struct ConvGrad {
   bf16* w;
   bf16* b;
@@ -963,7 +1014,8 @@ struct ConvGrad {
 };
 template <int F>
 __global__ void __launch_bounds__(1024) conv_sum_kernel(const float* __restrict__ part, int n, int width,
-                                                        int kind, ConvGrad out, const int* status) {
+                                                        int kind, ConvGrad out, const int* status,
+                                                        int* odd) {
   __shared__ float red[32][33];
   const int e = blockIdx.x * 32 + threadIdx.x;
   float v = 0.f;
@@ -981,10 +1033,12 @@ __global__ void __launch_bounds__(1024) conv_sum_kernel(const float* __restrict_
   } else if (kind == 3) {
     const int col = e / (3 * F), m = e % (3 * F);
     const int kz = col / (3 * F), kx = col / F % 3, co = col % F, ky = m / F, ci = m % F;
+    if (kz == 1 && ky == 1 && kx == 1 && !isfinite(v)) *odd = 1;
     out.w[co * out.s[0] + ci * out.s[1] + kz * out.s[2] + ky * out.s[3] + kx * out.s[4]] = r;
   } else {
     int tap = e / F;
     const int c = e % F;
+    if (kind == 2 && tap == 13 && !isfinite(v)) *odd = 1;
     if (tap == 27) {
       if (kind == 1 && out.b) out.b[c] = r;
       return;
@@ -993,6 +1047,19 @@ __global__ void __launch_bounds__(1024) conv_sum_kernel(const float* __restrict_
     if (kind == 2) tap = 26 - tap;
     out.w[c * out.s[kind - 1] + tap / 9 * out.s[2] + tap / 3 % 3 * out.s[3] + tap % 3 * out.s[4]] = r;
   }
+}
+
+// The sums of wgrad_plain_kernel's n runs of rows, [27][G][F] each.
+template <int F, int G>
+__global__ void __launch_bounds__(256) plain_sum_kernel(const float* __restrict__ part, int n, ConvGrad out,
+                                                        const int* status, const int* odd) {
+  const int e = blockIdx.x * 256 + threadIdx.x;
+  if (!*odd || e >= 27 * F * G) return;
+  float v = 0.f;
+  for (int i = 0; i < n; ++i) v += part[(long long)i * 27 * F * G + e];
+  const int tap = e / (F * G), co = e % (F * G) / F, ci = e % F;
+  out.w[co * out.s[0] + ci * out.s[1] + tap / 9 * out.s[2] + tap / 3 % 3 * out.s[3] + tap % 3 * out.s[4]] =
+      __float2bfloat16_rn(*status ? __int_as_float(0x7fffffff) : v);
 }
 
 typedef CUresult (*ConvEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
@@ -1139,8 +1206,23 @@ long long conv_sum_bytes(const ConvDims& d, int sms) {
 
 template <int F>
 int launch_sum(const float* part, long long n, int width, int kind, const ConvGrad& g, const int* status,
-               cudaStream_t st) {
-  conv_sum_kernel<F><<<(width + 31) / 32, dim3(32, 32), 0, st>>>(part, (int)n, width, kind, g, status);
+               int* odd, cudaStream_t st) {
+  conv_sum_kernel<F><<<(width + 31) / 32, dim3(32, 32), 0, st>>>(part, (int)n, width, kind, g, status, odd);
+  note_launch();
+  DTV_LAUNCH_CHECK();
+  return DTV_OK;
+}
+
+// The weight gradient of g and h again, voxel by voxel, if `odd` says so (`part` holds
+// the sums of n blocks of it). 22 x 27 blocks are four per SM.
+template <int F, int G>
+int launch_plain(const bf16* g, const bf16* h, const ConvDims& d, float* part, long long n, const ConvGrad& out,
+                 const int* status, const int* odd, cudaStream_t st) {
+  n = std::min(n, 22ll);
+  wgrad_plain_kernel<F, G><<<dim3(27, (unsigned)n), 256, 0, st>>>(g, h, d, part, odd);
+  note_launch();
+  DTV_LAUNCH_CHECK();
+  plain_sum_kernel<F, G><<<(27 * F * G + 255) / 256, 256, 0, st>>>(part, (int)n, out, status, odd);
   note_launch();
   DTV_LAUNCH_CHECK();
   return DTV_OK;
@@ -1148,12 +1230,13 @@ int launch_sum(const float* part, long long n, int width, int kind, const ConvGr
 
 template <int F>
 int launch_edge_grad(const bf16* s, const bf16* T, const ConvDims& d, int sms, float* part, int kind,
-                     const ConvGrad& g, const int* status, cudaStream_t st) {
+                     const ConvGrad& g, int* status, int* odd, cudaStream_t st) {
   const int n = edge_blocks(d, sms);
   wgrad_edge_kernel<F><<<n, 256, 0, st>>>(s, T, d, conv_tiles(d, kInX, kInY, kInZ), part);
   note_launch();
   DTV_LAUNCH_CHECK();
-  return launch_sum<F>(part, n, 28 * F, kind, g, status, st);
+  const int rc = launch_sum<F>(part, n, 28 * F, kind, g, status, odd, st);
+  return rc || kind != 2 ? rc : launch_plain<F, 1>(s, T, d, part, n, g, status, odd, st);
 }
 
 // the kernel of the data gradient: taps backwards, in and out swapped
@@ -1168,14 +1251,14 @@ int conv_block_backward(const bf16* gy, const bf16* x, const ConvW* w, const bf1
   typedef Wgrad<F> W;
   int sms = 0, rc = conv_sms(&sms);
   if (rc) return rc;
-  const int* status = reinterpret_cast<int*>(ws + ConvWs<F>::kStatus);
+  int* status = reinterpret_cast<int*>(ws + ConvWs<F>::kStatus);
   float* part = reinterpret_cast<float*>(ws + ConvWs<F>::kStatus + 16);
   rc = launch_weights<F>(conv_flip(w[2]), conv_flip(w[1]), conv_flip(w[0]), ws, st);
-  if (!rc && g[2].w) rc = launch_edge_grad<F>(gy, h2, d, sms, part, 2, g[2], status, st);
+  if (!rc && g[2].w) rc = launch_edge_grad<F>(gy, h2, d, sms, part, 2, g[2], status, status + 1, st);
   if (rc || !g2) return rc;
   rc = launch_in<F, true>(gy, ws, nullptr, h2, g2, d, part, st);
   if (!rc && g[1].b)
-    rc = launch_sum<F>(part, conv_tiles(d, kInX, kInY, kInZ), F, 0, g[1], status, st);
+    rc = launch_sum<F>(part, conv_tiles(d, kInX, kInY, kInZ), F, 0, g[1], status, nullptr, st);
   if (!rc && g[1].w) {
     CUtensorMap hmap, gmap;
     rc = conv_map<F>(&hmap, h1, d, kCY + 2);
@@ -1185,15 +1268,15 @@ int conv_block_backward(const bf16* gy, const bf16* x, const ConvW* w, const bf1
                                       W::kSmem));
     const MidWork wk = mid_work(d, sms);
     const long long n = std::min<long long>(wk.items, sms);
-    wgrad_mid_kernel<F><<<(unsigned)n, 192, W::kSmem, st>>>(hmap, gmap, d, wk, part,
-                                                            const_cast<int*>(status));
+    wgrad_mid_kernel<F><<<(unsigned)n, 192, W::kSmem, st>>>(hmap, gmap, d, wk, part, status);
     note_launch();
     DTV_LAUNCH_CHECK();
-    rc = launch_sum<F>(part, n, 27 * F * F, 3, g[1], status, st);
+    rc = launch_sum<F>(part, n, 27 * F * F, 3, g[1], status, status + 2, st);
+    if (!rc) rc = launch_plain<F, F>(g2, h1, d, part, n, g[1], status, status + 2, st);
   }
   if (rc || !g1) return rc;
   rc = launch_mid<F, true>(g2, ws, nullptr, h1, g1, d, sms, st);
-  if (!rc && (g[0].w || g[0].b)) rc = launch_edge_grad<F>(x, g1, d, sms, part, 1, g[0], status, st);
+  if (!rc && (g[0].w || g[0].b)) rc = launch_edge_grad<F>(x, g1, d, sms, part, 1, g[0], status, nullptr, st);
   if (!rc && gx) rc = launch_out<F>(g1, ws, nullptr, gx, d, sms, st);
   return rc;
 }
