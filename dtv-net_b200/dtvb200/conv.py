@@ -14,21 +14,35 @@ from .geometry import _ptr, _stream
 _CONVS = (0, 2, 4)  # of the block's modules
 
 
+_HOOKS = ("_forward_hooks", "_forward_pre_hooks", "_backward_hooks", "_backward_pre_hooks")
+
+
 def _plain(m: nn.Module, kind) -> bool:
     """A module of exactly this class whose call runs its class's forward alone."""
-    return (type(m) is kind and "forward" not in m.__dict__ and not m._forward_hooks
-            and not m._forward_pre_hooks and not m._backward_hooks and not m._backward_pre_hooks)
+    return (type(m) is kind and "forward" not in m.__dict__
+            and not any(getattr(m, h, None) for h in _HOOKS))
+
+
+def _watchers():
+    """Tests for whatever watches or transforms the calls made here: tracing, functorch,
+    forward-mode differentiation, dispatch and function modes, global module hooks. Some
+    have no public name; a torch that lacks one of these keeps the general path."""
+    try:
+        peek, level = torch._C._functorch.peek_interpreter_stack, torch.autograd.forward_ad
+        dispatch, function = torch._C._len_torch_dispatch_stack, torch._C._len_torch_function_stack
+        level._current_level
+        return (torch.compiler.is_compiling, torch.jit.is_tracing, lambda: peek() is not None,
+                lambda: level._current_level >= 0, lambda: dispatch() > 0, lambda: function() > 0,
+                torch.nn.modules.module._has_any_global_hook)
+    except AttributeError:
+        return (lambda: True,)
+
+
+_WATCHERS = _watchers()
 
 
 def _special_modes() -> bool:
-    """Whether something watches or transforms the calls made here: tracing, functorch,
-    forward-mode differentiation, dispatch and function modes, global module hooks."""
-    return (torch.compiler.is_compiling() or torch.jit.is_tracing()
-            or torch._C._functorch.peek_interpreter_stack() is not None
-            or torch.autograd.forward_ad._current_level >= 0
-            or torch._C._len_torch_dispatch_stack() > 0
-            or torch._C._len_torch_function_stack() > 0
-            or torch.nn.modules.module._has_any_global_hook())
+    return any(w() for w in _WATCHERS)
 
 
 def supported(body: nn.Sequential, x: torch.Tensor) -> bool:
