@@ -3,6 +3,7 @@ BF16 through the library's kernels (csrc/conv.cu)."""
 from __future__ import annotations
 
 import ctypes
+import threading
 
 import torch
 import torch.nn as nn
@@ -12,8 +13,6 @@ from . import _lib
 from .geometry import _ptr, _stream
 
 _CONVS = (0, 2, 4)  # of the block's modules
-
-
 _HOOKS = ("_forward_hooks", "_forward_pre_hooks", "_backward_hooks", "_backward_pre_hooks")
 
 
@@ -45,24 +44,87 @@ def _special_modes() -> bool:
     return any(w() for w in _WATCHERS)
 
 
+_UNKNOWN = object()
+
+
+def _checkpoint_hook():
+    """What marks the non-reentrant torch.utils.checkpoint that saves, or recomputes, the
+    tensors saved here: its pack hook, None outside one (_UNKNOWN where torch does not
+    tell)."""
+    try:
+        top = torch._C._autograd._top_saved_tensors_default_hooks(True)
+    except (AttributeError, TypeError):
+        return _UNKNOWN
+    if top is None or getattr(top[0], "__module__", None) != "torch.utils.checkpoint":
+        return None
+    return top[0]
+
+
+_local = threading.local()  # .run: the call of a SamePath that this thread is in
+
+
+class SamePath:
+    """``fn``, to be checkpointed: the blocks called in it take the paths of its first call
+    at every later one. What watches the calls (_watchers, module hooks) may be there in
+    the forward pass and not when a checkpoint repeats it, or the other way round, and
+    the two paths save different tensors, which a checkpoint refuses."""
+
+    def __init__(self, fn):
+        self.fn = fn
+        self.paths = None  # of the first call, in order
+        # one of the caller's own checkpoints may repeat the first call itself
+        self.general = _checkpoint_hook() is not None
+
+    def __call__(self, *args):
+        outer = getattr(_local, "run", None)
+        replay = None if self.paths is None else iter(self.paths)
+        if replay is None:
+            self.paths = []
+        _local.run = (self, replay, _checkpoint_hook())
+        try:
+            return self.fn(*args)
+        finally:
+            _local.run = outer
+
+
+def fused(body: nn.Sequential, x: torch.Tensor) -> bool:
+    """Whether this call of the block goes to the kernels. In a checkpoint that is not a
+    SamePath's it does not: nothing tells its repetition what was chosen."""
+    run, replay, hook = getattr(_local, "run", None) or (None, None, None)
+    if _checkpoint_hook() not in (None, hook):
+        return False
+    if replay is not None:
+        return next(replay, False) and _computable(body, x)
+    path = supported(body, x) and not (run is not None and run.general)
+    if run is not None:
+        run.paths.append(path)
+    return path
+
+
 def supported(body: nn.Sequential, x: torch.Tensor) -> bool:
-    """Whether the block's call is one that the kernels compute: FP32 input and weights
-    on a GPU under BF16 autocast, 16 or 32 features (the weights of all taps stay in
-    shared memory), the block as it was built."""
+    """Whether the block's call is one that the kernels compute and nothing watches."""
+    return (_computable(body, x) and not _special_modes() and _plain(body, nn.Sequential)
+            and all(_plain(m, nn.ReLU if i % 2 else nn.Conv3d) for i, m in enumerate(body)))
+
+
+def _computable(body: nn.Sequential, x: torch.Tensor) -> bool:
+    """Whether the kernels compute it: FP32 input and weights on a GPU under BF16 autocast,
+    16 or 32 features (the weights of all taps stay in shared memory), the block as it
+    was built."""
     if not (type(x) is torch.Tensor and x.is_cuda and x.dtype == torch.float32 and x.dim() == 5
             and x.shape[1] == 1 and x.numel() > 0 and torch.is_autocast_enabled("cuda")
             and torch.get_autocast_dtype("cuda") == torch.bfloat16):
         return False
-    if _special_modes() or not _plain(body, nn.Sequential) or len(body) != 5:
+    if type(body) is not nn.Sequential or len(body) != 5:
         return False
     f = body[0].out_channels if type(body[0]) is nn.Conv3d else 0
-    if f not in (16, 32) or not (_plain(body[1], nn.ReLU) and _plain(body[3], nn.ReLU)):
+    if f not in (16, 32) or type(body[1]) is not nn.ReLU or type(body[3]) is not nn.ReLU:
         return False
     if max(x.shape) >= 1 << 24 or x.numel() >= 1 << 32:
         return False
     for i, (ci, co) in zip(_CONVS, ((1, f), (f, f), (f, 1))):
         m = body[i]
-        if not (_plain(m, nn.Conv3d) and m.kernel_size == (3, 3, 3) and m.stride == (1, 1, 1)
+        if not (type(m) is nn.Conv3d and m.kernel_size == (3, 3, 3) and m.stride == (1, 1, 1)
                 and m.padding == (1, 1, 1) and m.dilation == (1, 1, 1) and m.groups == 1
                 and m.padding_mode == "zeros" and m.bias is not None):
             return False

@@ -241,7 +241,7 @@ class ConvBlock(nn.Module):
     """Conv3d(1, f) - ReLU - Conv3d(f, f) - ReLU - Conv3d(f, 1), 3x3x3 kernels
     (the shape of model/PDHG/RegularizationLayers/CNN.py:4-18 with three layers).
     Under BF16 autocast on a GPU the library's kernels compute it where they can
-    (conv.supported)."""
+    (conv.supported), but not in a checkpoint of the caller's own (conv.SamePath)."""
 
     def __init__(self, features: int = 32):
         super().__init__()
@@ -252,7 +252,7 @@ class ConvBlock(nn.Module):
 
     def forward(self, x):
         if not torch.jit.is_scripting():  # (a script keeps the modules, and so does a compiler)
-            if not torch.compiler.is_compiling() and conv.supported(self.body, x):
+            if not torch.compiler.is_compiling() and conv.fused(self.body, x):
                 return conv.conv_block(self.body, x)
         return self.body(x)
 
@@ -292,7 +292,8 @@ class UnrolledPDHG(nn.Module):
         xs = [x0]
         for s in range(self.stages):
             if self.checkpoint_stages and torch.is_grad_enabled():
-                x = checkpoint(self.stage, s, x, p, use_reentrant=False)
+                stage = self.stage if torch.compiler.is_compiling() else conv.SamePath(self.stage)
+                x = checkpoint(stage, s, x, p, use_reentrant=False)
             else:
                 x = self.stage(s, x, p)
             if return_all:
