@@ -1295,6 +1295,7 @@ int dtv_conv_block(const void* x, const void* const weights[3], const int64_t st
                    int32_t batch, int32_t features, void* workspace, void* stream) {
   DTV_CHECK(x && weights && strides && biases && h1 && h2 && y && size && workspace, "NULL argument");
   DTV_CHECK(size[0] > 0 && size[1] > 0 && size[2] > 0 && batch > 0, "empty volume");
+  DTV_CHECK((int64_t)size[0] * size[1] < (1ll << 31), "plane of 2^31 voxels or more");
   DTV_CHECK(features == 16 || features == 32, "features must be 16 or 32");
   ConvW w[3];
   const bf16* bias[3];
@@ -1329,6 +1330,7 @@ int dtv_conv_block_backward(const void* gy, const void* x, const void* const wei
   DTV_CHECK(gy && x && weights && strides && h1 && h2 && grad_weights && grad_strides && grad_biases &&
                 size && workspace, "NULL argument");
   DTV_CHECK(size[0] > 0 && size[1] > 0 && size[2] > 0 && batch > 0, "empty volume");
+  DTV_CHECK((int64_t)size[0] * size[1] < (1ll << 31), "plane of 2^31 voxels or more");
   DTV_CHECK(features == 16 || features == 32, "features must be 16 or 32");
   ConvW w[3];
   ConvGrad g[3];

@@ -3,6 +3,7 @@ BF16 through the library's kernels (csrc/conv.cu)."""
 from __future__ import annotations
 
 import ctypes
+import math
 import threading
 
 import torch
@@ -107,6 +108,13 @@ def supported(body: nn.Sequential, x: torch.Tensor) -> bool:
             and all(_plain(m, nn.ReLU if i % 2 else nn.Conv3d) for i, m in enumerate(body)))
 
 
+def _fits(shape) -> bool:
+    """Whether the kernels index a volume of this shape, [batch, 1, z, y, x]: a plane in 32
+    bits, an axis in FP32."""
+    return (max(shape) < 1 << 24 and math.prod(shape) < 1 << 32
+            and shape[-1] * shape[-2] < 1 << 31)
+
+
 def _computable(body: nn.Sequential, x: torch.Tensor) -> bool:
     """Whether the kernels compute it: FP32 input and weights on a GPU under BF16 autocast,
     16 or 32 features (the weights of all taps stay in shared memory), the block as it
@@ -120,7 +128,7 @@ def _computable(body: nn.Sequential, x: torch.Tensor) -> bool:
     f = body[0].out_channels if type(body[0]) is nn.Conv3d else 0
     if f not in (16, 32) or type(body[1]) is not nn.ReLU or type(body[3]) is not nn.ReLU:
         return False
-    if max(x.shape) >= 1 << 24 or x.numel() >= 1 << 32:
+    if not _fits(x.shape):
         return False
     for i, (ci, co) in zip(_CONVS, ((1, f), (f, f), (f, 1))):
         m = body[i]
