@@ -448,7 +448,7 @@ __global__ void __launch_bounds__(kBPThreads, kMode == kRec && kZAff && S == 1 ?
                                          (int)blockIdx.x, (int)blockIdx.y);
 }
 
-// Writes the records of a sinogram (all views): record (U, V) of a view from
+// Writes the records of a sinogram's views: record (U, V) of a view from
 // the four detector values (u, v) = (U - 2 .. U - 1, V - 2 .. V - 1), zero
 // outside the view. Only records that reach the view (U in [1, nu+1], V in
 // [1, nv+1]) are written; the rest keep the plan's initial zeros. A warp owns
@@ -585,19 +585,21 @@ static BPParams plan_bp_params(const Plan* p) {
   return bp;
 }
 
-// Copies one batch item's sinogram into the plan's staged form: the layered
-// texture (texture plans) or the records.
-static int stage_sino(Plan* p, const float* sino, cudaStream_t st) {
+// Copies one batch item's sinogram into the plan's layered texture.
+static int stage_sino_tex(Plan* p, const float* sino, cudaStream_t st) {
   const GeomParams& gp = p->gp;
-  if (p->sino_tex != nullptr) {
-    const dim3 grid((gp.nu + 31) / 32, (gp.nv + 31) / 32, gp.n_views);
-    stage_sino_tex_kernel<<<grid, 256, 0, st>>>(sino, p->sino_surf, gp.nu, gp.nv);
-    note_launch();
-    DTV_LAUNCH_CHECK();
-    return DTV_OK;
-  }
+  const dim3 grid((gp.nu + 31) / 32, (gp.nv + 31) / 32, gp.n_views);
+  stage_sino_tex_kernel<<<grid, 256, 0, st>>>(sino, p->sino_surf, gp.nu, gp.nv);
+  note_launch();
+  DTV_LAUNCH_CHECK();
+  return DTV_OK;
+}
+
+// Writes the records of `views` views.
+static int stage_sino_rec(Plan* p, const float* sino, int views, cudaStream_t st) {
+  const GeomParams& gp = p->gp;
   const int64_t warps = (int64_t)((gp.nu + 1 + 31) / 32) *
-                        ((gp.nv + 1 + kSinoRows - 1) / kSinoRows) * gp.n_views;
+                        ((gp.nv + 1 + kSinoRows - 1) / kSinoRows) * views;
   const int64_t blocks = (warps + 7) / 8;
   DTV_CHECK(blocks < 2147483647LL, "sinogram too large for one staging launch");
   stage_sino_kernel<<<(unsigned)blocks, 256, 0, st>>>(sino, p->d_sino_rec, gp.nu, gp.nv, warps);
@@ -635,26 +637,37 @@ int bp_cull_rule(const Plan* p) {
   return missed * 2 >= total ? 1 : 0;
 }
 
-// The views in chunks of kBPParamViews (their maps travel in the launch
-// parameters); later chunks add onto the first one's result.
-static int bp_view_chunks(const Plan* p, int mode, const float4* recs, BPOut dst,
+// The views in chunks of kBPParamViews (their maps travel in the launch parameters), and
+// where records are sampled in runs of as many views as the records of plan `rec` hold,
+// each staged from `sino` first; later chunks add onto the first one's result.
+static int bp_view_chunks(const Plan* p, int mode, Plan* rec, const float* sino, BPOut dst,
                           cudaStream_t st) {
   const GeomParams& gp = p->gp;
   const BPParams bp = plan_bp_params(p);
   const cudaTextureObject_t tex = p->sino_tex ? p->sino_tex[0] : 0;
   const int S = bp_split(gp);
   const BPLaunch l{dim3(bp_tiles(gp, S), (gp.nz + kZC - 1) / kZC), S, st};
+  const int run = mode == kTex ? gp.n_views : rec->sino_rec_views;
   BPMaps maps;
-  for (int n0 = 0; n0 < gp.n_views; n0 += kBPParamViews) {
-    const int cnt = std::min(kBPParamViews, gp.n_views - n0);
-    for (int j = 0; j < cnt; ++j) memcpy(maps.m[j], p->h_bpv[n0 + j].m, sizeof(maps.m[j]));
-    if (n0 > 0) {
-      dst.base = dst.out;
-      dst.diff_base = dst.diff;  // (kBoth only)
+  for (int r0 = 0; r0 < gp.n_views; r0 += run) {
+    const int r1 = std::min(r0 + run, gp.n_views);
+    const float4* recs = nullptr;  // as if of view 0
+    if (mode != kTex) {
+      const int rc = stage_sino_rec(rec, sino + (int64_t)r0 * gp.nu * gp.nv, r1 - r0, st);
+      if (rc) return rc;
+      recs = rec->d_sino_rec - r0 * bp.view_recs;
     }
-    launch_bp(mode, l, p->bp_zaffine != 0, bp, maps, n0, cnt, recs, tex, dst);
-    note_launch();
-    DTV_LAUNCH_CHECK();
+    for (int n0 = r0; n0 < r1; n0 += kBPParamViews) {
+      const int cnt = std::min(kBPParamViews, r1 - n0);
+      for (int j = 0; j < cnt; ++j) memcpy(maps.m[j], p->h_bpv[n0 + j].m, sizeof(maps.m[j]));
+      if (n0 > 0) {
+        dst.base = dst.out;
+        dst.diff_base = dst.diff;  // (kBoth only)
+      }
+      launch_bp(mode, l, p->bp_zaffine != 0, bp, maps, n0, cnt, recs, tex, dst);
+      note_launch();
+      DTV_LAUNCH_CHECK();
+    }
   }
   return DTV_OK;
 }
@@ -665,9 +678,10 @@ int backward_impl(Plan* p, const float* sino, int batch, const float* base, floa
   const int64_t per_item = (int64_t)gp.nu * gp.nv * gp.n_views;
   const int64_t vox = (int64_t)gp.nx * gp.ny * gp.nz;
   for (int b = 0; b < batch; ++b) {
-    int rc = stage_sino(p, sino + b * per_item, st);
+    const float* s = sino + b * per_item;
+    int rc = p->sino_tex ? stage_sino_tex(p, s, st) : DTV_OK;
     if (rc) return rc;
-    rc = bp_view_chunks(p, p->sino_tex ? kTex : kRec, p->d_sino_rec,
+    rc = bp_view_chunks(p, p->sino_tex ? kTex : kRec, p, s,
                         BPOut{out + b * vox, base ? base + b * vox : nullptr, nullptr, nullptr}, st);
     if (rc) return rc;
   }
@@ -683,13 +697,13 @@ int backward_refresh_impl(Plan* fast, Plan* exact, const float* sino, int batch,
   const int64_t per_item = (int64_t)gp.nu * gp.nv * gp.n_views;
   const int64_t vox = (int64_t)gp.nx * gp.ny * gp.nz;
   for (int b = 0; b < batch; ++b) {
-    int rc = stage_sino(exact, sino + b * per_item, st);
-    if (rc) return rc;
+    const float* s = sino + b * per_item;
     // beyond a layered texture's views the fast plan samples records too: no difference
     const bool both = fast->sino_tex != nullptr;
-    if (both && (rc = stage_sino(fast, sino + b * per_item, st))) return rc;
+    int rc = both ? stage_sino_tex(fast, s, st) : DTV_OK;
+    if (rc) return rc;
     const BPOut dst{out + b * vox, nullptr, both ? e_b + b * vox : nullptr, nullptr};
-    rc = bp_view_chunks(fast, both ? kBoth : kRec, exact->d_sino_rec, dst, st);
+    rc = bp_view_chunks(fast, both ? kBoth : kRec, exact, s, dst, st);
     if (rc) return rc;
     if (!both) DTV_CUDA_TRY(cudaMemsetAsync(e_b + b * vox, 0, vox * sizeof(float), st));
   }
@@ -778,7 +792,7 @@ int backward_many_impl(Plan* const* plans, const float* const* sinos, float* con
     for (int k = 0; k < cnt; ++k) {
       Plan* p = plans[ord[c0 + k]];
       const GeomParams& gp = p->gp;
-      const int rc = stage_sino(p, sinos[ord[c0 + k]], st);
+      const int rc = stage_sino_tex(p, sinos[ord[c0 + k]], st);
       if (rc) return rc;
       BPManyItem& it = m.it[k];
       it.bp = plan_bp_params(p);

@@ -180,6 +180,7 @@ struct Plan {
   // backprojector: the sinogram of one batch item as 16-byte records (one
   // bilinear detector cell each) or, texture plans, a layered array
   float4* d_sino_rec;
+  int sino_rec_views;  // views that d_sino_rec holds
   cudaArray_t* sino_arrays;
   cudaTextureObject_t* sino_tex;
   cudaSurfaceObject_t sino_surf;
@@ -219,6 +220,8 @@ constexpr int kNumRayTiles = 8;  // forward-projector ray tiles (DTV_TUNE_FP_RAY
 // default forward block order (DTV_TUNE_FP_BAND): bands of kDefaultBand tile
 // rows for staged volumes above kBandAboveBytes, view by view below
 constexpr int kDefaultBand = 4;
+// most bytes of a plan's sinogram records (plan.cu)
+constexpr int64_t kSinoRecBytes = 4LL << 30;
 constexpr double kBandAboveBytes = 32.0 * (1 << 20);
 constexpr int kPad = 2;  // zero border of the staged volume
 

@@ -298,10 +298,15 @@ int create_plan(const dtv_geometry* g, int max_batch, int flags, int device, Pla
     rd.res.array.array = p->sino_arrays[0];
     PLAN_CUDA(cudaCreateSurfaceObject(&p->sino_surf, &rd));
   } else {
-    // records: zero borders written once here, those that reach the view by each call
-    const int64_t recs = (int64_t)(gp.nu + 2 * kPad) * (gp.nv + 2 * kPad) * gp.n_views;
-    PLAN_CUDA(cudaMalloc(&p->d_sino_rec, sizeof(float4) * recs));
-    PLAN_CUDA(cudaMemset(p->d_sino_rec, 0, sizeof(float4) * recs));
+    // records: zero borders written once here, those that reach the view by each call.
+    // At most kSinoRecBytes of them: a longer scan is staged and projected in runs of
+    // views. A record is four times its pixel, so that without the limit a sinogram of
+    // 20 GB took 80 GB here; a run then is a large part of a second's work beside which
+    // another pass over the volume is nothing.
+    const int64_t view = (int64_t)(gp.nu + 2 * kPad) * (gp.nv + 2 * kPad) * (int64_t)sizeof(float4);
+    p->sino_rec_views = (int)std::min<int64_t>(gp.n_views, std::max<int64_t>(1, kSinoRecBytes / view));
+    PLAN_CUDA(cudaMalloc(&p->d_sino_rec, view * p->sino_rec_views));
+    PLAN_CUDA(cudaMemset(p->d_sino_rec, 0, view * p->sino_rec_views));
   }
   if (flags & DTV_PLAN_ADJOINT) {
     const size_t n = (size_t)gp.n_views * gp.nu * gp.nv * 2;
