@@ -50,7 +50,9 @@ constexpr int kZC = 8;
 // B = s(U+1, V) - A, C = s(U, V+1) - A, D the mixed difference.
 // kBoth: both, two sums per voxel (the correction pass of a texture plan
 // against an exact one).
-enum BPMode { kRec = 0, kTex = 1, kBoth = 2 };
+// kWide: kRec on detectors with more rows or columns than kIntMagicMost, cells by floorf
+// (a kernel of its own: as a branch it cost the record kernels 7 %).
+enum BPMode { kRec = 0, kTex = 1, kBoth = 2, kWide = 3 };
 
 // Where a block's sums go: out = base + sum (out = sum when base is NULL; base
 // may be out). kBoth: out takes the record sum E, and
@@ -101,6 +103,17 @@ __device__ __forceinline__ unsigned long long cell_base(const char* view, unsign
 __device__ __forceinline__ float4 cell_at(unsigned long long base, unsigned int tv_bits,
                                           unsigned int row_bytes) {
   return __ldg(reinterpret_cast<const float4*>(base + (unsigned long long)tv_bits * row_bytes));
+}
+
+// The sample at (u, v) of a view, cell by floorf and 64-bit index.
+__device__ __forceinline__ float sample_wide(const char* view, float u, float v, float mu, float mv) {
+  u = fminf(fmaxf(u, -2.f), mu);
+  v = fminf(fmaxf(v, -2.f), mv);
+  const float fu = floorf(u), fv = floorf(v);
+  const long long row = (long long)mu + 2 * kPad;
+  const float4 r = __ldg(reinterpret_cast<const float4*>(view) + ((long long)fv + kPad) * row +
+                         (long long)fu + kPad);
+  return bilinear(r, splat2(u - fu), v - fv);
 }
 
 // Whether view map w can see any voxel of the box [i0, i1] x [j0, j1] x
@@ -258,7 +271,7 @@ __device__ __forceinline__ void bp_columns(const BPParams& bp, const Maps& maps,
       float tu_f, dummy;
       unpack2(fu.t, tu_f, dummy);
       const unsigned long long base = cell_base(view, __float_as_uint(tu_f), row_bytes);
-      const bool inside = vlo >= -1.f && vhi < mv && u >= -1.f && u < mu && !bp.extent;
+      const bool inside = vlo >= -1.f && vhi < mv && u >= -1.f && u < mu && !bp.extent && kMode != kWide;
       if (kMode == kTex || inside) {
 #pragma unroll
         for (int z = 0; z < ZC; z += 2) {
@@ -266,7 +279,7 @@ __device__ __forceinline__ void bp_columns(const BPParams& bp, const Maps& maps,
               fma2(f32x2(kf0 + (float)z, kf0 + (float)(z + 1)), splat2(dv), splat2(vb));
           float v[2], w2[2] = {wgt, wgt};
           unpack2(v2, v[0], v[1]);
-          if constexpr (kMode != kRec) {
+          if constexpr (kMode == kTex || kMode == kBoth) {
 #pragma unroll
             for (int y = 0; y < 2; ++y) {
               const float tv = __fadd_rn(v[y], 0.5f);
@@ -297,7 +310,10 @@ __device__ __forceinline__ void bp_columns(const BPParams& bp, const Maps& maps,
           float t0, av;
           unpack2(fv.t, t0, dummy);
           unpack2(fv.a, av, dummy);
-          acc[z] = fmaf(bilinear(cell_at(base, __float_as_uint(t0), row_bytes), fu.a, av), wz, acc[z]);
+          const float val = kMode == kWide
+                                ? sample_wide(view, u, v, mu, mv)
+                                : bilinear(cell_at(base, __float_as_uint(t0), row_bytes), fu.a, av);
+          acc[z] = fmaf(val, wz, acc[z]);
           if constexpr (kMode == kBoth)
             act[z] = fmaf(tex2DLayered<float>(tex, tu, tv, n0 + jn), wz, act[z]);
         }
@@ -331,6 +347,7 @@ __device__ __forceinline__ void bp_columns(const BPParams& bp, const Maps& maps,
         // u and v are monotone along the run up to rounding, hence the margin
         beside = front && (uhi < -1.02f || ulo > mu + 0.02f || vhi < -1.02f || vlo > mv + 0.02f);
         inside = front && ulo >= -1.f && uhi < mu && vlo >= -1.f && vhi < mv;
+        inside = inside && kMode != kWide;
         if (bp.extent)
           inside = inside && __fadd_rn(uhi, 0.5f) <= bp.nx + 1.f && __fadd_rn(vhi, 0.5f) <= bp.ny + 1.f;
       }
@@ -360,7 +377,7 @@ __device__ __forceinline__ void bp_columns(const BPParams& bp, const Maps& maps,
           uu = f32x2(fminf(fmaxf(u0, -2.f), mu), fminf(fmaxf(u1, -2.f), mu));
           vv = f32x2(fminf(fmaxf(v0, -2.f), mv), fminf(fmaxf(v1, -2.f), mv));
         }
-        if constexpr (kMode != kRec) {
+        if constexpr (kMode == kTex || kMode == kBoth) {
           unpack2(p.u, u0, u1);
           unpack2(p.v, v0, v1);
           const float uy[2] = {u0, u1}, vy[2] = {v0, v1};
@@ -380,9 +397,14 @@ __device__ __forceinline__ void bp_columns(const BPParams& bp, const Maps& maps,
           unpack2(fv.a, av[0], av[1]);
 #pragma unroll
           for (int y = 0; y < 2; ++y) {
-            const float4 r = cell_at(vbase + (unsigned long long)__float_as_uint(tu[y]) * 16u,
-                                     __float_as_uint(tv[y]), row_bytes);
-            acc[z + y] = fmaf(bilinear(r, splat2(au[y]), av[y]), y ? w1 : w0, acc[z + y]);
+            float val;
+            if (checked && kMode == kWide)
+              val = sample_wide(view, y ? u1 : u0, y ? v1 : v0, mu, mv);
+            else
+              val = bilinear(cell_at(vbase + (unsigned long long)__float_as_uint(tu[y]) * 16u,
+                                     __float_as_uint(tv[y]), row_bytes),
+                             splat2(au[y]), av[y]);
+            acc[z + y] = fmaf(val, y ? w1 : w0, acc[z + y]);
           }
         }
       };
@@ -566,7 +588,11 @@ static void launch_bp_mode(const BPLaunch& l, bool zaff, const BPParams& bp, con
 static void launch_bp(int mode, const BPLaunch& l, bool zaff, const BPParams& bp,
                       const BPMaps& maps, int n0, int cnt, const float4* recs,
                       cudaTextureObject_t tex, const BPOut& dst) {
-  if (mode == kTex) launch_bp_mode<kTex>(l, zaff, bp, maps, n0, cnt, recs, tex, dst);
+  if (mode == kWide && zaff)
+    bp_kernel<kWide, true, 1, false><<<l.grid, kBPThreads, 0, l.st>>>(bp, maps, n0, cnt, recs, tex, dst);
+  else if (mode == kWide)
+    bp_kernel<kWide, false, 1, false><<<l.grid, kBPThreads, 0, l.st>>>(bp, maps, n0, cnt, recs, tex, dst);
+  else if (mode == kTex) launch_bp_mode<kTex>(l, zaff, bp, maps, n0, cnt, recs, tex, dst);
   else if (mode == kBoth) launch_bp_mode<kBoth>(l, zaff, bp, maps, n0, cnt, recs, tex, dst);
   else launch_bp_mode<kRec>(l, zaff, bp, maps, n0, cnt, recs, tex, dst);
 }
@@ -645,7 +671,8 @@ static int bp_view_chunks(const Plan* p, int mode, Plan* rec, const float* sino,
   const GeomParams& gp = p->gp;
   const BPParams bp = plan_bp_params(p);
   const cudaTextureObject_t tex = p->sino_tex ? p->sino_tex[0] : 0;
-  const int S = bp_split(gp);
+  if (mode == kRec && std::max(gp.nu, gp.nv) + 2 * kPad > kIntMagicMost) mode = kWide;
+  const int S = mode == kWide ? 1 : bp_split(gp);
   const BPLaunch l{dim3(bp_tiles(gp, S), (gp.nz + kZC - 1) / kZC), S, st};
   const int run = mode == kTex ? gp.n_views : rec->sino_rec_views;
   BPMaps maps;

@@ -108,6 +108,7 @@ __device__ __forceinline__ f32x2_t fma2(f32x2_t a, f32x2_t b, f32x2_t c) {
 // a quarter rate.
 constexpr float kIntMagic = 12582912.f;
 constexpr unsigned int kIntMagicBits = 0x4B400000u;
+constexpr int kIntMagicMost = 1 << 22;  // beyond it the sums' steps are more than 1
 
 // 1 / x by one Newton step r + r (1 - x r) on the approximate reciprocal. kAny: x may
 // be zero or infinite, where 1 - x r is no remainder and r, infinite or zero, stands.

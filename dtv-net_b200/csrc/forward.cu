@@ -65,11 +65,12 @@ struct SoftSampler {
 // record with one 64-bit multiply-add per axis; two samples go through packed
 // FP32.
 
-// kFar: a row of records spans 4 GB or more (its pitch needs 64 bits).
+// kFar: a row of records spans 4 GB or more (its pitch needs 64 bits), or an axis has
+// 2^22 voxels or more (kIntMagic's sums then round to more than 1): floors by floorf.
 template <bool kFar>
 struct RecSampler {
   using Pitch = typename std::conditional<kFar, unsigned long long, unsigned int>::type;
-  unsigned long long base;  // record (0, 0, 0), biased by the magic bits on each axis
+  unsigned long long base;  // record (0, 0, 0), biased by the magic bits on each axis (not far)
   Pitch py;                 // bytes from y to y + 1
   unsigned int px;          // bytes from x to x + 1
   float nx, ny, nz;
@@ -79,27 +80,41 @@ struct RecSampler {
     py = (Pitch)px * (Pitch)(rp.nx + 2 * kPad);
     const unsigned long long step = (unsigned long long)py + px + 16u;
     base = (unsigned long long)rec + (unsigned long long)kPad * step -
-           (unsigned long long)kIntMagicBits * step;
+           (kFar ? 0ull : (unsigned long long)kIntMagicBits * step);
     nx = (float)rp.nx; ny = (float)rp.ny; nz = (float)rp.nz;
   }
-  // floors plus kIntMagic in t, fractions in a
+  // floors plus kIntMagic (far: floors) in t, fractions in a
   __device__ __forceinline__ float at(float tx, float ty, float tz, float ax, float ay,
                                       float az) const {
-    const float4* r = reinterpret_cast<const float4*>(
-        base + (unsigned long long)__float_as_uint(ty) * py +
-        (unsigned long long)__float_as_uint(tx) * px +
-        (unsigned long long)__float_as_uint(tz) * 16u);
+    const auto index = [](float t) {
+      return kFar ? (unsigned long long)(long long)t : (unsigned long long)__float_as_uint(t);
+    };
+    const float4* r =
+        reinterpret_cast<const float4*>(base + index(ty) * py + index(tx) * px + index(tz) * 16u);
     const float4 lo = __ldg(r), hi = __ldg(r + 1);
     const float s0 = fmaf(ay, fmaf(ax, lo.w, lo.y), fmaf(ax, lo.z, lo.x));
     const float s1 = fmaf(ay, fmaf(ax, hi.w, hi.y), fmaf(ax, hi.z, hi.x));
     return fmaf(az, s1 - s0, s0);
   }
   __device__ __forceinline__ float one(float x, float y, float z) const {
+    if constexpr (kFar) {
+      const float fx = floorf(x), fy = floorf(y), fz = floorf(z);
+      return at(fx, fy, fz, x - fx, y - fy, z - fz);
+    }
     const float tx = __fadd_rd(x, kIntMagic), ty = __fadd_rd(y, kIntMagic),
                 tz = __fadd_rd(z, kIntMagic);
     return at(tx, ty, tz, x - (tx - kIntMagic), y - (ty - kIntMagic), z - (tz - kIntMagic));
   }
   __device__ __forceinline__ void two(f32x2_t x, f32x2_t y, f32x2_t z, float (&s)[2]) const {
+    if constexpr (kFar) {
+      float xs[2], ys[2], zs[2];
+      unpack2(x, xs[0], xs[1]);
+      unpack2(y, ys[0], ys[1]);
+      unpack2(z, zs[0], zs[1]);
+#pragma unroll
+      for (int j = 0; j < 2; ++j) s[j] = one(xs[j], ys[j], zs[j]);
+      return;
+    }
     const f32x2_t m = splat2(kIntMagic);
     const f32x2_t tx = add2_rm(x, m), ty = add2_rm(y, m), tz = add2_rm(z, m);
     float t[3][2], a[3][2];
@@ -584,9 +599,10 @@ static int stage_volume(Plan* p, const void* vol, int vol_dtype, int batch, cuda
   return rc;
 }
 
-// Whether a row of records spans 4 GB or more.
+// RecSampler's kFar.
 static bool rec_far(const GeomParams& g) {
-  return (int64_t)(g.nx + 2 * kPad) * (g.nz + 2 * kPad) * 16 >= (1LL << 32);
+  return (int64_t)(g.nx + 2 * kPad) * (g.nz + 2 * kPad) * 16 >= (1LL << 32) ||
+         std::max(g.nx, std::max(g.ny, g.nz)) + 2 * kPad > kIntMagicMost;
 }
 
 // `records`: the launch samples records, whose warps want two columns of 16 pixels
@@ -1102,7 +1118,8 @@ int adjoint_impl(Plan* p, const float* sino, int batch, float* out, cudaStream_t
   const GeomParams& gp = p->gp;
   RayParams rp = make_ray_params(gp);
   const int64_t vox = (int64_t)gp.nx * gp.ny * gp.nz;
-  if (p->adjoint_method == 1 && p->d_cells) {
+  const bool wide = std::max(gp.nx, std::max(gp.ny, gp.nz)) + 2 * kPad > kIntMagicMost;
+  if (p->adjoint_method == 1 && p->d_cells && !wide) {
     DTV_CUDA_TRY(cudaMemsetAsync(p->d_cells, 0, p->pad_elems * batch * sizeof(float4), st));
     // warps of 4 x 8 rays: 128^3 x 48 views 0.68 ms (1 x 32: 0.73, 2 x 16: 0.69;
     // 97x113x61 x 33 views: 271, 334, 291 us)
