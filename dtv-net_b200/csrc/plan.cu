@@ -180,6 +180,7 @@ int create_plan(const dtv_geometry* g, int max_batch, int flags, int device, Pla
   // Staged volumes of the software samplers (16-byte records; FP16-staged: the
   // padded volume): zero border written once here, interiors by each call.
   if (flags & DTV_PLAN_PAIRS_EXACT) {
+    // these plans' limit, a little below that of the padded grid (validate_geometry)
     const int64_t most = (int64_t)(gp.nx + 6) * (gp.ny + 6) * (gp.nz + 5);
     if (most >= (1LL << 31)) {
       free_plan(p);

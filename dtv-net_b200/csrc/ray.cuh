@@ -48,7 +48,7 @@ __device__ __forceinline__ double rcp64(double x) {
   r = __fma_rn(r, __fma_rn(-x, r, 1.0), r);
   return __fma_rn(r, __fma_rn(-x, r, 1.0), r);
 }
-// x / d from q = 1 / d: the quotient corrected by its remainder.
+// x / d from q = 1 / d: the quotient corrected by its remainder (Markstein 1990).
 __device__ __forceinline__ double div64(double x, double d, double q) {
   const double t = __dmul_rn(x, q);
   return __fma_rn(__fma_rn(-t, d, x), q, t);
