@@ -450,11 +450,12 @@ constexpr int kRecX = 32, kRecY = 4, kRecZ = 32;
 template <class Tin, bool kRound>
 __global__ void __launch_bounds__(256) stage_rec_kernel(const Tin* __restrict__ in,
                                                         float4* __restrict__ rec, int nx, int ny,
-                                                        int nz, int ztiles, int64_t pad_elems) {
+                                                        int nz, int xtiles, int ytiles,
+                                                        int64_t pad_elems) {
   __shared__ float s[kRecY + 1][kRecX + 1][kRecZ + 1];
-  const int b = blockIdx.z / ztiles;
-  const int x0 = (int)blockIdx.x * kRecX - 1, y0 = (int)blockIdx.y * kRecY - 1,
-            z0 = (int)(blockIdx.z % ztiles) * kRecZ;
+  const int b = blockIdx.y, row = (int)blockIdx.x / xtiles;
+  const int x0 = (int)blockIdx.x % xtiles * kRecX - 1, y0 = row % ytiles * kRecY - 1,
+            z0 = row / ytiles * kRecZ;
   const Tin* vol = in + (int64_t)b * nx * ny * nz;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   // rows (y, z) of the tile, 33 values from x0: a warp takes four of each y, and its
@@ -509,13 +510,13 @@ template <class Tin, bool kRound>
 static int stage_volume_rec(Plan* p, const Tin* vol, int batch, cudaStream_t st) {
   const GeomParams& g = p->gp;
   const int64_t vox = (int64_t)g.nx * g.ny * g.nz;
-  const int ztiles = (g.nz + kRecZ - 1) / kRecZ;
-  const int per = std::max(1, 65535 / ztiles);  // volumes per launch
-  for (int b = 0; b < batch; b += per) {
-    const dim3 grid((g.nx + 1 + kRecX - 1) / kRecX, (g.ny + 1 + kRecY - 1) / kRecY,
-                    ztiles * std::min(per, batch - b));
+  // a flat grid of tiles: an axis may have more of them than a grid's y or z holds
+  const int xtiles = (g.nx + 1 + kRecX - 1) / kRecX, ytiles = (g.ny + 1 + kRecY - 1) / kRecY;
+  const unsigned tiles = (unsigned)xtiles * ytiles * ((g.nz + kRecZ - 1) / kRecZ);
+  for (int b = 0; b < batch; b += 65535) {
+    const dim3 grid(tiles, std::min(65535, batch - b));
     stage_rec_kernel<Tin, kRound><<<grid, 256, 0, st>>>(vol + b * vox, p->d_vol_rec + b * p->pad_elems,
-                                                        g.nx, g.ny, g.nz, ztiles, p->pad_elems);
+                                                        g.nx, g.ny, g.nz, xtiles, ytiles, p->pad_elems);
     note_launch();
     DTV_LAUNCH_CHECK();
   }
@@ -1086,13 +1087,13 @@ __global__ void __launch_bounds__(256, 5) adjoint_cells_kernel(RayParams rp,
 // that the volume is written along x.
 __global__ void __launch_bounds__(256) adjoint_gather_kernel(const float4* __restrict__ cells,
                                                              float* __restrict__ out, int nx,
-                                                             int ny, int nz, int ytiles,
+                                                             int ny, int nz, int xtiles, int ytiles,
                                                              int64_t pad_elems) {
   __shared__ float s[8][32][33];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int b = blockIdx.z / ytiles;
-  const int x0 = blockIdx.x * 32, z0 = blockIdx.y * 32;
-  const int y = (int)(blockIdx.z % ytiles) * 8 + w;
+  const int b = blockIdx.y, row = (int)blockIdx.x / xtiles;
+  const int x0 = (int)blockIdx.x % xtiles * 32, z0 = row / ytiles * 32;
+  const int y = row % ytiles * 8 + w;
   const int z = z0 + lane;
   const int64_t pz = nz + 2 * kPad, px = nx + 2 * kPad;
   const int xs = min(32, nx - x0);
@@ -1153,12 +1154,12 @@ int adjoint_impl(Plan* p, const float* sino, int batch, float* out, cudaStream_t
       note_launch();
       DTV_LAUNCH_CHECK();
     }
-    const int ytiles = (gp.ny + 7) / 8;
-    const int per = std::max(1, 65535 / ytiles);  // volumes per launch
-    for (int b = 0; b < batch; b += per) {
-      const dim3 grid((gp.nx + 31) / 32, (gp.nz + 31) / 32, ytiles * std::min(per, batch - b));
+    const int xtiles = (gp.nx + 31) / 32, ytiles = (gp.ny + 7) / 8;
+    const unsigned gtiles = (unsigned)xtiles * ytiles * ((gp.nz + 31) / 32);
+    for (int b = 0; b < batch; b += 65535) {
+      const dim3 grid(gtiles, std::min(65535, batch - b));
       adjoint_gather_kernel<<<grid, 256, 0, st>>>(p->d_cells + b * p->pad_elems, out + b * vox,
-                                                  gp.nx, gp.ny, gp.nz, ytiles, p->pad_elems);
+                                                  gp.nx, gp.ny, gp.nz, xtiles, ytiles, p->pad_elems);
       note_launch();
       DTV_LAUNCH_CHECK();
     }
