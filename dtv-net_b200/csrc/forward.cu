@@ -1135,24 +1135,30 @@ int adjoint_impl(Plan* p, const float* sino, int batch, float* out, cudaStream_t
     const int64_t rows = std::max<int64_t>(1, (160LL << 20) / row_bytes);
     const int slabs = (int)((gp.ny + 3 + rows - 1) / rows);
     const int slab = (gp.ny + 3 + slabs - 1) / slabs;
+    const int64_t per_view = (int64_t)gp.nu * gp.nv, per_item = gp.n_views * per_view;
     for (int yb = -2; yb <= gp.ny; yb += slab) {
-      // pairs of batch items share a launch's threads, an odd one runs alone
       const int ye = std::min(yb + slab, gp.ny + 1);
-      const int64_t per_item = (int64_t)gp.n_views * gp.nu * gp.nv;
-      if (batch >= 2) {
-        const auto kernel = slabs > 1 ? adjoint_cells_kernel<true, 2> : adjoint_cells_kernel<false, 2>;
-        kernel<<<dim3(tiles, gp.n_views, batch / 2), 256, 0, st>>>(rp, p->d_fpv, p->d_rays, sino,
-                                                                   p->d_cells, p->pad_elems, yb, ye);
+      for (int v0 = 0; v0 < gp.n_views; v0 += 65535) {  // views in the grid's y
+        const FPView* views = p->d_fpv + v0;
+        const float4* rays = p->d_rays + 2 * v0 * per_view;
+        const float* sv = sino + v0 * per_view;
+        const int nv = std::min(65535, gp.n_views - v0);
+        // pairs of batch items share a launch's threads, an odd one runs alone
+        if (batch >= 2) {
+          const auto kernel = slabs > 1 ? adjoint_cells_kernel<true, 2> : adjoint_cells_kernel<false, 2>;
+          kernel<<<dim3(tiles, nv, batch / 2), 256, 0, st>>>(rp, views, rays, sv, p->d_cells,
+                                                             p->pad_elems, yb, ye);
+          note_launch();
+          DTV_LAUNCH_CHECK();
+        }
+        if (batch % 2 == 0) continue;
+        const auto kernel = slabs > 1 ? adjoint_cells_kernel<true, 1> : adjoint_cells_kernel<false, 1>;
+        kernel<<<dim3(tiles, nv, 1), 256, 0, st>>>(rp, views, rays, sv + (batch - 1) * per_item,
+                                                   p->d_cells + (batch - 1) * p->pad_elems,
+                                                   p->pad_elems, yb, ye);
         note_launch();
         DTV_LAUNCH_CHECK();
       }
-      if (batch % 2 == 0) continue;
-      const auto kernel = slabs > 1 ? adjoint_cells_kernel<true, 1> : adjoint_cells_kernel<false, 1>;
-      kernel<<<dim3(tiles, gp.n_views, 1), 256, 0, st>>>(
-          rp, p->d_fpv, p->d_rays, sino + (batch - 1) * per_item,
-          p->d_cells + (batch - 1) * p->pad_elems, p->pad_elems, yb, ye);
-      note_launch();
-      DTV_LAUNCH_CHECK();
     }
     const int xtiles = (gp.nx + 31) / 32, ytiles = (gp.ny + 7) / 8;
     const unsigned gtiles = (unsigned)xtiles * ytiles * ((gp.nz + 31) / 32);
