@@ -606,16 +606,28 @@ static bool rec_far(const GeomParams& g) {
          std::max(g.nx, std::max(g.ny, g.nz)) + 2 * kPad > kIntMagicMost;
 }
 
-// `records`: the launch samples records, whose warps want two columns of 16 pixels
-// (tile 0, the default, then stands for those). A half warp's rays pass one (x, y)
-// column and read its records once; four columns of 8 touch more 128-byte lines, and
-// one of 32 needs blocks of 32 rows, which cross more of the volume at a time. 256^3 x
-// 64 views of 384^2: 2 x 16 3.28 ms, 4 x 8 3.49, 1 x 32 3.45, 8 x 4 4.07, 16 x 2 5.90;
-// 151x163x97 x 45 views of 231x149: 0.366, 0.387, 0.357 (1 x 32).
+// The ray tile of a launch that samples records, {log2 tu, log2 tv, log2 wu}: warps of
+// two columns of 16 pixels. A half warp's rays pass one (x, y) column and read its records
+// once; lower warps touch more 128-byte lines and one of 32 needs blocks of 32 rows, which
+// cross more of the volume at a time. 256^3 x 64 views of 384^2: 2 x 16 3.28 ms, 4 x 8
+// 3.49, 1 x 32 3.45, 8 x 4 4.07, 16 x 2 5.90; 151x163x97 x 45 views of 231x149: 0.366,
+// 0.387, 0.357 (1 x 32). Of detectors of up to four rows a warp and a block take no more
+// rows than there are: 512x512 x 360 views of 768 x 1 2106 -> 587 us, 200x180x3 x 60 views
+// of 256 x 3 70 -> 42. From five rows idle lanes can cost less than lower warps do
+// (96x96x64 x 45 views of 120 x 8: 31 us in 2 x 16, 41 in 4 x 8).
+static void rec_tile(int nv, int (&t)[3]) {
+  const int l = nv > 4 ? 4 : nv > 2 ? 2 : nv > 1 ? 1 : 0;
+  t[0] = 8 - l;
+  t[1] = l;
+  t[2] = 5 - l;
+}
+
+// `records`: the launch samples records (tile 0, the default, then stands for rec_tile).
 static RayParams plan_ray_params(const Plan* p, bool records) {
-  static const int kRecTile[3] = {4, 4, 1};
   RayParams rp = make_ray_params(p->gp);
-  const int* t = records && p->fp_ray_tile == 0 ? kRecTile : kRayTiles[p->fp_ray_tile];
+  int own[3];
+  rec_tile(p->gp.nv, own);
+  const int* t = records && p->fp_ray_tile == 0 ? own : kRayTiles[p->fp_ray_tile];
   rp.ltu = t[0];
   rp.ltv = t[1];
   rp.lwu = t[2];
@@ -666,8 +678,11 @@ int forward_refresh_impl(Plan* fast, Plan* exact, const void* vol, int vol_dtype
   rc = stage_volume(exact, vol, vol_dtype, batch, st);
   if (rc) return rc;
   RayParams rp = plan_ray_params(fast, false);
-  // the record order's columns per warp: two where the tile has 16 rows
-  const int rec_lwu = std::max(1, 5 - rp.ltv);
+  // the record order's columns per warp: two where the tile has 16 rows, as many as the
+  // tile takes for detectors of few rows (rec_tile)
+  int own[3];
+  rec_tile(gp.nv, own);
+  const int rec_lwu = std::min(rp.ltu, std::max(own[2], 5 - rp.ltv));
   // band-major plans march bands of one tile row here: with the exact
   // sampler's records beside the z-pairs, the narrower slab keeps more of both
   // in L2 (5.66 ms against 5.74 ms with the plan's 4 rows at 256^3 x 64 views)
