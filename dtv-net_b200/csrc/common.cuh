@@ -210,9 +210,11 @@ struct Plan {
   int bp_zaffine;            // every view's u and h are independent of z
   // adjoint ray table (DTV_PLAN_ADJOINT): per view and pixel, (p0, count) and (dp, 0)
   float4* d_rays;
-  // adjoint cell records (DTV_PLAN_ADJOINT): float4, the padded grid of d_vol_rec per batch item
+  // adjoint cell records (DTV_PLAN_ADJOINT): float4, room for the padded grid of d_vol_rec per
+  // batch item
   float4* d_cells;
   int adjoint_method;  // DTV_TUNE_ADJOINT
+  float adjoint_rows;  // detector rows per voxel (adjoint_impl's choice of scatter)
   double fp_samples;  // per volume, < 0 until computed
   uint64_t geom_key;  // hash of the geometry and its per-view tables
 };
@@ -239,6 +241,7 @@ int forward_refresh_impl(Plan* fast, Plan* exact, const void* vol, int vol_dtype
 int backward_refresh_impl(Plan* fast, Plan* exact, const float* sino, int batch, float* out,
                           float* e_b, cudaStream_t st);
 int bp_cull_rule(const Plan* p);
+float adjoint_rows(const Plan* p);
 int adjoint_impl(Plan* p, const float* sino, int batch, float* out, cudaStream_t st);
 int encode_pair_maps(Plan* p);
 // several plans' projections in one launch (forward.cu, backward.cu)

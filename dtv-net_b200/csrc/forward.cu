@@ -959,7 +959,7 @@ __global__ void __launch_bounds__(kAdjThreads) adjoint_brick_kernel(
 // records: 1.29 and 9.5 ms, bound by instruction issue (117 per 32 samples, 91 %).
 //
 // A thread takes NB batch items through the same samples: the positions, records
-// and runs are theirs alike (2 x 128^3: 1.32 -> 1.17 ms).
+// and runs are theirs alike (2 x 128^3: 1.32 -> 1.17 ms; adjoint_impl says when).
 //
 // Five blocks per SM: the bound gives the compiler a few registers more than it took
 // (47 against 43; 256^3 9.45 -> 8.98 ms, 128^3 0.697 -> 0.680); six spill (9.48).
@@ -1130,12 +1130,129 @@ __global__ void __launch_bounds__(256) adjoint_gather_kernel(const float4* __res
   for (int k = 0; k < min(32, nz - z0); ++k) o[(int64_t)(z0 + k) * ny * nx] = s[w][k][lane];
 }
 
+// ---- the same without merging ------------------------------------------------------------
+// For calls that have nothing to merge or too few rays to hide a warp's shuffles: records
+// x fastest over the cells that reach the volume (x and y from -1, z in it), threads in
+// the rays' own order, along u, so that a warp's reductions of neighbouring rays meet in
+// the L2's sectors. Cells by floorf: any axis length. Shared memory that it does not use
+// holds it to three blocks per SM: more reductions in flight contend for records (128^3,
+// 0.3 detector rows per voxel: 253 us with three blocks, 258 with four, 283 with six;
+// 512x512x1, 768 x 1: 545, 574, 604).
+constexpr int kScatterSmem = 70 * 1024;
+__global__ void __launch_bounds__(256) adjoint_scatter_kernel(float scale, const float4* __restrict__ rays,
+                                                              const float* __restrict__ sino,
+                                                              float4* __restrict__ cells, int64_t per_item,
+                                                              int batch, int nx, int ny, int nz, int zb0,
+                                                              int zb1) {
+  const int64_t cplane = (int64_t)(nx + 1) * (ny + 1);
+  for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < per_item * batch;
+       r += (int64_t)gridDim.x * blockDim.x) {
+    const float val = __ldg(sino + r) * scale;
+    if (val == 0.f) continue;
+    const int64_t b = r / per_item, ray = r - b * per_item;
+    const float4 a = __ldg(rays + 2 * ray), c = __ldg(rays + 2 * ray + 1);
+    float4* cb = cells + b * cplane * nz;
+    // the k range of the slab [zb0, zb1) from the ray's (monotone) z, widened by one
+    const int count = __float_as_int(a.w);
+    int k0 = 0, k1 = count;
+    if (c.z != 0.f) {
+      const float inv = 1.f / c.z, ka = ((float)zb0 - a.z) * inv, kb = ((float)zb1 - a.z) * inv;
+      const float n = (float)count;  // clamp in float: the estimates may be huge
+      k0 = (int)fminf(fmaxf(floorf(fminf(ka, kb)) - 1.f, 0.f), n);
+      k1 = (int)fminf(fmaxf(ceilf(fmaxf(ka, kb)) + 1.f, 0.f), n);
+    }
+    for (int k = k0; k < k1; ++k) {
+      const float kf = (float)k;
+      const float x = fmaf(kf, c.x, a.x), y = fmaf(kf, c.y, a.y), z = fmaf(kf, c.z, a.z);
+      const float fx = floorf(x), fy = floorf(y), fz = floorf(z);
+      const int ix = (int)fx, iy = (int)fy, iz = (int)fz;
+      if (iz < zb0 || iz >= zb1 || ix < -1 || ix >= nx || iy < -1 || iy >= ny) continue;
+      const float ax = x - fx, ay = y - fy, az = z - fz, bx = 1.f - ax, by = 1.f - ay;
+      float4* cell = cb + (int64_t)(iy + 1) * (nx + 1) + ix + 1;
+      if (iz >= 0) {
+        const float w = val * (1.f - az);
+        atomicAdd(cell + iz * cplane, make_float4(w * bx * by, w * ax * by, w * bx * ay, w * ax * ay));
+      }
+      if (iz + 1 < nz) {
+        const float w = val * az;
+        atomicAdd(cell + (iz + 1) * cplane,
+                  make_float4(w * bx * by, w * ax * by, w * bx * ay, w * ax * ay));
+      }
+    }
+  }
+}
+
+__global__ void __launch_bounds__(256) adjoint_scatter_gather_kernel(const float4* __restrict__ cells,
+                                                                     float* __restrict__ out, int nx, int ny,
+                                                                     int64_t total) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    const int x = (int)(i % nx);
+    const int64_t q = i / nx, z = q / ny;  // z over the whole batch
+    const int y = (int)(q - z * ny);
+    const float4* r = cells + ((z * (ny + 1) + y + 1) * (nx + 1) + x + 1);  // cell (x, y)
+    out[i] = __ldg(&r->x) + __ldg(&r[-1].y) + __ldg(&r[-(nx + 1)].z) + __ldg(&r[-(nx + 1) - 1].w);
+  }
+}
+
+static int adjoint_scatter(Plan* p, const float* sino, int batch, float* out, cudaStream_t st) {
+  const GeomParams& gp = p->gp;
+  const int64_t cplane = (int64_t)(gp.nx + 1) * (gp.ny + 1);
+  DTV_CUDA_TRY(cudaMemsetAsync(p->d_cells, 0, cplane * gp.nz * batch * sizeof(float4), st));
+  const int64_t rays = (int64_t)gp.n_views * gp.nu * gp.nv;
+  const int grid = (int)std::min<int64_t>((rays * batch + 255) / 256, 148LL * 64);
+  // z-slabs whose records (at most 72 MB over the batch) stay in L2; cells from z = -1
+  const int slab = (int)std::max<int64_t>(1, (72LL << 20) / (cplane * (int64_t)sizeof(float4) * batch));
+  DTV_CUDA_TRY(cudaFuncSetAttribute(adjoint_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    kScatterSmem));
+  for (int zb0 = -1; zb0 < gp.nz; zb0 += slab) {
+    adjoint_scatter_kernel<<<grid, 256, kScatterSmem, st>>>((float)gp.scale, p->d_rays, sino, p->d_cells, rays, batch,
+                                                 gp.nx, gp.ny, gp.nz, zb0, std::min(zb0 + slab, gp.nz));
+    note_launch();
+    DTV_LAUNCH_CHECK();
+  }
+  const int64_t total = (int64_t)gp.nx * gp.ny * gp.nz * batch;
+  adjoint_scatter_gather_kernel<<<(int)std::min<int64_t>((total + 255) / 256, 148LL * 32), 256, 0, st>>>(
+      p->d_cells, out, gp.nx, gp.ny, total);
+  note_launch();
+  DTV_LAUNCH_CHECK();
+  return DTV_OK;
+}
+
+// Detector rows per voxel along z, seen from the volume's centre, over a sample of views.
+float adjoint_rows(const Plan* p) {
+  const GeomParams& gp = p->gp;
+  const double x = 0.5 * (gp.nx - 1), y = 0.5 * (gp.ny - 1), z = 0.5 * (gp.nz - 1);
+  double sum = 0.0;
+  int n = 0;
+  for (int i = 0; i < gp.n_views; i += std::max(1, gp.n_views / 48), ++n) {
+    const float* m = p->h_bpv[i].m;
+    const double h = m[8] * x + m[9] * y + m[10] * z + m[11];
+    const double v = m[4] * x + m[5] * y + m[6] * z + m[7];
+    const double d = fabs((m[6] * h - m[10] * v) / (h * h));
+    if (d < 1e6) sum += d;  // (NaN and infinity of a source plane through the centre left out)
+  }
+  return (float)(sum / n);
+}
+
 int adjoint_impl(Plan* p, const float* sino, int batch, float* out, cudaStream_t st) {
   const GeomParams& gp = p->gp;
   RayParams rp = make_ray_params(gp);
   const int64_t vox = (int64_t)gp.nx * gp.ny * gp.nz;
-  const bool wide = std::max(gp.nx, std::max(gp.ny, gp.nz)) + 2 * kPad > kIntMagicMost;
-  if (p->adjoint_method == 1 && p->d_cells && !wide) {
+  if (p->adjoint_method == 1 && p->d_cells) {
+    // Merging pays from about half a detector row per voxel on, where the rows fill a
+    // warp's eight lanes, and with enough warps to hide its shuffles: below 3500 (a call
+    // of 1300 at 40^3, 1.2 rows per voxel: 25.0 us without, 28.0 with; 2600: 36.6, 34.3;
+    // 5400 at 64^3: 84, 60), on few rows (512x512 x 360 views of 768 x 1: 545, 2288) or
+    // sparse ones (0.3 per voxel, 96^3: 95, 145; 128^3: 257, 310; 0.46: 1180, 1152) the
+    // plain scatter is the faster one. Axes beyond kIntMagicMost have it too.
+    const int64_t warps = (int64_t)gp.n_views * gp.nu * gp.nv / 32;
+    const bool wide = std::max(gp.nx, std::max(gp.ny, gp.nz)) + 2 * kPad > kIntMagicMost;
+    if (p->adjoint_rows < 0.4f || gp.nv < 5 || warps * batch < 3500 || wide)
+      return adjoint_scatter(p, sino, batch, out, st);
+    // Two items per thread where many rays share records: 2 x 96^3, 1.2 rows per voxel,
+    // 18600 warps: 287 us, 304 singly; 0.9: 267, 248; 2 x 64^3, 1.2, 5400 warps: 94, 89.
+    const bool pairs = p->adjoint_rows >= 1.1f && warps >= 9000;
     DTV_CUDA_TRY(cudaMemsetAsync(p->d_cells, 0, p->pad_elems * batch * sizeof(float4), st));
     // warps of 4 x 8 rays: 128^3 x 48 views 0.68 ms (1 x 32: 0.73, 2 x 16: 0.69;
     // 97x113x61 x 33 views: 271, 334, 291 us)
@@ -1154,25 +1271,23 @@ int adjoint_impl(Plan* p, const float* sino, int batch, float* out, cudaStream_t
     for (int yb = -2; yb <= gp.ny; yb += slab) {
       const int ye = std::min(yb + slab, gp.ny + 1);
       for (int v0 = 0; v0 < gp.n_views; v0 += 65535) {  // views in the grid's y
-        const FPView* views = p->d_fpv + v0;
-        const float4* rays = p->d_rays + 2 * v0 * per_view;
-        const float* sv = sino + v0 * per_view;
         const int nv = std::min(65535, gp.n_views - v0);
-        // pairs of batch items share a launch's threads, an odd one runs alone
-        if (batch >= 2) {
-          const auto kernel = slabs > 1 ? adjoint_cells_kernel<true, 2> : adjoint_cells_kernel<false, 2>;
-          kernel<<<dim3(tiles, nv, batch / 2), 256, 0, st>>>(rp, views, rays, sv, p->d_cells,
-                                                             p->pad_elems, yb, ye);
+        auto scatter = [&](auto kernel, int first, int z) {  // items from `first`
+          kernel<<<dim3(tiles, nv, z), 256, 0, st>>>(
+              rp, p->d_fpv + v0, p->d_rays + 2 * v0 * per_view, sino + v0 * per_view + first * per_item,
+              p->d_cells + first * p->pad_elems, p->pad_elems, yb, ye);
           note_launch();
           DTV_LAUNCH_CHECK();
-        }
-        if (batch % 2 == 0) continue;
-        const auto kernel = slabs > 1 ? adjoint_cells_kernel<true, 1> : adjoint_cells_kernel<false, 1>;
-        kernel<<<dim3(tiles, nv, 1), 256, 0, st>>>(rp, views, rays, sv + (batch - 1) * per_item,
-                                                   p->d_cells + (batch - 1) * p->pad_elems,
-                                                   p->pad_elems, yb, ye);
-        note_launch();
-        DTV_LAUNCH_CHECK();
+          return (int)DTV_OK;
+        };
+        const int two = pairs ? batch / 2 : 0;
+        int rc = DTV_OK;
+        if (two > 0)
+          rc = scatter(slabs > 1 ? adjoint_cells_kernel<true, 2> : adjoint_cells_kernel<false, 2>, 0, two);
+        if (!rc && batch > 2 * two)
+          rc = scatter(slabs > 1 ? adjoint_cells_kernel<true, 1> : adjoint_cells_kernel<false, 1>, 2 * two,
+                       batch - 2 * two);
+        if (rc) return rc;
       }
     }
     const int xtiles = (gp.nx + 31) / 32, ytiles = (gp.ny + 7) / 8;

@@ -314,6 +314,7 @@ int create_plan(const dtv_geometry* g, int max_batch, int flags, int device, Pla
     PLAN_CUDA(cudaMalloc(&p->d_rays, n * sizeof(float4)));
     PLAN_CUDA(cudaMalloc(&p->d_cells, (size_t)p->pad_elems * max_batch * sizeof(float4)));
     p->adjoint_method = 1;
+    p->adjoint_rows = adjoint_rows(p);
     rc = build_ray_table(p, 0);
     if (!rc) {
       cudaError_t e = cudaStreamSynchronize(0);
