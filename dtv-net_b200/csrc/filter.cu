@@ -36,7 +36,8 @@ namespace dtv {
 
 constexpr int kFiltThreads = 256;
 constexpr int kFiltMaxWidth = 8192;
-constexpr int kOut = 8;  // outputs of each parity per thread
+constexpr int64_t kFiltSmall = 10000;  // threads (filt_small)
+// outputs of each parity per thread: 8, or 2 for calls with few rows (filt_small)
 
 // Shared layout: the taps (one set per block), then per row a padded sequence
 // of pairs; slot lead + m holds (x[2m+1], x[2m+2]), so that both parities'
@@ -50,13 +51,16 @@ struct FiltShape {
   int rows;     // rows per block
   int threads;  // per block
 };
+template <int kOut>
 __host__ __device__ constexpr int filt_skew(int i) { return i + i / kOut; }
 // the skewed offset of slot d from one at a multiple of kOut
+template <int kOut>
 __host__ __device__ constexpr int filt_off(int d) {
   return d >= 0 ? d + d / kOut : d - (-d + kOut - 1) / kOut;
 }
 // Rows per block: what 256 threads hold, less where the grid would have fewer
 // than four blocks per SM.
+template <int kOut>
 static FiltShape filt_shape(int width, int64_t rows) {
   FiltShape f;
   f.n = width / 2;
@@ -64,7 +68,7 @@ static FiltShape filt_shape(int width, int64_t rows) {
   f.taps = ((width / 2 + 1) / 2 + kOut - 1) / kOut * kOut;
   f.lead = f.taps + kOut;
   // the right window reaches taps + kOut beyond the last output's slot
-  f.seq = filt_skew(f.lead + f.groups * kOut + f.taps + kOut) + 1;
+  f.seq = filt_skew<kOut>(f.lead + f.groups * kOut + f.taps + kOut) + 1;
   f.rows = (int)std::max<int64_t>(1, std::min<int64_t>(kFiltThreads / f.groups, rows / (4 * 148)));
   f.rows = std::min(f.rows, 16);
   f.threads = std::min(kFiltThreads, (f.groups * f.rows + 31) / 32 * 32);
@@ -76,6 +80,7 @@ static size_t filt_smem(const FiltShape& f) {
 
 // At most 72 registers: rows of 1680 columns then have four blocks of 224 threads per
 // SM (unbounded the compiler takes 80; 6144 x 1680: 411 us, with the bound 362).
+template <int kOut>
 __global__ void __maxnreg__(72) fbp_filter_kernel(const float* __restrict__ in,
                                                                   float* __restrict__ out, int64_t rows,
                                                                   int rows_per_view, int width,
@@ -107,24 +112,24 @@ __global__ void __maxnreg__(72) fbp_filter_kernel(const float* __restrict__ in,
     for (int c = threadIdx.x; c < width; c += blockDim.x) {
       float x = __ldg(in + (r0 + rr) * width + c);
       if (!adjoint) x *= cosine(row, c);
-      s[2 * filt_skew(f.lead + ((c - 1) >> 1)) + ((c - 1) & 1)] = x;
+      s[2 * filt_skew<kOut>(f.lead + ((c - 1) >> 1)) + ((c - 1) & 1)] = x;
     }
   }
   __syncthreads();
   for (int job = threadIdx.x; job < f.groups * nr; job += blockDim.x) {
     const int g = job % f.groups, rr = job / f.groups;
     const int m0 = g * kOut;
-    const f32x2_t* mid = seqs + rr * f.seq + filt_skew(f.lead + m0);
-    const f32x2_t* right = mid + filt_skew(f.taps - kOut);
-    const f32x2_t* left = mid - filt_skew(f.taps - kOut);
+    const f32x2_t* mid = seqs + rr * f.seq + filt_skew<kOut>(f.lead + m0);
+    const f32x2_t* right = mid + filt_skew<kOut>(f.taps - kOut);
+    const f32x2_t* left = mid - filt_skew<kOut>(f.taps - kOut);
     // windows of the last tap, slot of offset o at o mod kOut: right offsets
     // taps - 1 + e, left offsets -taps + e
     f32x2_t acc[kOut], rw[kOut], lw[kOut];
 #pragma unroll
     for (int e = 0; e < kOut; ++e) {
       acc[e] = 0;
-      rw[(e + kOut - 1) % kOut] = right[filt_off(kOut - 1 + e)];
-      lw[(e + 1) % kOut] = left[filt_off(e - kOut)];
+      rw[(e + kOut - 1) % kOut] = right[filt_off<kOut>(kOut - 1 + e)];
+      lw[(e + 1) % kOut] = left[filt_off<kOut>(e - kOut)];
     }
     // kOut taps from j; those beyond the last of the width (kLast) meet columns whose
     // infinities or NaN do not belong to the sum
@@ -138,8 +143,8 @@ __global__ void __maxnreg__(72) fbp_filter_kernel(const float* __restrict__ in,
           for (int e = 0; e < kOut; ++e)
             acc[e] = fma2(t, add2(rw[(e + q) % kOut], lw[(e - q + kOut) % kOut]), acc[e]);
         }
-        rw[(q + kOut - 1) % kOut] = right[filt_off(q - 1)];
-        lw[(kOut - q) % kOut] = left[filt_off(kOut - 1 - q)];
+        rw[(q + kOut - 1) % kOut] = right[filt_off<kOut>(q - 1)];
+        lw[(kOut - q) % kOut] = left[filt_off<kOut>(kOut - 1 - q)];
       }
       right -= kOut + 1;
       left += kOut + 1;
@@ -154,8 +159,8 @@ __global__ void __maxnreg__(72) fbp_filter_kernel(const float* __restrict__ in,
       // the centre tap: x[2m] and x[2m+1]
       float y0, y1, c0, c1, unused;
       unpack2(acc[e], y0, y1);
-      unpack2(mid[filt_off(e - 1)], unused, c0);
-      unpack2(mid[filt_off(e)], c1, unused);
+      unpack2(mid[filt_off<kOut>(e - 1)], unused, c0);
+      unpack2(mid[filt_off<kOut>(e)], c1, unused);
       y0 = fmaf(0.125f, c0, y0);
       y1 = fmaf(0.125f, c1, y1);
       const int u = 2 * (m0 + e);
@@ -167,6 +172,39 @@ __global__ void __maxnreg__(72) fbp_filter_kernel(const float* __restrict__ in,
       out[r * width + u + 1] = y1;
     }
   }
+}
+
+// Whether the threads of eight outputs per parity leave most of the GPU idle: each sums
+// over half the row one tap after the other, so more threads of two finish earlier, as
+// long as they fit the GPU about once and a row one block. 40 rows of 250: 6.2 us with
+// eight, 4.1 with two; 600 of 250 7.2, 5.1; 40 of 1000 12.9, 8.7; 600 of 1000 23.7, 30.1;
+// 40 of 1680 16.8, 20.1.
+static bool filt_small(int width, int64_t rows) {
+  return width <= 1024 && (width / 2 + 7) / 8 * rows < kFiltSmall;
+}
+
+template <int kOut>
+static int filt_launch(const float* in, float* out, int64_t rows, int32_t rows_per_view, int32_t width,
+                       float sdd, float mid_i, float mid_j, int32_t adjoint, cudaStream_t st) {
+  const FiltShape f = filt_shape<kOut>(width, rows);
+  const size_t smem = filt_smem(f);
+  if (smem > 48 * 1024) {
+    // per-device function attribute, raised once to the widest row's need
+    static std::atomic<unsigned long long> raised{0};
+    int dev = 0;
+    DTV_CUDA_TRY(cudaGetDevice(&dev));
+    const unsigned long long bit = 1ull << (dev & 63);
+    if (!(raised.load() & bit)) {
+      DTV_CUDA_TRY(cudaFuncSetAttribute(fbp_filter_kernel<kOut>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)filt_smem(filt_shape<kOut>(kFiltMaxWidth, 1))));
+      raised |= bit;
+    }
+  }
+  fbp_filter_kernel<kOut><<<(unsigned)((rows + f.rows - 1) / f.rows), f.threads, smem, st>>>(
+      in, out, rows, rows_per_view, width, f, sdd, mid_i, mid_j, adjoint ? 1 : 0);
+  note_launch();
+  DTV_LAUNCH_CHECK();
+  return DTV_OK;
 }
 
 }  // namespace dtv
@@ -184,23 +222,7 @@ extern "C" int dtv_fbp_filter(const float* in, float* out, int64_t rows, int32_t
   DTV_CHECK(width >= 2 && width % 2 == 0 && width <= kFiltMaxWidth,
             "row width must be even and in [2, %d]", kFiltMaxWidth);
   DTV_CHECK(sdd > 0.f, "sdd must be positive");
-  const FiltShape f = filt_shape(width, rows);
-  const size_t smem = filt_smem(f);
-  if (smem > 48 * 1024) {
-    // per-device function attribute, raised once to the widest row's need
-    static std::atomic<unsigned long long> raised{0};
-    int dev = 0;
-    DTV_CUDA_TRY(cudaGetDevice(&dev));
-    const unsigned long long bit = 1ull << (dev & 63);
-    if (!(raised.load() & bit)) {
-      DTV_CUDA_TRY(cudaFuncSetAttribute(fbp_filter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)filt_smem(filt_shape(kFiltMaxWidth, 1))));
-      raised |= bit;
-    }
-  }
-  fbp_filter_kernel<<<(unsigned)((rows + f.rows - 1) / f.rows), f.threads, smem, as_stream(stream)>>>(
-      in, out, rows, rows_per_view, width, f, sdd, mid_i, mid_j, adjoint ? 1 : 0);
-  note_launch();
-  DTV_LAUNCH_CHECK();
-  return DTV_OK;
+  if (filt_small(width, rows))
+    return filt_launch<2>(in, out, rows, rows_per_view, width, sdd, mid_i, mid_j, adjoint, as_stream(stream));
+  return filt_launch<8>(in, out, rows, rows_per_view, width, sdd, mid_i, mid_j, adjoint, as_stream(stream));
 }
