@@ -39,8 +39,12 @@ struct BPMaps {
 static_assert(sizeof(BPMaps) <= 31 * 1024, "kernel parameter space");
 constexpr int kBPThreads = kBPTile * kBPTile;
 // voxels per thread along z (16 measured 3 % slower through the texture unit and
-// 10 - 20 % through records: fewer resident warps)
-constexpr int kZC = 8;
+// 10 - 20 % through records: fewer resident warps); of volumes of up to kFlat slices
+// kZCFlat, so that a thread does not project slices that are not there (231x152x1 x 32
+// views of 389 x 3, records: 16.9 -> 10.8 us; 512x512x1 x 360 views, texture: 704 -> 294);
+// of four slices not where blocks look for their views first, twice then (75x78x4 x 176
+// modules: 17 us, 21)
+constexpr int kZC = 8, kZCFlat = 2, kFlat = 4;
 
 // Where a bilinear detector sample comes from.
 // kTex: the texture unit (a layered FP32 texture, 8-bit weights), one fetch.
@@ -137,7 +141,7 @@ __host__ __device__ __forceinline__ bool box_seen(const float* w, float i0, floa
   return !(hmin > 1e-3f && (umax < -2.f || umin > nu + 1.f || vmax < -2.f || vmin > nv + 1.f));
 }
 
-// One block's columns: column tile `tile`, z-chunk `zc` of kZC voxels, views
+// One block's columns: column tile `tile`, z-chunk `zc` of ZC voxels, views
 // n0 .. n0 + n_chunk - 1. S == 1: a tile is 16 x 16 columns. S > 1 (volumes
 // too small to fill the GPU otherwise): the block's S groups of 256 / S threads
 // own the same tile of (64 / (2 S)) x 8 columns and each takes one of S equal
@@ -166,12 +170,11 @@ struct BPShape {
   static constexpr int kW = kGroup / kH;                  // tile columns (x)
 };
 
-template <int kMode, bool kZAff, int S, bool kCull, class Maps>
+template <int kMode, bool kZAff, int S, bool kCull, int ZC, class Maps>
 __device__ __forceinline__ void bp_columns(const BPParams& bp, const Maps& maps, int n0, int n_chunk,
                                            const float4* __restrict__ recs, cudaTextureObject_t tex,
                                            const BPOut& dst, int tile, int zc) {
-  static_assert(kZC % 2 == 0, "voxels go in pairs");
-  constexpr int ZC = kZC;
+  static_assert(ZC % 2 == 0, "voxels go in pairs");
   using Shape = BPShape<S>;
   const int tiles_x = (bp.nx + Shape::kW - 1) / Shape::kW;
   const int t = (int)threadIdx.x;
@@ -461,12 +464,12 @@ __device__ __forceinline__ void bp_columns(const BPParams& bp, const Maps& maps,
 
 // Unsplit record kernels are held to 48 registers for five blocks per SM: their
 // loads' latency is the bound (256^3 x 64 views: 0.97 -> 0.90 ms).
-template <int kMode, bool kZAff, int S, bool kCull>
+template <int kMode, bool kZAff, int S, bool kCull, int ZC>
 __global__ void __launch_bounds__(kBPThreads, kMode == kRec && kZAff && S == 1 ? 5 : 1) bp_kernel(BPParams bp, const __grid_constant__ BPMaps maps,
                                                         int n0, int n_chunk,
                                                         const float4* __restrict__ recs,
                                                         cudaTextureObject_t tex, BPOut dst) {
-  bp_columns<kMode, kZAff, S, kCull>(bp, ParamMaps{&maps}, n0, n_chunk, recs, tex, dst,
+  bp_columns<kMode, kZAff, S, kCull, ZC>(bp, ParamMaps{&maps}, n0, n_chunk, recs, tex, dst,
                                          (int)blockIdx.x, (int)blockIdx.y);
 }
 
@@ -547,29 +550,38 @@ static int bp_split(const GeomParams& gp) {
     S *= 2;
   return S;
 }
-static size_t bp_smem(int mode, int S) {
-  return (size_t)(S - 1) * (mode == kBoth ? 2 : 1) * kZC * (kBPThreads / S) * sizeof(float);
+static size_t bp_smem(int mode, int S, int zc) {
+  return (size_t)(S - 1) * (mode == kBoth ? 2 : 1) * zc * (kBPThreads / S) * sizeof(float);
 }
 
 struct BPLaunch {
   dim3 grid;
-  int S;
+  int S, zc;
   cudaStream_t st;
 };
 
-template <int kMode, bool kZAff, bool kCull>
+template <int kMode, bool kZAff, bool kCull, int ZC>
 static void launch_bp_shape(const BPLaunch& l, const BPParams& bp, const BPMaps& maps, int n0,
                             int cnt, const float4* recs, cudaTextureObject_t tex,
                             const BPOut& dst) {
-  const size_t sm = bp_smem(kMode, l.S);
-  if (l.S == 8)
-    bp_kernel<kMode, kZAff, 8, kCull><<<l.grid, kBPThreads, sm, l.st>>>(bp, maps, n0, cnt, recs, tex, dst);
-  else if (l.S == 4)
-    bp_kernel<kMode, kZAff, 4, kCull><<<l.grid, kBPThreads, sm, l.st>>>(bp, maps, n0, cnt, recs, tex, dst);
-  else if (l.S == 2)
-    bp_kernel<kMode, kZAff, 2, kCull><<<l.grid, kBPThreads, sm, l.st>>>(bp, maps, n0, cnt, recs, tex, dst);
-  else
-    bp_kernel<kMode, kZAff, 1, kCull><<<l.grid, kBPThreads, sm, l.st>>>(bp, maps, n0, cnt, recs, tex, dst);
+  const auto kernel = l.S == 8   ? bp_kernel<kMode, kZAff, 8, kCull, ZC>
+                      : l.S == 4 ? bp_kernel<kMode, kZAff, 4, kCull, ZC>
+                      : l.S == 2 ? bp_kernel<kMode, kZAff, 2, kCull, ZC>
+                                 : bp_kernel<kMode, kZAff, 1, kCull, ZC>;
+  kernel<<<l.grid, kBPThreads, bp_smem(kMode, l.S, ZC), l.st>>>(bp, maps, n0, cnt, recs, tex, dst);
+}
+
+template <int kMode, bool kZAff, bool kCull>
+static void launch_bp_chunk(const BPLaunch& l, const BPParams& bp, const BPMaps& maps, int n0,
+                            int cnt, const float4* recs, cudaTextureObject_t tex,
+                            const BPOut& dst) {
+  if constexpr (kMode != kBoth) {
+    if (l.zc == kZCFlat) {
+      launch_bp_shape<kMode, kZAff, kCull, kZCFlat>(l, bp, maps, n0, cnt, recs, tex, dst);
+      return;
+    }
+  }
+  launch_bp_shape<kMode, kZAff, kCull, kZC>(l, bp, maps, n0, cnt, recs, tex, dst);
 }
 
 template <int kMode>
@@ -577,11 +589,11 @@ static void launch_bp_mode(const BPLaunch& l, bool zaff, const BPParams& bp, con
                            int n0, int cnt, const float4* recs, cudaTextureObject_t tex,
                            const BPOut& dst) {
   if (bp.cull) {
-    if (zaff) launch_bp_shape<kMode, true, true>(l, bp, maps, n0, cnt, recs, tex, dst);
-    else launch_bp_shape<kMode, false, true>(l, bp, maps, n0, cnt, recs, tex, dst);
+    if (zaff) launch_bp_chunk<kMode, true, true>(l, bp, maps, n0, cnt, recs, tex, dst);
+    else launch_bp_chunk<kMode, false, true>(l, bp, maps, n0, cnt, recs, tex, dst);
   } else {
-    if (zaff) launch_bp_shape<kMode, true, false>(l, bp, maps, n0, cnt, recs, tex, dst);
-    else launch_bp_shape<kMode, false, false>(l, bp, maps, n0, cnt, recs, tex, dst);
+    if (zaff) launch_bp_chunk<kMode, true, false>(l, bp, maps, n0, cnt, recs, tex, dst);
+    else launch_bp_chunk<kMode, false, false>(l, bp, maps, n0, cnt, recs, tex, dst);
   }
 }
 
@@ -589,9 +601,9 @@ static void launch_bp(int mode, const BPLaunch& l, bool zaff, const BPParams& bp
                       const BPMaps& maps, int n0, int cnt, const float4* recs,
                       cudaTextureObject_t tex, const BPOut& dst) {
   if (mode == kWide && zaff)
-    bp_kernel<kWide, true, 1, false><<<l.grid, kBPThreads, 0, l.st>>>(bp, maps, n0, cnt, recs, tex, dst);
+    bp_kernel<kWide, true, 1, false, kZC><<<l.grid, kBPThreads, 0, l.st>>>(bp, maps, n0, cnt, recs, tex, dst);
   else if (mode == kWide)
-    bp_kernel<kWide, false, 1, false><<<l.grid, kBPThreads, 0, l.st>>>(bp, maps, n0, cnt, recs, tex, dst);
+    bp_kernel<kWide, false, 1, false, kZC><<<l.grid, kBPThreads, 0, l.st>>>(bp, maps, n0, cnt, recs, tex, dst);
   else if (mode == kTex) launch_bp_mode<kTex>(l, zaff, bp, maps, n0, cnt, recs, tex, dst);
   else if (mode == kBoth) launch_bp_mode<kBoth>(l, zaff, bp, maps, n0, cnt, recs, tex, dst);
   else launch_bp_mode<kRec>(l, zaff, bp, maps, n0, cnt, recs, tex, dst);
@@ -673,7 +685,10 @@ static int bp_view_chunks(const Plan* p, int mode, Plan* rec, const float* sino,
   const cudaTextureObject_t tex = p->sino_tex ? p->sino_tex[0] : 0;
   if (mode == kRec && std::max(gp.nu, gp.nv) + 2 * kPad > kIntMagicMost) mode = kWide;
   const int S = mode == kWide ? 1 : bp_split(gp);
-  const BPLaunch l{dim3(bp_tiles(gp, S), (gp.nz + kZC - 1) / kZC), S, st};
+  // (the view split stays that of kZC, for the many-plan launches' sums)
+  const bool flat = gp.nz <= (bp.cull ? kFlat - 1 : kFlat);
+  const int zc = flat && (mode == kRec || mode == kTex) ? kZCFlat : kZC;
+  const BPLaunch l{dim3(bp_tiles(gp, S), (gp.nz + zc - 1) / zc), S, zc, st};
   const int run = mode == kTex ? gp.n_views : rec->sino_rec_views;
   BPMaps maps;
   for (int r0 = 0; r0 < gp.n_views; r0 += run) {
@@ -782,12 +797,12 @@ __global__ void __launch_bounds__(kBPThreads) bp_many_kernel(const __grid_consta
   const int nv = it.bp.n_views;
   if (it.map0 >= 0) {
     const RowMaps rows{m.m + it.map0};
-    if (it.zaffine) bp_columns<kTex, true, S, false>(it.bp, rows, 0, nv, nullptr, it.tex, dst, tile, zc);
-    else bp_columns<kTex, false, S, false>(it.bp, rows, 0, nv, nullptr, it.tex, dst, tile, zc);
+    if (it.zaffine) bp_columns<kTex, true, S, false, kZC>(it.bp, rows, 0, nv, nullptr, it.tex, dst, tile, zc);
+    else bp_columns<kTex, false, S, false, kZC>(it.bp, rows, 0, nv, nullptr, it.tex, dst, tile, zc);
   } else {
     const TableMaps rows{it.views};
-    if (it.zaffine) bp_columns<kTex, true, S, false>(it.bp, rows, 0, nv, nullptr, it.tex, dst, tile, zc);
-    else bp_columns<kTex, false, S, false>(it.bp, rows, 0, nv, nullptr, it.tex, dst, tile, zc);
+    if (it.zaffine) bp_columns<kTex, true, S, false, kZC>(it.bp, rows, 0, nv, nullptr, it.tex, dst, tile, zc);
+    else bp_columns<kTex, false, S, false, kZC>(it.bp, rows, 0, nv, nullptr, it.tex, dst, tile, zc);
   }
 }
 
@@ -840,7 +855,7 @@ int backward_many_impl(Plan* const* plans, const float* const* sinos, float* con
     DTV_CHECK(blocks < 2147483647LL, "too many blocks for one launch");
     m.count = cnt;
     const unsigned nb = (unsigned)blocks;
-    const size_t sm = bp_smem(kTex, S);
+    const size_t sm = bp_smem(kTex, S, kZC);
     if (S == 8) bp_many_kernel<8><<<nb, kBPThreads, sm, st>>>(m, accumulate);
     else if (S == 4) bp_many_kernel<4><<<nb, kBPThreads, sm, st>>>(m, accumulate);
     else if (S == 2) bp_many_kernel<2><<<nb, kBPThreads, sm, st>>>(m, accumulate);
