@@ -19,7 +19,7 @@ texture pipe and the shared-memory/FMA pipes work side by side.
 DTV_TUNE_ADJOINT applies to plans with adjoint tables: the exact adjoint
 scatters either per 16^3 brick through shared-memory atomics (0) or into
 per-cell records with 16-byte vector atomics in L2 (1), merged between a
-warp's neighbouring rays first; the first may win where few rays meet a volume. It is timed on plan.adjoint.
+warp's neighbouring rays first where the scan is dense. It is timed on plan.adjoint.
 
 DTV_TUNE_FP_BAND picks the forward projector's block order: view by view (0),
 or bands of B tile rows with every view of a band before the next band, which

@@ -184,7 +184,8 @@ DTV_API int dtv_plan_destroy(dtv_plan* plan);
  *   (block tu x tv pixels, warp wu x wv pixels): 0 (16x16, 8x4) default,
  *   1 (16x16, 16x2), 2 (32x8, 32x1), 3 (16x16, 4x8), 4 (32x8, 8x4),
  *   5 (8x32, 8x4), 6 (64x4, 32x1), 7 (8x32, 4x8); for plans that sample records
- *   (software FP32 and exact), 0 is (16x16, 2x16).
+ *   (software FP32 and exact), 0 is (16x16, 2x16), with fewer rows for
+ *   detectors of up to four.
  * No counterpart in the reference (its kernels use one fixed launch shape). */
 #define DTV_TUNE_FP_RAY_TILE 1
 /*   DTV_TUNE_FP_TEX_SHARE: with DTV_PLAN_TMA, how many eighths of the ray
